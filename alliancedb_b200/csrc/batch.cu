@@ -147,6 +147,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     for (uint32_t w = 0; w < W; w++) {
         const uint64_t nr = r_off[w + 1] - r_off[w], ns = s_off[w + 1] - s_off[w];
         bits[w] = (uint8_t)bits_for_window(nr, ns);
+        if (!bits[w] && nr > 4096) bits[w] = 1;   // the join's chains need a slot index in bits + log2(heads) key bits
         wbase[w] = (uint32_t)D;
         uoffR[w] = (uint32_t)uR;
         uoffS[w] = (uint32_t)uS;
@@ -304,7 +305,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ja.bits = 0;   // per-window fan-out: the kernel reads each window's bits
     ja.mat = nullptr; ja.mat_n = nullptr; ja.mat_cap = 0;
     ja.wbase = d_wbase; ja.wbits = d_bits; ja.nwin = W; ja.wacc = wacc;
-    radix_join_items<TableKind::Chain><<<ctx->num_sms * kJoinMinBlocks, kJoinThreads, kJoinSmem, st>>>(ja);
+    radix_join_items<false><<<ctx->num_sms * kJoinMinBlocks, kJoinThreads, kJoinSmem, st>>>(ja);
     ADB_CK(cudaGetLastError());
     ADB_CK(cudaEventRecord(ctx->ev[3], st));
     ctx->kernels += 14;

@@ -332,9 +332,8 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
                     unsigned long long *acc) {
     switch (a->fam) {
         case Family::Radix:
-            return run_radix(ctx, j, false, radix_bits_for(j.nR, p ? p->radix_bits : 0), acc);
         case Family::RadixHist:
-            return run_radix(ctx, j, true, radix_bits_for(j.nR, p ? p->radix_bits : 0), acc);
+            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), acc);
         case Family::Npo: return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
         case Family::SortMerge: return run_smj(ctx, j, p ? p->part_fanout : 0, a->model == 1, acc);
         case Family::Shj:

@@ -36,7 +36,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
 // ---- radix (PRO / RJ_st / PRH / PRHO) ----
 int radix_bits_for(uint64_t nR, int requested);
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
-int run_radix(Context *ctx, const DevJoin &j, bool hist_table, int bits, unsigned long long *acc);
+int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc);
 
 // ---- NPO / NPO_st ----
 uint32_t npo_region_bits(uint64_t nR, int requested);

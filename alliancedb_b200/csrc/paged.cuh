@@ -62,9 +62,11 @@ struct PartOut {
 };
 
 struct PassIn {
-    // flat input (pass 1): the relation
+    // flat input (pass 1): the relation, and the CTAs that share it (the
+    // others of the launch idle)
     const uint64_t *in;
     uint64_t n;
+    int G;
     // paged input (pass 2): the previous pass's pages, grouped by its digit
     const uint64_t *pages;
     const uint8_t *pcount;
@@ -162,8 +164,8 @@ partition_pass(PassArgs a) {
     uint32_t p1 = 0;              // paged: input partition; segmented: segment
     DigitFn df = a.df;
     if (kMode == 0) {
-        const uint64_t chunk = chunk_of(in.n, a.G);
-        b = (uint64_t)g * chunk;
+        const uint64_t chunk = chunk_of(in.n, in.G);
+        b = min(in.n, (uint64_t)g * chunk);
         e = min(in.n, b + chunk);
     } else if ((uint32_t)g < in.uoff[a.F1]) {
         uint32_t lo = 0, hi = a.F1;   // largest p with uoff[p] <= g

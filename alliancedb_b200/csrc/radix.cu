@@ -9,21 +9,30 @@
 //   R chunks      part_rslots, make_items_paged, part_rchunks
 //   join          radix_join_items: persistent, work-stealing build + probe
 // The fan-out 2^bits is chosen so an R partition fills about one CTA's
-// shared-memory table (17408 tuples).
+// shared-memory table (8704 tuples).
 #include "joins.cuh"
 #include "paged.cuh"
 #include "radix_join.cuh"
 
 namespace adb {
 
-// CTAs of a flat pass: one per tile up to the CTAs resident at once.
-static int flat_ctas(uint64_t nR, uint64_t nS, int num_sms, uint32_t /*F*/) {
-    const uint64_t n = nR > nS ? nR : nS;
-    const uint64_t cap = (uint64_t)num_sms * kPassMinBlocks;
-    uint64_t g = (n + kPTile - 1) / kPTile;
-    if (g < 1) g = 1;
-    if (g > cap) g = cap;
-    return (int)g;
+// CTAs of a flat pass, split over the relations by size, at most one per tile.
+// Every (CTA, digit) stream ends in a partial page, which the join reads and
+// copies like a full one, so smaller inputs get one wave of resident CTAs
+// (2^22 x 2^22, 512 digits: pass 87 -> 79 us, join kernel 122 -> 60 us against two
+// waves, whose pages are half empty and overfill the join's R chunks).  From
+// 2^27 tuples on the partial pages no longer count and a second wave evens out
+// skewed digits (2^27 x 2^27, pass 1: theta 0 1.057 -> 1.046 ms, theta 1.5 1.154 ->
+// 1.088 ms).
+static void flat_ctas(uint64_t nR, uint64_t nS, int num_sms, int G[2]) {
+    const uint64_t all = (uint64_t)num_sms * kPassMinBlocks * (nR + nS >= (1ull << 27) ? 2 : 1);
+    const uint64_t n[2] = {nR, nS};
+    for (int r = 0; r < 2; r++) {
+        uint64_t g = nR + nS ? (all * n[r] + (nR + nS) / 2) / (nR + nS) : 1;
+        const uint64_t tiles = (n[r] + kPTile - 1) / kPTile;
+        if (g > tiles) g = tiles;
+        G[r] = (int)(g < 1 ? 1 : g);
+    }
 }
 
 // Launches one partition pass (both relations: grid.y = relation).
@@ -36,14 +45,14 @@ static void launch_pass(const PassArgs &a, uint32_t F, int G, bool paged, cudaSt
 }
 
 int radix_bits_for(uint64_t nR, int requested) {
-    if (requested > 0) return requested > 14 ? 14 : requested;
+    if (requested > 0) return requested > 15 ? 15 : requested;
     // one pass (<= 9 bits) leaves up to one partial page per CTA in every
     // partition, so it aims at half a join chunk; two passes at a full chunk
     constexpr uint64_t kTarget = kRSlots >= 16384 ? 16384 : 8192;   // power of two <= kRSlots
     int b = (int)ceil_log2_u64((nR + kTarget / 2 - 1) / (kTarget / 2));
     if (b > (int)kMaxPassBits) b = (int)ceil_log2_u64((nR + kTarget - 1) / kTarget);
     if (b < 1) b = 1;
-    if (b > 14) b = 14;
+    if (b > 15) b = 15;
     return b;
 }
 
@@ -53,7 +62,8 @@ int radix_bits_for(uint64_t nR, int requested) {
 struct PartPlan {
     int passes;
     uint32_t F1, F2, Fout;
-    int G1, G2;
+    int g1[2];                 // pass 1: CTAs of R, S
+    int G1, G2;                // CTAs per relation (pass 1: the larger of g1)
     uint32_t pool1, pool2;
     uint32_t unit_pages;       // pass-2 work unit
     uint64_t pages1, pages2;   // pool pages per relation
@@ -65,8 +75,9 @@ static PartPlan plan_partition(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b
     p.F1 = 1u << b1;
     p.F2 = b2 ? 1u << b2 : 1u;
     p.Fout = p.F1 * p.F2;
-    p.G1 = flat_ctas(nR, nS, num_sms, p.F1);
-    const uint32_t a = flat_pool_cap(nR, p.G1, p.F1), b = flat_pool_cap(nS, p.G1, p.F1);
+    flat_ctas(nR, nS, num_sms, p.g1);
+    p.G1 = p.g1[0] > p.g1[1] ? p.g1[0] : p.g1[1];
+    const uint32_t a = flat_pool_cap(nR, p.g1[0], p.F1), b = flat_pool_cap(nS, p.g1[1], p.F1);
     p.pool1 = a > b ? a : b;
     p.pages1 = (uint64_t)p.G1 * p.pool1;
     if (b2) {
@@ -128,6 +139,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     for (int r = 0; r < 2; r++) {
         a1.in[r].in = r ? j.S : j.R;
         a1.in[r].n = r ? j.nS : j.nR;
+        a1.in[r].G = p.g1[r];
         take_pageset(ctx, a1.out[r], p.pages1, p.G1);
     }
     a1.df = d1;
@@ -230,7 +242,7 @@ size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms) {
            Workspace::need(2, 4);
 }
 
-int run_radix(Context *ctx, const DevJoin &j, bool hist_table, int bits, unsigned long long *acc) {
+int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc) {
     cudaStream_t st = ctx->stream;
     uint32_t b1, b2;
     split_bits(bits, &b1, &b2);
@@ -267,10 +279,8 @@ int run_radix(Context *ctx, const DevJoin &j, bool hist_table, int bits, unsigne
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;
     a.wbase = nullptr; a.wbits = nullptr; a.nwin = 0; a.wacc = nullptr;
     const int grid = ctx->num_sms * kJoinMinBlocks;
-    if (hist_table)
-        radix_join_items<TableKind::Hist><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
-    else
-        radix_join_items<TableKind::Chain><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    if (j.mat) radix_join_items<true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    else radix_join_items<false><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
     ADB_CK(cudaGetLastError());
     ctx->kernels += 4;
     return ADB_OK;
@@ -283,9 +293,9 @@ int radix_set_attrs() {
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem(1u << kMaxPassBits, false)));
     ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)pass_smem(1u << kMaxPassBits, true)));
-    ADB_CK(cudaFuncSetAttribute(radix_join_items<TableKind::Chain>,
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<false>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
-    ADB_CK(cudaFuncSetAttribute(radix_join_items<TableKind::Hist>,
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<true>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
     return ADB_OK;
 }

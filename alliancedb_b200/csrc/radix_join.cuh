@@ -3,16 +3,16 @@
 // Replaces, per partition pair (R_p, S_p) produced by paged.cuh:
 //   bucket_chaining_join   hashing/joins/parallel_radix_join.cpp:291-354   (PRO, RJ_st)
 //   histogram_join         hashing/joins/parallel_radix_join.cpp:373-432   (PRH, PRHO)
+// (one chained table for all four: a histogram table, built with two passes
+// over R and a scan, took 0.35 ms where the chained one took 0.15 at 2^24)
 // and the task-queue loop of prj_thread (:1409-1416) with a persistent kernel
 // that takes work items from a global counter (work stealing).  A work item is
 // (partition p, R chunk, S chunk): an R chunk is a run of R_p's pages packed
-// greedily up to kRSlots tuples (part_rchunks), copied into shared memory with
-// one bulk async copy per page
-// (cp.async.bulk global->shared, completion counted on an mbarrier), the table
-// is built there, and up to kSPages pages of S_p are streamed from global
-// memory and probed, one warp per page.  Large R partitions (duplicate or
-// skewed build keys, or |R| beyond 2^12 * 16K) take several R chunks; large S
-// partitions (skewed probe keys) several S chunks.
+// greedily up to kRSlots tuples (part_rchunks), read page by page and linked
+// into a chained table in shared memory, and up to kSPages pages of S_p are
+// streamed from global memory and probed, one warp per page.  Large R
+// partitions (duplicate or skewed build keys, or |R| beyond 2^15 * 8K) take
+// several R chunks; large S partitions (skewed probe keys) several S chunks.
 #pragma once
 
 #include "adb_common.cuh"
@@ -20,16 +20,15 @@
 
 namespace adb {
 
-constexpr int kJoinThreads = 1024;
-constexpr int kJoinMinBlocks = 1;                          // CTAs per SM
-constexpr uint32_t kRSlots = 17408;                        // R tuples a CTA holds (136 KB)
+constexpr int kJoinThreads = 512;
+constexpr int kJoinMinBlocks = 2;                          // CTAs per SM: one's copies and build hide behind the other's probe
+constexpr uint32_t kRSlots = 8704;                         // R tuples a CTA holds (68 KB)
 constexpr uint32_t kChunkW = kRSlots - kPageTuples;        // chunk weight budget
 constexpr uint32_t kMinPageW = 32;                         // weight floor of a page
 constexpr uint32_t kRMaxPages = kChunkW / kMinPageW + 16;  // pages of one R chunk (bound)
 constexpr int kProbeWarps = kJoinThreads / 32 - 1;        // the last warp is the control warp
 constexpr uint32_t kSPages = kProbeWarps * 32;             // S pages per item: <= 32 per probing warp (one per lane)
-constexpr uint32_t kMaxHeads = kRSlots >= 16384 ? 8192 : 4096;   // Chain: bucket heads (~2 slots each)
-constexpr uint32_t kMaxHist = kMaxHeads / 4;               // Hist: buckets
+constexpr uint32_t kMaxHeadsLog2 = 13;                     // bucket heads: one per slot up to 2^13
 
 __device__ __forceinline__ uint32_t page_weight(uint32_t cnt) {
     const uint32_t e = (cnt + 1) & ~1u;                    // slots a page occupies (16-byte copies)
@@ -225,21 +224,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase) {
     return false;
 }
 
-enum class TableKind { Chain = 0, Hist = 1 };
-
-// Shared memory: tup[kRSlots] u64 | aux[kRSlots] u16 | X | two page tables
-// {pg[kRMaxPages + 1] u32, dst << 8 | count [kRMaxPages + 1] u32} | mbarrier,
-// reduction, two item records and scan scratch.
-// X holds the Chain heads (kMaxHeads u32) or the Hist permutation (kRSlots u16)
-// followed by its bucket starts (kMaxHist + 2 u32).
-constexpr size_t kXBytes = ((size_t)kRSlots * 2 + ((size_t)kMaxHist + 2) * 4) > (size_t)kMaxHeads * 4
-                               ? ((size_t)kRSlots * 2 + ((size_t)kMaxHist + 2) * 4 + 15) & ~(size_t)15
-                               : (size_t)kMaxHeads * 4;
+// Shared memory: tup[kRSlots] u64 | heads[2^kMaxHeadsLog2] u32 | two page tables
+// {pg[kRMaxPages + 1] u32, dst << 8 | count [kRMaxPages + 1] u32} | reduction and
+// two item records.
 constexpr size_t kPageTabBytes = ((size_t)kRMaxPages + 1) * 4 * 2;
-constexpr size_t kJoinSmem = (size_t)kRSlots * 8 + (size_t)kRSlots * 2 + kXBytes + 2 * kPageTabBytes + 1024;
-static_assert(((size_t)kRSlots * 10 + kXBytes + 2 * kPageTabBytes) % 8 == 0, "mbarrier must be 8-byte aligned");
+constexpr size_t kJoinSmem = (size_t)kRSlots * 8 + ((size_t)4 << kMaxHeadsLog2) + 2 * kPageTabBytes + 1024;
+static_assert(((size_t)kRSlots * 8 + 2 * kPageTabBytes) % 8 == 0, "reduction words must be 8-byte aligned");
 static_assert(kJoinMinBlocks * (kJoinSmem + 1024) <= 233472, "join CTAs exceed the SM's shared memory");
-static_assert(kRSlots < (1u << 24) && kRMaxPages < (uint32_t)kJoinThreads, "page table packing");
+static_assert(kRSlots <= (2u << kMaxHeadsLog2), "a slot index must fit the key bits a bucket shares");
 
 struct JoinArgs {
     const uint64_t *Rpages, *Spages;
@@ -253,7 +245,7 @@ struct JoinArgs {
     uint32_t *work_counter;
     unsigned long long *acc;         // [0] count, [1] checksum
     int *err;
-    int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report completed waits as run out
+    int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report a wait that ran out
     uint32_t F;
     uint32_t bits;                   // bits the partitioning consumed (the hash skips them)
     uint64_t *mat;                   // optional <S-key, S-payload> output
@@ -272,7 +264,8 @@ struct ItemRec {
     uint64_t rb, sb;          // first page-list index of the R chunk / S chunk
     uint32_t item, p, win;    // item (>= n_items: none), partition, window
     uint32_t nrpg, nspg;      // pages of the R chunk / S chunk
-    uint32_t rslots;          // R chunk slots in shared memory (pages rounded up to even counts)
+    uint32_t lnb;             // log2 of the bucket heads: one per slot of the R chunk (pages rounded up to even counts)
+    uint32_t shift;           // key bits the partitioning consumed
 };
 
 // The items of one CTA form a pipeline run by its last warp (the control
@@ -281,25 +274,37 @@ struct ItemRec {
 //   i + 1 (page ids, 16-byte aligned shared-memory destinations) and takes
 //   item i + 2 from the work counter; the probing warps load their S page ids
 //   of item i + 1.
-// Per item: one bulk async copy per R page (cp.async.bulk global -> shared,
-// completion counted on an mbarrier with a bounded wait), the table build by
-// all warps, then the probe by warps 0 .. kProbeWarps - 1, each holding two S
+// Per item: the table build by all warps (a page per warp, kB pages' loads in
+// flight), then the probe by warps 0 .. kProbeWarps - 1, each holding two S
 // pages in flight ahead of the one it probes.
-template <TableKind K>
+//
+// The table: bucket heads indexed by the lnb key bits above the b bits the
+// partitioning consumed, one head per R slot (up to 2^13), and chains through
+// the tuples themselves.  All keys of a bucket share their low b + lnb bits,
+// so a linked tuple's key holds the next slot of its chain there (its own
+// slot: the end); the bits above stay for the comparison.  One 8-byte read per
+// visited tuple gives payload, comparison bits and link.
+//
+// Bound: instruction issue and the ALU pipe (60 % busy), not DRAM.  |R| = |S| =
+// 2^27, ms: one 1024-thread CTA per SM with two slots per head, separate next
+// array and bulk-copied pages 1.05 dense keys / 1.74 keys spread over 32 bits;
+// this form 0.76 / 1.34 (two CTAs, so that one builds while the other probes:
+// -0.08 / -0.05; one head per slot and links in the tuples: -0.13 / -0.5; pages
+// read straight into the build, without the copy's per-page issue cost of
+// about 58 cycles and its wait: -0.03; the probe's half of the checksum before
+// the walk: -0.05 / -0.07).  Batched windows (512, 2^10 .. 2^22 tuples): the
+// whole call 7.86 -> 6.01 ms.  Adding a warp's matches together after the walk
+// instead of as they are found: 0.83 / 1.14, and 1.27 instead of 1.23 ms with
+// every key four times in both relations (2^26), so not kept.
+template <bool kMat>
 __global__ void __launch_bounds__(kJoinThreads, kJoinMinBlocks)
 radix_join_items(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t *tup = reinterpret_cast<uint64_t *>(smem);
-    uint16_t *aux = reinterpret_cast<uint16_t *>(tup + kRSlots);        // next[] (Chain) / rank (Hist)
-    unsigned char *xr = reinterpret_cast<unsigned char *>(aux + kRSlots);
-    uint16_t *perm = reinterpret_cast<uint16_t *>(xr);                   // Hist: bucket-ordered slots
-    uint32_t *heads = K == TableKind::Chain ? reinterpret_cast<uint32_t *>(xr)      // Chain: heads
-                                            : reinterpret_cast<uint32_t *>(perm + kRSlots);  // Hist: starts
-    uint32_t *ptab = reinterpret_cast<uint32_t *>(xr + kXBytes);         // [2] x {pg[], dst << 8 | cnt []}
-    uint64_t *bar = reinterpret_cast<uint64_t *>(ptab + 4 * (kRMaxPages + 1));
-    uint64_t *red = bar + 2;
+    uint32_t *heads = reinterpret_cast<uint32_t *>(tup + kRSlots);
+    uint32_t *ptab = heads + (1u << kMaxHeadsLog2);                      // [2] x {pg[], dst << 8 | cnt []}
+    uint64_t *red = reinterpret_cast<uint64_t *>(ptab + 4 * (kRMaxPages + 1));
     ItemRec *rec = reinterpret_cast<ItemRec *>(red + 64);                // [2]
-    uint32_t *scan = reinterpret_cast<uint32_t *>(rec + 2);              // 32 u32
 
     const uint32_t n_items = *a.n_items;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -323,6 +328,7 @@ radix_join_items(JoinArgs a) {
                 const ItemGeo g = item_geo(a, item, p, kSPages);
                 r->p = p;
                 r->win = w;
+                r->shift = a.wacc ? a.wbits[w] : a.bits;
                 r->rb = g.rb;
                 r->sb = g.sb;
                 r->nrpg = g.nrpg;
@@ -331,11 +337,7 @@ radix_join_items(JoinArgs a) {
         }
         __syncwarp();
     };
-    // control warp: page table of item r (page ids, packed destination and
-    // count) and the mbarrier's expected bytes for its copies.  (No bulk L2
-    // prefetch of the pages: one cp.async.bulk.prefetch per 512-byte page
-    // occupies the SM's bulk-copy unit for tens of cycles and delays the
-    // item's own copies.)
+    // control warp: page table of item r (page ids, packed destination and count)
     auto table = [&](ItemRec *r, uint32_t *pt) {
         if (r->item >= n_items) return;
         const uint64_t rb = r->rb;
@@ -365,16 +367,12 @@ radix_join_items(JoinArgs a) {
             }
         }
         if (lane == 0) {
-            r->rslots = carry;
-            // the item's copies are issued after the next barrier; the barrier
-            // is in the item's phase already (the previous item's copies landed)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(bar, carry * 8);
+            uint32_t l = carry > 1 ? 32u - __clz(carry - 1) : 0u;
+            r->lnb = l < kMaxHeadsLog2 ? l : kMaxHeadsLog2;
         }
         __syncwarp();
     };
 
-    if (threadIdx.x == 0) mbar_init(bar, 1);
     if (warp == kCtl) {
         take(&rec[0]);
         table(&rec[0], ptab);
@@ -382,22 +380,21 @@ radix_join_items(JoinArgs a) {
     }
     __syncthreads();
 
-    // S page ids of a probing warp for item r: lane i holds page warp + kProbeWarps * i
-    auto s_ids = [&](const ItemRec &r, uint32_t &pg, uint32_t &cnt) {
-        pg = 0;
-        cnt = 0;
+    // S pages of a probing warp for item r: lane i holds page warp + kProbeWarps * i
+    // as id << 6 | count - 1 (kNone: no page)
+    auto s_ids = [&](const ItemRec &r) {
+        uint32_t v = kNone;
         if (warp < kProbeWarps && r.item < n_items) {
             const uint32_t i = (uint32_t)warp + (uint32_t)kProbeWarps * lane;
             if (i < r.nspg) {
-                pg = a.Slist[r.sb + i];
-                cnt = a.Scount[pg];
+                const uint32_t pg = a.Slist[r.sb + i];
+                v = pg << 6 | (a.Scount[pg] - 1u);
             }
         }
+        return v;
     };
-    uint32_t my_pg, my_cnt;
-    s_ids(rec[0], my_pg, my_cnt);
+    uint32_t my_pg = s_ids(rec[0]);
 
-    uint32_t phase = 0;
     int cur = 0;
     Acc acc;
     while (true) {
@@ -405,157 +402,106 @@ radix_join_items(JoinArgs a) {
         if (C.item >= n_items) break;
         const uint32_t *tpg = ptab + cur * 2 * (kRMaxPages + 1);
         const uint32_t *tpk = tpg + kRMaxPages + 1;
-        const uint32_t shift = a.wacc ? a.wbits[C.win] : a.bits;
+        const uint32_t shift = C.shift;
         const uint32_t nrpg = C.nrpg, nspg = C.nspg;
 
-        // --- R chunk: one bulk copy per page from the page table (the
-        //     control warp announced the bytes when it built the table)
-        for (uint32_t k = threadIdx.x; k < nrpg; k += blockDim.x) {
-            const uint32_t v = tpk[k], cnt = v & 0xFFu;
-            if (cnt) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                bulk_g2s(tup + (v >> 8), a.Rpages + (uint64_t)tpg[k] * kPageTuples, ((cnt + 1) & ~1u) * 8, bar);
-            }
-        }
-
-        // --- the probing warp's first two S pages (ids loaded during the previous item)
+        // --- the probing warp's first two S pages (ids loaded during the
+        //     previous item): lane l holds tuples 2l, 2l + 1 of a page, cn the
+        //     page's count (0: none)
         const uint32_t npw = warp < kProbeWarps && (uint32_t)warp < nspg
                                  ? (nspg - warp + kProbeWarps - 1) / kProbeWarps : 0u;
-        auto load_page = [&](uint32_t i, uint64_t &x0, uint64_t &x1, uint32_t &cn) {
-            const uint32_t pgi = __shfl_sync(0xffffffffu, my_pg, i & 31);
-            cn = __shfl_sync(0xffffffffu, my_cnt, i & 31);
-            if (i >= npw) cn = 0;
-            const uint64_t *Sp = a.Spages + (uint64_t)pgi * kPageTuples;
-            x0 = lane < (int)cn ? ld_stream(Sp + lane) : 0;
-            x1 = lane + 32 < (int)cn ? ld_stream(Sp + lane + 32) : 0;
+        auto load_page = [&](uint32_t i, ulonglong2 &x, uint32_t &cn) {
+            const uint32_t v = __shfl_sync(0xffffffffu, my_pg, i & 31);
+            cn = i < npw ? (v & 63u) + 1u : 0u;
+            // an odd page's pad word is read with its last tuple
+            if (2 * lane < (int)cn)
+                x = __ldcs(reinterpret_cast<const ulonglong2 *>(a.Spages + (uint64_t)(v >> 6) * kPageTuples) + lane);
         };
-        uint64_t c0 = 0, c1 = 0, n0 = 0, n1 = 0;
-        uint32_t ccnt = 0, ncnt = 0;
+        ulonglong2 x0 = make_ulonglong2(0, 0), x1 = x0, x2 = x0;
+        uint32_t n0 = 0, n1 = 0, n2 = 0;
         if (warp < kProbeWarps) {
-            load_page(0, c0, c1, ccnt);
-            load_page(1, n0, n1, ncnt);
+            load_page(0, x0, n0);
+            load_page(1, x1, n1);
         }
 
-        uint32_t nb = 1;
-        while (nb < C.rslots) nb <<= 1;
-        if (K == TableKind::Chain) {
-            nb >>= 1;                                  // about two slots per head
-            if (nb > kMaxHeads) nb = kMaxHeads;
-        } else {
-            nb >>= 2;                                  // get_hist_size: |R_i| / 4 buckets
-            if (nb > kMaxHist) nb = kMaxHist;
-        }
-        if (nb < 1) nb = 1;
-        const uint32_t bmask = nb - 1;
-        for (uint32_t i = threadIdx.x; i < nb + 2; i += blockDim.x) heads[i] = 0;
-        if (!mbar_wait(bar, phase) || a.waits_run_out) atomicExch(a.err, 1);
-        phase ^= 1;
+        const uint32_t lnb = C.lnb;
+        const uint32_t bmask = (1u << lnb) - 1;
+        const uint32_t lim = 1u << (shift + lnb), lmask = lim - 1;   // link bits of a linked key
+        for (uint32_t i = threadIdx.x; i < ((1u << lnb) + 3) / 4; i += kJoinThreads)
+            reinterpret_cast<uint4 *>(heads)[i] = make_uint4(kNone, kNone, kNone, kNone);
+        if (a.waits_run_out && threadIdx.x == 0) atomicExch(a.err, 1);
         __syncthreads();
 
-        // --- build (warp per page, two tuples per lane)
-        if (K == TableKind::Chain) {
-            for (uint32_t k = warp; k < nrpg; k += kWarps) {
-                const uint32_t v = tpk[k], c = v & 0xFFu, base = v >> 8;
-                for (uint32_t l = lane; l < c; l += 32) {
-                    const uint32_t s = base + l;
-                    const uint32_t h = (tkey(tup[s]) >> shift) & bmask;
-                    aux[s] = (uint16_t)atomicExch(&heads[h], s + 1);
+        // --- build: a warp per page, two tuples per lane, kB pages in flight
+        auto link = [&](uint32_t s, uint64_t t) {
+            const uint32_t old = atomicExch(&heads[(tkey(t) >> shift) & bmask], s);
+            return tword((tkey(t) & ~lmask) | (old == kNone ? s : old), tpay(t));
+        };
+        constexpr int kB = 4;
+        for (uint32_t k0 = warp; k0 < nrpg; k0 += kB * kWarps) {
+            ulonglong2 r[kB];
+            uint32_t v[kB];
+#pragma unroll
+            for (int j = 0; j < kB; j++) {
+                const uint32_t k = k0 + j * kWarps;
+                v[j] = k < nrpg ? tpk[k] : 0u;
+                if (2 * lane < (int)(v[j] & 0xFFu))
+                    r[j] = __ldcs(reinterpret_cast<const ulonglong2 *>(a.Rpages + (uint64_t)tpg[k] * kPageTuples) + lane);
+            }
+#pragma unroll
+            for (int j = 0; j < kB; j++) {
+                const uint32_t s = (v[j] >> 8) + 2 * lane;
+                if (2 * lane < (int)(v[j] & 0xFFu)) {
+                    r[j].x = link(s, r[j].x);
+                    if (2 * lane + 1 < (int)(v[j] & 0xFFu)) r[j].y = link(s + 1, r[j].y);
+                    *reinterpret_cast<ulonglong2 *>(tup + s) = r[j];
                 }
             }
-            __syncthreads();
-        } else {
-            for (uint32_t k = warp; k < nrpg; k += kWarps) {
-                const uint32_t v = tpk[k], c = v & 0xFFu, base = v >> 8;
-                for (uint32_t l = lane; l < c; l += 32) {
-                    const uint32_t s = base + l;
-                    const uint32_t h = (tkey(tup[s]) >> shift) & bmask;
-                    aux[s] = (uint16_t)atomicAdd(&heads[h + 1], 1u);
-                }
-            }
-            __syncthreads();
-            {   // bucket starts: heads[h + 1] = start of bucket h, heads[nb + 1] = total
-                const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
-                const uint32_t d0 = threadIdx.x * per, d1 = min(nb, d0 + per);
-                uint32_t loc = 0;
-                for (uint32_t d = d0; d < d1; d++) loc += heads[d + 1];
-                uint32_t tot;
-                uint32_t ex = block_exclusive_scan(loc, scan, &tot);
-                for (uint32_t d = d0; d < d1; d++) {
-                    const uint32_t c = heads[d + 1];
-                    heads[d + 1] = ex;
-                    ex += c;
-                }
-                __syncthreads();
-                if (threadIdx.x == 0) heads[nb + 1] = tot;
-            }
-            __syncthreads();
-            for (uint32_t k = warp; k < nrpg; k += kWarps) {
-                const uint32_t v = tpk[k], c = v & 0xFFu, base = v >> 8;
-                for (uint32_t l = lane; l < c; l += 32) {
-                    const uint32_t s = base + l;
-                    const uint32_t h = (tkey(tup[s]) >> shift) & bmask;
-                    perm[heads[h + 1] + aux[s]] = (uint16_t)s;
-                }
-            }
-            __syncthreads();
         }
+        __syncthreads();
 
         if (warp == kCtl) {
-            // the next item's page table and prefetches, then the item after it
-            // (rec[cur] is free: every thread copied it before the barriers above)
+            // the next item's page table, then the item after it (rec[cur] is
+            // free: every thread copied it before the barriers above)
             table(&rec[cur ^ 1], ptab + (cur ^ 1) * 2 * (kRMaxPages + 1));
             take(&rec[cur]);
         } else {
             // the next item's S page ids, in flight during this probe
-            uint32_t nx_pg, nx_cnt;
-            s_ids(rec[cur ^ 1], nx_pg, nx_cnt);
-            // --- probe; page i + 2 is loaded before page i is probed
-            for (uint32_t i = 0; i < npw; i++) {
-                uint64_t m0 = 0, m1 = 0;
-                uint32_t mcnt = 0;
-                if (i + 2 < npw) load_page(i + 2, m0, m1, mcnt);
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    if (lane + 32 * half >= (int)ccnt) continue;
-                    const uint64_t s = half ? c1 : c0;
-                    const uint32_t key = tkey(s);
-                    const uint32_t h = (key >> shift) & bmask;
-                    uint64_t sh = 0;
-                    bool have_sh = false;
-                    if (K == TableKind::Chain) {
-                        for (uint32_t hit = heads[h]; hit; hit = aux[hit - 1]) {
-                            const uint64_t r = tup[hit - 1];
-                            if (tkey(r) == key) {
-                                if (!have_sh) { sh = s_half(key, tpay(s)); have_sh = true; }
-                                acc.count++;
-                                acc.sum += pair_hash_pre(key, tpay(r), sh);
-                                if (a.mat) {
-                                    const unsigned long long m = atomicAdd(a.mat_n, 1ull);
-                                    if (m < a.mat_cap) a.mat[m] = s;
-                                }
-                            }
-                        }
-                    } else {
-                        const uint32_t e = heads[h + 2];
-                        for (uint32_t t = heads[h + 1]; t < e; t++) {
-                            const uint64_t r = tup[perm[t]];
-                            if (tkey(r) == key) {
-                                if (!have_sh) { sh = s_half(key, tpay(s)); have_sh = true; }
-                                acc.count++;
-                                acc.sum += pair_hash_pre(key, tpay(r), sh);
-                                if (a.mat) {
-                                    const unsigned long long m = atomicAdd(a.mat_n, 1ull);
-                                    if (m < a.mat_cap) a.mat[m] = s;
-                                }
-                            }
+            const uint32_t nx_pg = s_ids(rec[cur ^ 1]);
+            uint32_t matches = 0;
+            auto probe = [&](uint64_t s) {
+                const uint32_t key = tkey(s);
+                uint32_t at = heads[(key >> shift) & bmask];
+                if (at == kNone) return;
+                const uint64_t sh = s_half(key, tpay(s));
+                while (true) {
+                    const uint64_t r = tup[at];
+                    const uint32_t nx = tkey(r) & lmask;
+                    if ((tkey(r) ^ key) < lim) {
+                        
+                        acc.sum += pair_hash_pre(key, tpay(r), sh);
+                        matches++;
+                        if (kMat) {
+                            const unsigned long long m = atomicAdd(a.mat_n, 1ull);
+                            if (m < a.mat_cap) a.mat[m] = s;
                         }
                     }
+                    if (nx == at) break;
+                    at = nx;
                 }
-                c0 = n0; c1 = n1; ccnt = ncnt;
-                n0 = m0; n1 = m1; ncnt = mcnt;
+            };
+            for (uint32_t i = 0; i < npw; i++) {
+                n2 = 0;
+                if (i + 2 < npw) load_page(i + 2, x2, n2);
+                if (2 * lane < (int)n0) probe(x0.x);
+                __syncwarp();
+                if (2 * lane + 1 < (int)n0) probe(x0.y);
+                __syncwarp();
+                x0 = x1; n0 = n1;
+                x1 = x2; n1 = n2;
             }
+            acc.count += matches;
             my_pg = nx_pg;
-            my_cnt = nx_cnt;
         }
         if (a.wacc) {   // batched windows: this item's sums to its window
             block_flush(acc, a.wacc + 2 * C.win, red);

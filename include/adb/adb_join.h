@@ -84,10 +84,10 @@ typedef struct adb_join_params {
     uint64_t seed;              /* JBCR's random split of S */
     int32_t realtime;           /* adb_stream_join: 1 = release each micro-batch at its timestamp
                                    (wall clock, the reference's WAIT gating, fetcher.cpp:120-190) */
-    int32_t test_flags;         /* 0 in normal use.  ADB_TEST_WAITS_RUN_OUT: every bounded device wait
-                                   of the partitioned and sort-merge joins, once it has completed,
-                                   reports that it ran out, so callers can test their ADB_ERR_TIMEOUT
-                                   handling without making a GPU wait for real */
+    int32_t test_flags;         /* 0 in normal use.  ADB_TEST_WAITS_RUN_OUT: the partitioned and
+                                   sort-merge joins do their work and then report that a bounded device
+                                   wait ran out, so callers can test their ADB_ERR_TIMEOUT handling
+                                   without making a GPU wait for real */
 } adb_join_params;
 
 #define ADB_TEST_WAITS_RUN_OUT 1
