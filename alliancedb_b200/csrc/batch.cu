@@ -275,10 +275,8 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ADB_CK(cudaMemsetAsync(tot, 0, (2ull * Dt + 2) * 4, st));
     ADB_CK(cudaMemsetAsync(fill, 0, (2ull * Dt + 2) * 4, st));
     ADB_CK(cudaMemsetAsync(ctr, 0, 8, st));
-    ADB_CK(cudaEventRecord(ctx->ev[0], st));
     partition_pass<2, kPassThreads><<<dim3(G, 2), kPassThreads, pass_smem(1u << kMaxPassBits, false), st>>>(a);
     ADB_CK(cudaGetLastError());
-    ADB_CK(cudaEventRecord(ctx->ev[1], st));
     dscan<uint64_t>(st, tot, Dt, pstart, bsum64);
     dscan<uint64_t>(st, tot + Dt, Dt, pstart + (Dt + 1), bsum64);
     page_place_atomic<<<dim3(G, 2), 256, 0, st>>>(a, fill, fill + Dt);
@@ -291,7 +289,6 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     part_rchunks<<<(Dt + 7) / 8, 256, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, kChunkW, chunk_off,
                                               cstart);
     ADB_CK(cudaGetLastError());
-    ADB_CK(cudaEventRecord(ctx->ev[2], st));
     JoinArgs ja;
     ja.Rpages = a.out[0].pages; ja.Spages = a.out[1].pages;
     ja.Rcount = a.out[0].pcount; ja.Scount = a.out[1].pcount;
@@ -307,7 +304,6 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ja.wbase = d_wbase; ja.wbits = d_bits; ja.nwin = W; ja.wacc = wacc;
     radix_join_items<false><<<ctx->num_sms * kJoinMinBlocks, kJoinThreads, kJoinSmem, st>>>(ja);
     ADB_CK(cudaGetLastError());
-    ADB_CK(cudaEventRecord(ctx->ev[3], st));
     ctx->kernels += 14;
     ADB_CK(cudaMemcpyAsync(h_out, wacc, (2 * W + 8) * 8, cudaMemcpyDeviceToHost, st));
     return ADB_OK;

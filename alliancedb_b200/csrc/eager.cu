@@ -475,9 +475,7 @@ int run_eager(Context *ctx, const DevJoin &j, Family fam, int model, uint64_t ba
     EagerWindow w;
     take_window(ctx, p, w, seed);
     ADB_TRY(reset_window(ctx, p, w));
-    ADB_CK(cudaEventRecord(ctx->ev[1], ctx->stream));
-    ADB_CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    ADB_CK(cudaEventRecord(ctx->ev[3], ctx->stream));
+    ADB_CK(mark(ctx, 1));
     if (fam == Family::Shj)   // arrival order = micro-batch order; no real-time release
         return eager_window_throughput(ctx, p, w, j.R, j.nR, j.S, j.nS, 1, sr, ss, acc);
     for (uint64_t k = 0; k < runs; k++) {

@@ -73,6 +73,8 @@ struct Context {
     cudaEvent_t ev[12] = {};
     Workspace ws;
     unsigned long long *h_res = nullptr;   // pinned: [0] count [1] checksum [2] err [3] mat_n ...
+    unsigned long long *d_small = nullptr; // device accumulators of the single-launch joins, 0 between calls
+    unsigned marks = 0;                    // phase events recorded by the current call (bit k: ev[k])
     // pinned, grow-only host buffers of the batched path: the per-call plan (one
     // host -> device copy) and the per-window results (one copy back); growing
     // one needs its previous use finished
@@ -102,6 +104,12 @@ struct CtxLock {
     std::unique_lock<std::recursive_mutex> lk;
 };
 CtxLock ctx_acquire(int *status);
+
+// Records phase event k (1 .. 3) of the current call on its stream.
+inline cudaError_t mark(Context *ctx, int k) {
+    ctx->marks |= 1u << k;
+    return cudaEventRecord(ctx->ev[k], ctx->stream);
+}
 
 // The per-device context (created on first use).  Returns nullptr and sets
 // the error if no device is usable.

@@ -33,6 +33,10 @@ uint64_t paged_final_pool_pages(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t 
 int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitFn *d2, PartOut *out,
                         unsigned long long *acc);
 
+// ---- hash joins of a small build side, small.cu ----
+bool small_fits(uint64_t nR, uint64_t nS);
+int run_small(Context *ctx, const DevJoin &j);
+
 // ---- radix (PRO / RJ_st / PRH / PRHO) ----
 int radix_bits_for(uint64_t nR, int requested);
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);

@@ -212,7 +212,6 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
     const uint32_t rb = npo_region_bits(j.nR, region_bits);
     PartOut po{};
     if (rb) ADB_TRY(run_paged_partition(ctx, j, DigitFn{32u - rb, (1u << rb) - 1u, true}, nullptr, &po, acc));
-    ADB_CK(cudaEventRecord(ctx->ev[1], st));
     uint64_t *table = ctx->ws.take<uint64_t>(1ULL << l2);
     unsigned long long *sent = ctx->ws.take<unsigned long long>(1);
     ADB_CK(cudaMemsetAsync(table, 0xFF, (1ULL << l2) * 8, st));
@@ -232,8 +231,7 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
         nb = nb < 1 ? 1 : nb;
         np = np < 1 ? 1 : np;
         npo_build_pages<<<ctx->num_sms * nb, kNpoThreads, 0, st>>>(PR, table, l2, rb, sent, err);
-        ADB_CK(cudaEventRecord(ctx->ev[2], st));
-        ADB_CK(cudaEventRecord(ctx->ev[3], st));
+        ADB_CK(mark(ctx, 2));
         if (j.mat)
             npo_probe_pages<true><<<ctx->num_sms * np, kNpoThreads, 0, st>>>(PS, table, l2, sent, acc, j.mat,
                                                                               acc + 3, j.mat_cap);
@@ -248,8 +246,7 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
             return (int)(b < 1 ? 1 : (b > cap ? cap : b));
         };
         npo_build<<<blocks(j.nR), threads, 0, st>>>(j.R, j.nR, table, l2, sent, err);
-        ADB_CK(cudaEventRecord(ctx->ev[2], st));
-        ADB_CK(cudaEventRecord(ctx->ev[3], st));
+        ADB_CK(mark(ctx, 2));
         if (j.mat)
             npo_probe<true><<<blocks(j.nS), threads, 0, st>>>(j.S, j.nS, table, l2, sent, acc, j.mat, acc + 3,
                                                               j.mat_cap);

@@ -354,7 +354,7 @@ int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool /*multipass*/,
     const DigitFn d2{b1, (1u << b2) - 1};
     PartOut po;
     ADB_TRY(run_paged_partition(ctx, j, d1, b2 ? &d2 : nullptr, &po, acc));
-    ADB_CK(cudaEventRecord(ctx->ev[1], st));
+    ADB_CK(mark(ctx, 1));
 
     const uint32_t F = po.Fout;
     uint32_t *rch = ctx->ws.take<uint32_t>(F);
@@ -369,8 +369,7 @@ int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool /*multipass*/,
     make_items_paged<<<1, 1024, 0, st>>>(rch, sch, F, items_off, chunk_off, ctr);
     part_rchunks<<<(F + 7) / 8, 256, 0, st>>>(po.pstart, po.R.plist, po.R.pcount, F, kSmjChunkW, chunk_off, cstart);
     ADB_CK(cudaGetLastError());
-    ADB_CK(cudaEventRecord(ctx->ev[2], st));
-    ADB_CK(cudaEventRecord(ctx->ev[3], st));
+    ADB_CK(mark(ctx, 2));
 
     SmjArgs a;
     a.Rpages = po.R.pages; a.Spages = po.S.pages;

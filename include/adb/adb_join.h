@@ -98,7 +98,8 @@ typedef struct adb_join_result {
     int32_t status;             /* adb_status */
     int32_t kernels;            /* kernels this call launched */
     float ms_device;            /* device time of the join, CUDA events on the library stream */
-    float ms_phase[4];          /* device time per phase; radix: partition pass 1, pass 2 (0 with one pass),
+    float ms_phase[4];          /* device time per phase; a small hash join (one launch): all in the last;
+                                   radix: partition pass 1, pass 2 (0 with one pass),
                                    work list, join kernel; NPO: grouping by table region, build, -, probe;
                                    m-way: partitioning,
                                    work list, -, sort + merge-join kernel */
