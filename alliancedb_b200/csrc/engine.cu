@@ -332,7 +332,10 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
         case Family::Radix:
         case Family::RadixHist:
             return radix_scratch(nR, nS, radix_bits_for(nR, p ? p->radix_bits : 0), num_sms);
-        case Family::Npo: return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
+        case Family::Npo:
+            if (npo_partitioned(nR, nS, p ? p->radix_bits : 0))
+                return radix_scratch(nR, nS, radix_bits_for(nR, 0), num_sms);
+            return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
         case Family::SortMerge: return smj_scratch(nR, nS, p ? p->part_fanout : 0, num_sms);
         case Family::Shj:
         case Family::Pmj:
@@ -347,8 +350,11 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), acc);
-        case Family::Npo: return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
+            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), false, acc);
+        case Family::Npo:
+            if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0))
+                return run_radix(ctx, j, radix_bits_for(j.nR, 0), true, acc);
+            return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
         case Family::SortMerge: return run_smj(ctx, j, p ? p->part_fanout : 0, a->model == 1, acc);
         case Family::Shj:
         case Family::Pmj:
@@ -374,8 +380,8 @@ static int join_device_core(Context *ctx, const AlgoEntry *a, DevJoin j, const a
         ADB_TRY(run_small(ctx, j));
         ADB_CK(cudaEventRecord(ctx->ev[6], st));
     } else {
-        unsigned long long *acc = ctx->ws.take<unsigned long long>(4);
-        ADB_CK(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), st));
+        unsigned long long *acc = ctx->ws.take<unsigned long long>(8);
+        ADB_CK(cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st));
         if (j.nR && j.nS) ADB_TRY(dispatch(ctx, a, j, p, acc));
         ADB_CK(cudaEventRecord(ctx->ev[6], st));
         ADB_CK(cudaMemcpyAsync(ctx->h_res, acc, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));

@@ -2,7 +2,8 @@
 // batched/served paths.  Each driver: scratch size for a call, then the
 // launch sequence on ctx->stream.  Results land in acc[0] (count) and acc[1]
 // (checksum) of a device accumulator the caller zeroed; acc[2] is the error
-// word (a timed-out device wait sets it), acc[3] the materialised count.
+// word (a timed-out device wait sets it), acc[3] the materialised count, acc[4]
+// NPO's build tuples equal to its empty marker.
 #pragma once
 
 #include "engine.cuh"
@@ -40,9 +41,10 @@ int run_small(Context *ctx, const DevJoin &j);
 // ---- radix (PRO / RJ_st / PRH / PRHO) ----
 int radix_bits_for(uint64_t nR, int requested);
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
-int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc);
+int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned long long *acc);
 
 // ---- NPO / NPO_st ----
+bool npo_partitioned(uint64_t nR, uint64_t nS, int requested);
 uint32_t npo_region_bits(uint64_t nR, int requested);
 size_t npo_scratch(uint64_t nR, uint64_t nS, int region_bits, int num_sms);
 int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long *acc);

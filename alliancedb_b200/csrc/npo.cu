@@ -3,24 +3,24 @@
 // the table for |R|/BUCKET_SIZE buckets, build with all threads, barrier,
 // probe S chunks).
 //
-// The table is one global open-addressing array of 2^l2 slots (npo_join.cuh),
-// as the reference's is one shared bucket array.  Up to 256 MB (|R| <= 2^24)
-// the join is: clear the table, one build launch, one probe launch over the
-// relations as they are.
+// The table is one global array of four-slot buckets (npo_join.cuh), as the
+// reference's is one shared bucket array: clear it, one build launch, one
+// probe launch over the relations as they are.  That is fast while the table
+// stays in L2; larger build sides go to the partitioned join on hashed digits
+// (npo_partitioned below).
 //
-// A larger table (8 B x 2 |R|: 2 GiB at |R| = 2^27) is 16x the L2, and build
-// and probe in input order would each touch a random DRAM sector per tuple.
-// There the table is cut into 2^rb regions of 2^21 slots (16 MB): region g
+// With a forced region count (radix_bits > 0) the table is an open-addressing
+// array of 2^l2 slots cut into 2^rb regions: region g
 // holds the slots whose index has top bits g, i.e. the keys whose top rb bits
 // of key * kFibMul are g.  One paged partition pass (paged.cuh, hashed digit)
 // groups R and S by region, and build and probe walk the page lists in region
 // order, each warp taking a few adjacent pages at a time and every warp of the
-// grid sweeping the same stretch of the list.  At any time the grid inserts into or probes one or two regions,
-// so the atomics and the sector reads hit L2; in the build each page of
-// region g also prefetches its share of region g + 1's table lines into L2,
-// so the next region arrives by line reads instead of random sector misses.
-// At |R| = |S| = 2^27 this takes NPO from 10.9 ms (build 6.94, probe 3.89)
-// to 4.26 ms (grouping 1.06, build 1.95, probe 1.19).
+// grid sweeping the same stretch of the list.  At any time the grid inserts into
+// or probes one or two regions, so the atomics and the sector reads hit L2; in
+// the build each page of region g also prefetches its share of region g + 1's
+// table lines into L2, so the next region arrives by line reads instead of
+// random sector misses.  At |R| = |S| = 2^27 with 7 bits: 4.26 ms (grouping 1.06,
+// build 1.95, probe 1.19) against 10.9 ms in input order and 3.2 ms partitioned.
 // Matches, count and checksum are the same as in input order.
 #include "joins.cuh"
 #include "npo_join.cuh"
@@ -34,30 +34,37 @@ static uint32_t npo_log2(uint64_t nR) {
     return l < 2 ? 2 : l;
 }
 
-constexpr uint32_t kNpoRegionLog2 = 21;     // slots per table region (16 MB)
-// Tables up to 2^25 slots (256 MB) are not grouped.  Measured (whole join,
-// |R| = |S|, grouped / not): 2^23 0.66 / 0.58 ms, 2^24 2.08 / 1.47 ms,
-// 2^25 1.25 / 2.45 ms, 2^26 2.48 / 5.28 ms, 2^27 4.80 / 10.9 ms.  The grouped
-// build runs at 68-69 G inserts/s from 2^25 up but at 11-23 G/s at 2^23 and
-// 2^24 (tables of 1-2x the L2), whatever the region size; the cause is not
-// known.
-constexpr uint32_t kNpoUngroupedLog2 = 25;
+// Build sides whose table would not stay in L2 are joined by the partitioned
+// join, on digits of key * kFibMul (radix.cu): the same join without a random
+// DRAM access per tuple.  Device time, us, table / partitioned, for keys over 32
+// bits, four of each key on both sides, and dense keys with theta 1:
+//   2^21.8 x 2^21.8  154 / 170    299 / 225    122 / 175
+//   2^22   x 2^22    184 / 190    346 / 253    148 / 199
+//   2^22   x 2^24    336 / 558    818 / 806    238 / 438
+//   2^23   x 2^23    470 / 342    642 / 421    412 / 389
+//   2^24   x 2^24   1210 / 570
+// Up to 2^22 the table still wins against a larger S, whose two extra trips
+// through memory the partitioning would add.
+constexpr uint64_t kNpoTableMax = 7ull << 19;   // 3.67 M tuples, an 88 MB table
+bool npo_partitioned(uint64_t nR, uint64_t nS, int requested) {
+    return requested == 0 && nR > kNpoTableMax && !(nR <= 1ull << 22 && nS >= 2 * nR) &&
+           nR < 1ull << 31 && nS < 1ull << 31;   // the paged passes' slot numbers are 32 bits
+}
 
-// Table-region bits: 0 (no grouping) up to a 256 MB table, else regions of
-// 2^21 slots.  requested > 0 forces that many bits, < 0 no grouping; at
-// most 2^9 regions (one partition pass) of at least 16 slots (one L2 line).
+// Table-region bits: requested > 0 forces that many, at most 2^9 regions (one
+// partition pass) of at least 16 slots (one L2 line); otherwise none.
 uint32_t npo_region_bits(uint64_t nR, int requested) {
-    const uint32_t l2 = npo_log2(nR);
-    if (requested < 0) return 0;
-    int rb = requested > 0 ? requested : (l2 > kNpoUngroupedLog2 ? (int)(l2 - kNpoRegionLog2) : 0);
+    if (requested <= 0) return 0;
+    const int l2 = (int)npo_log2(nR);
+    int rb = requested;
     if (rb > (int)kMaxPassBits) rb = (int)kMaxPassBits;
-    if (rb > (int)l2 - 4) rb = (int)l2 - 4;
+    if (rb > l2 - 4) rb = l2 - 4;
     return rb < 0 ? 0u : (uint32_t)rb;
 }
 
 size_t npo_scratch(uint64_t nR, uint64_t nS, int region_bits, int num_sms) {
     const uint32_t rb = npo_region_bits(nR, region_bits);
-    return Workspace::need(1ULL << npo_log2(nR), 8) + Workspace::need(1, 8) +
+    return Workspace::need(rb ? 1ULL << npo_log2(nR) : 4 * npo_buckets(nR), 8) +
            (rb ? paged_partition_scratch(nR, nS, rb, 0, num_sms) : 0);
 }
 
@@ -212,10 +219,10 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
     const uint32_t rb = npo_region_bits(j.nR, region_bits);
     PartOut po{};
     if (rb) ADB_TRY(run_paged_partition(ctx, j, DigitFn{32u - rb, (1u << rb) - 1u, true}, nullptr, &po, acc));
-    uint64_t *table = ctx->ws.take<uint64_t>(1ULL << l2);
-    unsigned long long *sent = ctx->ws.take<unsigned long long>(1);
-    ADB_CK(cudaMemsetAsync(table, 0xFF, (1ULL << l2) * 8, st));
-    ADB_CK(cudaMemsetAsync(sent, 0, 8, st));
+    const uint64_t nb = npo_buckets(j.nR), slots = rb ? 1ULL << l2 : 4 * nb;
+    uint64_t *table = ctx->ws.take<uint64_t>(slots);
+    unsigned long long *sent = acc + 4;
+    ADB_CK(cudaMemsetAsync(table, 0xFF, slots * 8, st));
     int *err = reinterpret_cast<int *>(acc + 2);
     if (rb) {
         const NpoPages PR{po.R.pages, po.R.pcount, po.R.plist, po.R.log, po.pstart, po.Fout};
@@ -240,18 +247,23 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
                                                                                nullptr, 0);
     } else {
         const int threads = 256;
-        auto blocks = [&](uint64_t n) {
-            uint64_t b = (n + threads - 1) / threads;
-            const uint64_t cap = (uint64_t)ctx->num_sms * 8;
+        // every CTA resident at once: one grid-stride sweep without a second wave
+        int rb_sm = 0, rp_sm = 0;
+        ADB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rb_sm, npo_build, threads, 0));
+        if (j.mat) ADB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rp_sm, npo_probe<true>, threads, 0));
+        else ADB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rp_sm, npo_probe<false>, threads, 0));
+        auto blocks = [&](uint64_t n, int per_sm) {
+            const uint64_t b = (n + threads - 1) / threads, cap = (uint64_t)ctx->num_sms * (per_sm < 1 ? 1 : per_sm);
             return (int)(b < 1 ? 1 : (b > cap ? cap : b));
         };
-        npo_build<<<blocks(j.nR), threads, 0, st>>>(j.R, j.nR, table, l2, sent, err);
+        npo_build<<<blocks(j.nR, rb_sm), threads, 0, st>>>(j.R, j.nR, table, (uint32_t)nb, sent, err);
         ADB_CK(mark(ctx, 2));
         if (j.mat)
-            npo_probe<true><<<blocks(j.nS), threads, 0, st>>>(j.S, j.nS, table, l2, sent, acc, j.mat, acc + 3,
-                                                              j.mat_cap);
+            npo_probe<true><<<blocks(j.nS, rp_sm), threads, 0, st>>>(j.S, j.nS, table, (uint32_t)nb, sent, acc, j.mat,
+                                                                     acc + 3, j.mat_cap);
         else
-            npo_probe<false><<<blocks(j.nS), threads, 0, st>>>(j.S, j.nS, table, l2, sent, acc, nullptr, nullptr, 0);
+            npo_probe<false><<<blocks(j.nS, rp_sm), threads, 0, st>>>(j.S, j.nS, table, (uint32_t)nb, sent, acc,
+                                                                      nullptr, nullptr, 0);
     }
     ADB_CK(cudaGetLastError());
     ctx->kernels += 2;

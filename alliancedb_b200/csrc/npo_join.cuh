@@ -16,6 +16,7 @@
 #pragma once
 
 #include "adb_common.cuh"
+#include "partition.cuh"
 
 namespace adb {
 
@@ -38,18 +39,6 @@ __device__ __forceinline__ void npo_insert_from(uint64_t *table, uint64_t mask, 
     }
 }
 
-// static: each translation unit that includes this header gets its own copy
-static __global__ void npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ table,
-                          uint32_t log2n, unsigned long long *sentinel_cnt, int *err) {
-    const uint64_t mask = (1ULL << log2n) - 1;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += stride) {
-        const uint64_t w = R[i];
-        if (w == kEmpty) { atomicAdd(sentinel_cnt, 1ull); continue; }
-        npo_insert_from(table, mask, npo_hash(tkey(w), log2n), w, err);
-    }
-}
-
 // Count, checksum and optional materialisation of a probe's matches.
 template <bool kMaterialize>
 struct NpoSink {
@@ -66,6 +55,19 @@ struct NpoSink {
         }
     }
 };
+
+// The matches of S tuple s (key 0xFFFFFFFF) with the nsent build tuples that
+// equal the empty marker.
+template <bool kMaterialize>
+__device__ __forceinline__ void npo_add_sentinels(NpoSink<kMaterialize> &sink, uint64_t s, uint64_t nsent) {
+    sink.a.count += nsent;
+    sink.a.sum += nsent * pair_hash(0xFFFFFFFFu, 0xFFFFFFFFu, tpay(s));
+    if (kMaterialize)
+        for (uint64_t t = 0; t < nsent; t++) {
+            const unsigned long long k = atomicAdd(sink.mat_n, 1ull);
+            if (k < sink.mat_cap) sink.mat[k] = s;
+        }
+}
 
 // A probe's first read: the four slots b .. b + 3 from b = slot & ~1, the
 // 16-byte pair holding the start slot and the pair after it (wrapping at the
@@ -123,15 +125,7 @@ __device__ __forceinline__ bool npo_probe_window(NpoSink<kMaterialize> &sink, ui
         const ulonglong2 h2 = j & 2 ? hi : lo;
         sink.match(s, key, tpay(j & 1 ? h2.y : h2.x), sh);
     }
-    if (key == 0xFFFFFFFFu && nsent) {
-        sink.a.count += nsent;
-        sink.a.sum += nsent * pair_hash_pre(key, 0xFFFFFFFFu, sh);
-        if (kMaterialize)
-            for (uint64_t t = 0; t < nsent; t++) {
-                const unsigned long long k = atomicAdd(sink.mat_n, 1ull);
-                if (k < sink.mat_cap) sink.mat[k] = s;
-            }
-    }
+    if (key == 0xFFFFFFFFu && nsent) npo_add_sentinels(sink, s, nsent);
     return open;
 }
 
@@ -144,39 +138,144 @@ __device__ __forceinline__ void npo_probe_one(NpoSink<kMaterialize> &sink, const
     if (npo_probe_window(sink, s, slot, lo, hi, nsent, sh)) npo_probe_rest(sink, table, mask, s, slot, sh);
 }
 
-// Probe: each thread takes kProbeU S tuples at a time (a grid-stride group),
-// so that kProbeU random table reads are in flight per thread; a probe reads
-// its four-slot window first (npo_window: two 16-byte loads).
-constexpr int kProbeU = 4;
+// ---------------------------------------------------------------------------
+// The bucket table: nb buckets of four slots (one 32-byte sector), bucket =
+// the high word of hash x nb, so any nb will do.  A tuple claims the slot its
+// hash picks in its bucket with one compare-and-swap; where that is taken it
+// reads the bucket for a free slot and goes on to the next bucket when there is
+// none.  A probe reads its bucket with one 32-byte load and goes on only past a
+// full one: rare for a lane, but some lane of a warp nearly always does, so the
+// table has three slots per build tuple (24 bytes): at two, 14 % of the buckets
+// are full and the probe's instructions double; at four the table outgrows the
+// L2 sooner.  3,000,017 x 5,000,011 tuples, keys over 32 bits (build with the
+// table's clearing / probe, us): linear probing in 2^ceil(log2 2|R|) slots with a
+// four-slot window 62 / 115; buckets at two slots per tuple 77 / 96, at three
+// 68 / 70, at four 90 / 64.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ uint64_t npo_buckets(uint64_t nR) { return nR > 2 ? (3 * nR + 3) / 4 : 1; }
+
+__device__ __forceinline__ void npo_ld_bucket(const uint64_t *p, uint64_t (&v)[4]) {
+    asm volatile("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+                 : "l"(p));
+}
+
+constexpr int kProbeU = 1;      // probe: tuples per lane in flight
+
+static __global__ void __launch_bounds__(256)
+npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ table, uint32_t nb,
+          unsigned long long *sentinel_cnt, int *err) {
+    const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
+    auto cas = [&](uint64_t slot, uint64_t w) {
+        return atomicCAS(reinterpret_cast<unsigned long long *>(table) + slot, (unsigned long long)kEmpty,
+                         (unsigned long long)w) == kEmpty;
+    };
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += T) {
+        const uint64_t w = ld_stream(R + i);
+        if (w == kEmpty) { atomicAdd(sentinel_cnt, 1ull); continue; }
+        const uint32_t h = tkey(w) * kFibMul, st = h >> 5 & 3;
+        uint32_t b = __umulhi(h, nb);
+        if (cas(4ull * b + st, w)) continue;
+        // the slot was taken: read the bucket for a free one, the next where there is none
+        for (uint64_t tries = 0;; tries++) {
+            uint64_t v[4];
+            asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                         : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+                         : "l"(table + 4ull * b)
+                         : "memory");
+            uint32_t empty = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (v[j] == kEmpty) empty |= 1u << j;
+            if (empty) {
+                const uint32_t k = (st + __ffs((empty | empty << 4) >> st) - 1) & 3;
+                if (cas(4ull * b + k, w)) break;
+            } else {
+                b = b + 1 == nb ? 0 : b + 1;
+            }
+            if (tries > 8ull * nb) { atomicExch(err, 2); break; }   // table full: cannot happen at load <= 0.5
+        }
+    }
+}
+
+// One bucket against S tuple s: its first match into (found, pay), further ones
+// (repeated build keys) to the sink.  Returns whether the bucket is full, so
+// that the next one must be read too.
+template <bool kMaterialize>
+__device__ __forceinline__ bool npo_scan(NpoSink<kMaterialize> &sink, uint64_t s, uint64_t sh, const uint64_t (&v)[4],
+                                         bool &found, uint32_t &pay) {
+    const uint32_t key = tkey(s);
+    uint32_t hits = 0;
+    bool full = true;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const bool empty = v[j] == kEmpty;
+        full = full && !empty;
+        if (tkey(v[j]) == key && !empty) hits |= 1u << j;
+    }
+    while (hits) {
+        const int j = __ffs(hits) - 1;
+        hits &= hits - 1;
+        const uint32_t lo = j & 1 ? tpay(v[1]) : tpay(v[0]), hi = j & 1 ? tpay(v[3]) : tpay(v[2]);
+        if (found) sink.match(s, key, pay, sh);
+        pay = j & 2 ? hi : lo;
+        found = true;
+    }
+    return full;
+}
 
 template <bool kMaterialize>
-__global__ void npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restrict__ table,
-                          uint32_t log2n, const unsigned long long *sentinel_cnt, unsigned long long *acc,
-                          uint64_t *mat, unsigned long long *mat_n, uint64_t mat_cap) {
+__global__ void __launch_bounds__(256)
+npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restrict__ table, uint32_t nb,
+          const unsigned long long *sentinel_cnt, unsigned long long *acc, uint64_t *mat, unsigned long long *mat_n,
+          uint64_t mat_cap) {
     __shared__ uint64_t red[64];
-    const uint64_t mask = (1ULL << log2n) - 1;
     const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nsent = *sentinel_cnt;
     NpoSink<kMaterialize> sink{Acc(), mat, mat_n, mat_cap};
-    for (uint64_t g0 = tid; g0 < nS; g0 += T * kProbeU) {
-        uint64_t s[kProbeU], slot[kProbeU];
-        ulonglong2 lo[kProbeU], hi[kProbeU];
-        bool ok[kProbeU];
+    uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint64_t n[kProbeU];
 #pragma unroll
-        for (int u = 0; u < kProbeU; u++) {   // S tuples g0, g0 + T, ...: coalesced across the warp
-            const uint64_t i = g0 + (uint64_t)u * T;
-            ok[u] = i < nS;
-            s[u] = ok[u] ? __ldcs(reinterpret_cast<const unsigned long long *>(S) + i) : 0ULL;
+    for (int u = 0; u < kProbeU; u++) n[u] = i0 + u * T < nS ? ld_stream(S + i0 + u * T) : 0ULL;
+    for (; i0 < nS; i0 += kProbeU * T) {
+        uint64_t s[kProbeU], v[kProbeU][4], sh[kProbeU];
+        uint32_t b[kProbeU], pay[kProbeU];
+        bool found[kProbeU];
+#pragma unroll
+        for (int u = 0; u < kProbeU; u++) {   // the buckets' loads, then the next tuples', before any is used
+            s[u] = n[u];
+            b[u] = __umulhi(tkey(s[u]) * kFibMul, nb);
+            npo_ld_bucket(table + 4ull * b[u], v[u]);
         }
 #pragma unroll
-        for (int u = 0; u < kProbeU; u++) {   // the windows: all loads issued before any is used
-            slot[u] = npo_hash(tkey(s[u]), log2n);
-            if (ok[u]) npo_window(table, mask, slot[u], lo[u], hi[u]);
+        for (int u = 0; u < kProbeU; u++) {
+            const uint64_t k = i0 + (kProbeU + u) * T;
+            n[u] = k < nS ? ld_stream(S + k) : 0ULL;
         }
+#pragma unroll
+        for (int u = 0; u < kProbeU; u++) {
+            sh[u] = s_half(tkey(s[u]), tpay(s[u]));
+            found[u] = false;
+            pay[u] = 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kProbeU; u++) {
+            if (i0 + u * T < nS) {
+                bool more = npo_scan(sink, s[u], sh[u], v[u], found[u], pay[u]);
+                for (uint32_t t = 1; more && t < nb; t++) {
+                    b[u] = b[u] + 1 == nb ? 0 : b[u] + 1;
+                    uint64_t x[4];
+                    npo_ld_bucket(table + 4ull * b[u], x);
+                    more = npo_scan(sink, s[u], sh[u], x, found[u], pay[u]);
+                }
+                if (tkey(s[u]) == 0xFFFFFFFFu && nsent) npo_add_sentinels(sink, s[u], nsent);
+            }
+        }
+        // the lanes of a warp find their matches in different buckets; the
+        // checksum then runs once for all of them
 #pragma unroll
         for (int u = 0; u < kProbeU; u++)
-            if (ok[u]) npo_probe_one(sink, table, mask, s[u], slot[u], lo[u], hi[u], nsent);
+            if (found[u]) sink.match(s[u], tkey(s[u]), pay[u], sh[u]);
     }
     block_flush(sink.a, acc, red);
 }

@@ -27,6 +27,7 @@
 // contents behind; each call clears the table part it uses and the result
 // words before building.  Calls that overlap on the GPU (different streams or
 // threads at the same time) race on the array: serialise them.
+#include <algorithm>
 #include <mutex>
 
 #include "engine.cuh"
@@ -36,8 +37,8 @@ namespace adb {
 
 constexpr uint64_t kNoAllocTableSlots = 1ULL << 22;                 // 32 MiB of slots
 constexpr uint64_t kNoAllocMaxBuild = kNoAllocTableSlots / 2;       // 2^21 build tuples
-// A table of 2^ceil(log2(2 nR)) <= kNoAllocTableSlots slots is at most half
-// full, so every insert finds an empty slot before it has tried them all and
+// A table of three slots per tuple, or of all kNoAllocTableSlots, is at most
+// half full, so every insert finds an empty slot before it has tried them all and
 // npo_build never sets its table-full error word: the two result words are the
 // whole outcome of a call.
 static_assert(2 * kNoAllocMaxBuild <= kNoAllocTableSlots, "the fixed table must stay at most half full");
@@ -103,11 +104,10 @@ extern "C" int adb_npo_join_noalloc(const adb_tuple *dR, uint64_t nR, const adb_
     unsigned long long *scratch = nullptr;
     ADB_TRY(noalloc_scratch_ptr(&scratch));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint32_t l2 = ceil_log2_u64(2 * (nR ? nR : 1));
-    if (l2 < 2) l2 = 2;   // at least four slots (the probe's first read is a four-slot window)
+    const uint64_t nb = std::min(npo_buckets(nR), kNoAllocTableSlots / 4);
     uint64_t *table = reinterpret_cast<uint64_t *>(scratch);
     unsigned long long *acc = scratch + kNoAllocTableSlots;   // count, checksum, err, sentinel
-    ADB_CK(cudaMemsetAsync(table, 0xFF, (1ULL << l2) * sizeof(uint64_t), st));
+    ADB_CK(cudaMemsetAsync(table, 0xFF, 4 * nb * sizeof(uint64_t), st));
     ADB_CK(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), st));
     if (nR && nS) {
         const int threads = 256;
@@ -115,9 +115,9 @@ extern "C" int adb_npo_join_noalloc(const adb_tuple *dR, uint64_t nR, const adb_
             const uint64_t b = (n + threads - 1) / threads;
             return (int)(b < 1 ? 1 : (b > (uint64_t)kNumSMs * 8 ? (uint64_t)kNumSMs * 8 : b));
         };
-        npo_build<<<blocks(nR), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dR), nR, table, l2, acc + 3,
+        npo_build<<<blocks(nR), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dR), nR, table, (uint32_t)nb, acc + 3,
                                                   reinterpret_cast<int *>(acc + 2));
-        npo_probe<false><<<blocks(nS), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dS), nS, table, l2,
+        npo_probe<false><<<blocks(nS), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dS), nS, table, (uint32_t)nb,
                                                          acc + 3, acc, nullptr, nullptr, 0);
     }
     noalloc_emit<<<1, 32, 0, st>>>(acc, d_out);

@@ -39,7 +39,8 @@ static void flat_ctas(uint64_t nR, uint64_t nS, int num_sms, int G[2]) {
 static void launch_pass(const PassArgs &a, uint32_t F, int G, bool paged, cudaStream_t st) {
     const dim3 grid(G, 2);
     const size_t smem = pass_smem(F, paged);
-    if (paged) partition_pass<1, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
+    if (paged && a.df.hashed) partition_pass<1, kPassThreads, true><<<grid, kPassThreads, smem, st>>>(a);
+    else if (paged) partition_pass<1, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
     else if (a.df.hashed) partition_pass<0, kPassThreads, true><<<grid, kPassThreads, smem, st>>>(a);
     else partition_pass<0, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
 }
@@ -242,12 +243,13 @@ size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms) {
            Workspace::need(2, 4);
 }
 
-int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc) {
+int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned long long *acc) {
     cudaStream_t st = ctx->stream;
     uint32_t b1, b2;
     split_bits(bits, &b1, &b2);
-    const DigitFn d1{0u, (1u << b1) - 1};
-    const DigitFn d2{b1, (1u << b2) - 1};
+    // the key's low bits, or the high bits of key * kFibMul
+    const DigitFn d1{hashed ? 32u - b1 : 0u, (1u << b1) - 1, hashed};
+    const DigitFn d2{hashed ? 32u - b1 - b2 : b1, (1u << b2) - 1, hashed};
     PartOut po;
     ADB_TRY(run_paged_partition(ctx, j, d1, b2 ? &d2 : nullptr, &po, acc));
     if (b2) ADB_CK(mark(ctx, 2));   // phases: pass 1 | pass 2 | work list | join
@@ -279,7 +281,9 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc)
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;
     a.wbase = nullptr; a.wbits = nullptr; a.nwin = 0; a.wacc = nullptr;
     const int grid = ctx->num_sms * kJoinMinBlocks;
-    if (j.mat) radix_join_items<true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    if (j.mat && hashed) radix_join_items<true, true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    else if (j.mat) radix_join_items<true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    else if (hashed) radix_join_items<false, true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
     else radix_join_items<false><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
     ADB_CK(cudaGetLastError());
     ctx->kernels += 4;
@@ -287,16 +291,16 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, unsigned long long *acc)
 }
 
 int radix_set_attrs() {
-    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)pass_smem(1u << kMaxPassBits, false)));
-    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads, true>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem(1u << kMaxPassBits, false)));
-    ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)pass_smem(1u << kMaxPassBits, true)));
-    ADB_CK(cudaFuncSetAttribute(radix_join_items<false>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
-    ADB_CK(cudaFuncSetAttribute(radix_join_items<true>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
+    const int flat = (int)pass_smem(1u << kMaxPassBits, false), paged = (int)pass_smem(1u << kMaxPassBits, true);
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads>, attr, flat));
+    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads, true>, attr, flat));
+    ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads>, attr, paged));
+    ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads, true>, attr, paged));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<false>, attr, (int)kJoinSmem));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<true>, attr, (int)kJoinSmem));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<false, true>, attr, (int)kJoinSmem));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<true, true>, attr, (int)kJoinSmem));
     return ADB_OK;
 }
 

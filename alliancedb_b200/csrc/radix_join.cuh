@@ -279,10 +279,11 @@ struct ItemRec {
 // pages in flight ahead of the one it probes.
 //
 // The table: bucket heads indexed by the lnb key bits above the b bits the
-// partitioning consumed, one head per R slot (up to 2^13), and chains through
-// the tuples themselves.  All keys of a bucket share their low b + lnb bits,
-// so a linked tuple's key holds the next slot of its chain there (its own
-// slot: the end); the bits above stay for the comparison.  One 8-byte read per
+// partitioning consumed (kHashed: the lnb bits of key * kFibMul below the b
+// highest), one head per R slot (up to 2^13), and chains through the tuples
+// themselves.  All keys of a bucket share their low b + lnb bits, so a linked
+// tuple's key holds the next slot of its chain there (its own slot: the end);
+// the bits above stay for the comparison.  One 8-byte read per
 // visited tuple gives payload, comparison bits and link.
 //
 // Bound: instruction issue and the ALU pipe (60 % busy), not DRAM.  |R| = |S| =
@@ -296,7 +297,7 @@ struct ItemRec {
 // whole call 7.86 -> 6.01 ms.  Adding a warp's matches together after the walk
 // instead of as they are found: 0.83 / 1.14, and 1.27 instead of 1.23 ms with
 // every key four times in both relations (2^26), so not kept.
-template <bool kMat>
+template <bool kMat, bool kHashed = false>
 __global__ void __launch_bounds__(kJoinThreads, kJoinMinBlocks)
 radix_join_items(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -424,18 +425,27 @@ radix_join_items(JoinArgs a) {
             load_page(1, x1, n1);
         }
 
-        const uint32_t lnb = C.lnb;
+        // the bits of x (the key, or its hash) that a bucket shares: the lowest
+        // `link` ones, or the highest
+        const uint32_t lnb = C.lnb, link = shift + lnb;
         const uint32_t bmask = (1u << lnb) - 1;
-        const uint32_t lim = 1u << (shift + lnb), lmask = lim - 1;   // link bits of a linked key
+        const uint32_t lim = 1u << link, lmask = lim - 1;
+        auto hash = [&](uint64_t t) { return kHashed ? tkey(t) * kFibMul : tkey(t); };
+        auto bucket = [&](uint32_t x) { return kHashed ? x >> (32 - link) & bmask : x >> shift & bmask; };
+        auto linked = [&](uint32_t x, uint32_t next) {
+            return kHashed ? next << (32 - link) | (x << link) >> link : (x & ~lmask) | next;
+        };
+        auto next_of = [&](uint32_t w) { return kHashed ? w >> (32 - link) : w & lmask; };
+        auto same = [&](uint32_t w, uint32_t x) { return kHashed ? (w ^ x) << link == 0 : (w ^ x) < lim; };
         for (uint32_t i = threadIdx.x; i < ((1u << lnb) + 3) / 4; i += kJoinThreads)
             reinterpret_cast<uint4 *>(heads)[i] = make_uint4(kNone, kNone, kNone, kNone);
         if (a.waits_run_out && threadIdx.x == 0) atomicExch(a.err, 1);
         __syncthreads();
 
         // --- build: a warp per page, two tuples per lane, kB pages in flight
-        auto link = [&](uint32_t s, uint64_t t) {
-            const uint32_t old = atomicExch(&heads[(tkey(t) >> shift) & bmask], s);
-            return tword((tkey(t) & ~lmask) | (old == kNone ? s : old), tpay(t));
+        auto enter = [&](uint32_t s, uint64_t t) {
+            const uint32_t x = hash(t), old = atomicExch(&heads[bucket(x)], s);
+            return tword(linked(x, old == kNone ? s : old), tpay(t));
         };
         constexpr int kB = 4;
         for (uint32_t k0 = warp; k0 < nrpg; k0 += kB * kWarps) {
@@ -452,8 +462,8 @@ radix_join_items(JoinArgs a) {
             for (int j = 0; j < kB; j++) {
                 const uint32_t s = (v[j] >> 8) + 2 * lane;
                 if (2 * lane < (int)(v[j] & 0xFFu)) {
-                    r[j].x = link(s, r[j].x);
-                    if (2 * lane + 1 < (int)(v[j] & 0xFFu)) r[j].y = link(s + 1, r[j].y);
+                    r[j].x = enter(s, r[j].x);
+                    if (2 * lane + 1 < (int)(v[j] & 0xFFu)) r[j].y = enter(s + 1, r[j].y);
                     *reinterpret_cast<ulonglong2 *>(tup + s) = r[j];
                 }
             }
@@ -470,14 +480,14 @@ radix_join_items(JoinArgs a) {
             const uint32_t nx_pg = s_ids(rec[cur ^ 1]);
             uint32_t matches = 0;
             auto probe = [&](uint64_t s) {
-                const uint32_t key = tkey(s);
-                uint32_t at = heads[(key >> shift) & bmask];
+                const uint32_t key = tkey(s), x = hash(s);
+                uint32_t at = heads[bucket(x)];
                 if (at == kNone) return;
                 const uint64_t sh = s_half(key, tpay(s));
                 while (true) {
                     const uint64_t r = tup[at];
-                    const uint32_t nx = tkey(r) & lmask;
-                    if ((tkey(r) ^ key) < lim) {
+                    const uint32_t nx = next_of(tkey(r));
+                    if (same(tkey(r), x)) {
                         
                         acc.sum += pair_hash_pre(key, tpay(r), sh);
                         matches++;

@@ -53,17 +53,14 @@ ALG_BYTES = {"PRO": 24, "RJ_st": 24, "PRH": 24, "PRHO": 24, "NPO": 16, "NPO_st":
 # Per family: phase index (adb_join_result.ms_phase) -> (kernel, algorithmic
 # bytes per input tuple of one launch, DRAM bytes per input tuple of one launch
 # from an ncu capture of dram__bytes_read.sum + dram__bytes_write.sum at
-# |R| = |S| = 2^24, for NPO at 2^25, the smallest size it groups by table
-# region; None where not captured).  The traffic of a full-size
+# |R| = |S| = 2^24; None where not captured).  The traffic of a full-size
 # launch is that figure times the launch's tuples: the kernels stream every
 # tuple once, so traffic grows in proportion.
 KERNELS = {
     "radix": {0: ("partition_pass<0,512> (pass 1)", 16, (270247168 + 213934080) / 2**25),
               1: ("partition_pass<1,512> (pass 2)", 16, (276288768 + 214363648) / 2**25),
-              3: ("radix_join_items<Chain>", 8, (273622272 + 3668736) / 2**25)},
-    "npo": {0: ("partition_pass<0,512,hashed> (grouping by table region)", 16, (540667392 + 486182144) / 2**26),
-            1: ("npo_build_pages", 8, (812415744 + 381705728) / 2**26),
-            3: ("npo_probe_pages", 8, (809180672 + 3512320) / 2**26)},
+              3: ("radix_join_items", 8, (273622272 + 3668736) / 2**25)},
+    "npo": {1: ("npo_build", 8, None), 3: ("npo_probe", 8, None)},
     "smj": {0: ("partition_pass (both passes)", 32,
                 (271074048 + 215111680 + 279591680 + 219554048) / 2**25),
             3: ("smj_items", 8, (282003456 + 3525376) / 2**25)},
@@ -497,7 +494,9 @@ def main():
     e2e_value = 2 * n * world / (e2e_ms / 1e3)
 
     # ---- roofline of the dominant kernel
-    fam = "npo" if args.algo.startswith("NPO") else ("smj" if args.algo.startswith("m-") else "radix")
+    # (NPO is the partitioned join on hashed digits once its table outgrows L2, |R| > 3.67 M)
+    fam = ("npo" if args.algo.startswith("NPO") and n <= 7 << 19 else "smj" if args.algo.startswith("m-")
+           else "radix")
     ph = np.array(phases).mean(axis=0)
     cands = KERNELS[fam]
     dom = max(cands, key=lambda k: ph[k])
@@ -520,15 +519,14 @@ def main():
                      "frac": achieved / hbm, "peak_source": peak_kind,
                      "alg_bytes_per_launch": dom_bytes, "kernel_ms": float(ph[dom]),
                      "traffic": traffic, "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                                           "per tuple at |R|=|S|=2^24 (NPO 2^25), scaled to this launch"
+                                                           "per tuple at |R|=|S|=2^24, scaled to this launch"
                                                            if traffic else None,
                      "pipeline": {"alg_bytes_per_tuple": ALG_BYTES.get(args.algo, 24), "achieved": pipe_gbs,
                                   "frac": pipe_gbs / hbm}},
         "phases_ms": [float(x) for x in ph],
         **({"random_access": {
-            "note": "NPO's table (2 slots per R tuple) is far larger than L2; R and S are grouped by table region "
-                    "first, so the inserts (one compare-and-swap each) and the probes (one 32-byte sector each) "
-                    "hit the L2-resident region",
+            "note": "NPO's table (3 slots per R tuple) stays in L2: the inserts (one compare-and-swap each) and the "
+                    "probes (one 32-byte bucket each) are bound by its random access rate",
             "build_cas_per_s": n / (ph[1] / 1e3), "probes_per_s": n / (ph[3] / 1e3)}} if fam == "npo" else {}),
         "gpu_launches": kernels_per_step * args.steps,
         "clocks": clk.summary(),
