@@ -95,26 +95,7 @@ static void dscan(cudaStream_t st, const uint32_t *in, uint32_t n, T *out, T *bs
     dscan_apply<T><<<nb, 1024, 0, st>>>(in, n, bsum, out);
 }
 
-// items per partition (R chunks x S chunks) next to the R chunk counts
-__global__ void items_per_part(const uint32_t *rch, const uint32_t *sch, uint32_t n, uint32_t *items) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
-        items[p] = (rch[p] && sch[p]) ? rch[p] * sch[p] : 0u;
-}
-
 __global__ void copy_last_u32(const uint32_t *src, uint32_t *dst) { *dst = *src; }
-
-// Places each unit's pages into its partitions' page lists (positions by atomics).
-__global__ void page_place_atomic(PassArgs a, uint32_t *fill0, uint32_t *fill1) {
-    const int relidx = blockIdx.y, g = blockIdx.x;
-    const PageSet &o = relidx ? a.out[1] : a.out[0];
-    uint32_t *fill = relidx ? fill1 : fill0;
-    const uint32_t used = o.nlog[g];
-    const uint32_t pool_base = (relidx ? a.in[1] : a.in[0]).unit_pool[g];
-    for (uint32_t k = threadIdx.x; k < used; k += blockDim.x) {
-        const uint32_t D = o.log[pool_base + k];
-        o.plist[o.pstart[D] + atomicAdd(&fill[D], 1u)] = pool_base + k;
-    }
-}
 
 // ---- fan-out per window-size bucket -----------------------------------------
 // bucket = ceil(log2(max(|R_w|, |S_w|))); default: R partitions of about 8K tuples
@@ -197,11 +178,11 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     const uint32_t nbs = Dt / kScanBlock + 2;
     const size_t meta = Workspace::need(W, 1) + 3 * Workspace::need(W + 1, 4) + 2 * Workspace::need(W + 1, 8) +
                         2 * Workspace::need(G + 1, 4);
-    const size_t bytes = meta + 2 * (Workspace::need(pages * kPageTuples, 8) + 2 * Workspace::need(pages, 4) +
-                                     Workspace::need(pages, 1) + Workspace::need(G, 4)) +
-                         4 * Workspace::need(2ull * Dt + 2, 4) + 2 * Workspace::need(2ull * (Dt + 1), 8) +
-                         2 * Workspace::need(nbs, 8) + 4 * Workspace::need(Dt + 1, 4) +
-                         Workspace::need(pages * kPageTuples / kChunkW + Dt + 1, 8) + Workspace::need(2 * W + 8, 8);
+    const size_t bytes = meta + 2 * (Workspace::need(pages * kPageTuples, 8) + 3 * Workspace::need(pages, 4) +
+                                     Workspace::need(pages, 1) + Workspace::need(G, 4) + Workspace::need(G, 8)) +
+                         Workspace::need(2ull * Dt, 4) + Workspace::need(2ull * (Dt + 1), 8) +
+                         Workspace::need(nbs, 8) + WorkList::bytes(Dt, pages, kChunkW) +
+                         Workspace::need(2 * W + 8, 8);
     ADB_TRY(ctx->ws.reserve(bytes + 8192));
 
     // the plan (window bits, partition bases, unit offsets, segments, unit pools):
@@ -243,6 +224,8 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
         o.log = ctx->ws.take<uint32_t>(pages);
         o.pcount = ctx->ws.take<uint8_t>(pages);
         o.nlog = ctx->ws.take<uint32_t>(G);
+        o.doff = ctx->ws.take<uint32_t>(pages);
+        o.udesc = ctx->ws.take<uint2>(G);
         o.plist = ctx->ws.take<uint32_t>(pages);
     }
     a.df = DigitFn{0u, 0u};
@@ -255,47 +238,34 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     unsigned long long *wacc = ctx->ws.take<unsigned long long>(2 * W + 8);
     unsigned long long *acc = wacc + 2 * W;   // err word at acc[2]
     a.err = reinterpret_cast<int *>(acc + 2);
-    uint32_t *tot = ctx->ws.take<uint32_t>(2ull * Dt + 2);
-    uint32_t *fill = ctx->ws.take<uint32_t>(2ull * Dt + 2);
-    a.seg_totals = tot;
+    uint32_t *tot = ctx->ws.take<uint32_t>(2ull * Dt);
+    a.totals = tot;
     uint64_t *pstart = ctx->ws.take<uint64_t>(2ull * (Dt + 1));
     a.out[0].pstart = pstart;
     a.out[1].pstart = pstart + (Dt + 1);
     uint64_t *bsum64 = ctx->ws.take<uint64_t>(nbs);
-    uint32_t *bsum32 = reinterpret_cast<uint32_t *>(ctx->ws.take<uint64_t>(nbs));
-    uint32_t *rch = ctx->ws.take<uint32_t>(Dt + 1);
-    uint32_t *sch = ctx->ws.take<uint32_t>(Dt + 1);
-    uint32_t *items = ctx->ws.take<uint32_t>(2ull * Dt + 2);
-    uint32_t *items_off = ctx->ws.take<uint32_t>(Dt + 1);
-    uint32_t *chunk_off = ctx->ws.take<uint32_t>(Dt + 1);
-    uint64_t *cstart = ctx->ws.take<uint64_t>(pages * kPageTuples / kChunkW + Dt + 1);
-    uint32_t *ctr = ctx->ws.take<uint32_t>(2);
+    uint32_t *bsum32 = reinterpret_cast<uint32_t *>(bsum64);   // the scans run one after the other
+    WorkList wl;
+    wl.take(ctx->ws, Dt, pages, kChunkW);
 
     ADB_CK(cudaMemsetAsync(wacc, 0, (2 * W + 8) * 8, st));
-    ADB_CK(cudaMemsetAsync(tot, 0, (2ull * Dt + 2) * 4, st));
-    ADB_CK(cudaMemsetAsync(fill, 0, (2ull * Dt + 2) * 4, st));
-    ADB_CK(cudaMemsetAsync(ctr, 0, 8, st));
+    ADB_CK(cudaMemsetAsync(tot, 0, 2ull * Dt * 4, st));
+    ADB_CK(cudaMemsetAsync(wl.ctr, 0, 12, st));
     partition_pass<2, kPassThreads><<<dim3(G, 2), kPassThreads, pass_smem(1u << kMaxPassBits, false), st>>>(a);
     ADB_CK(cudaGetLastError());
     dscan<uint64_t>(st, tot, Dt, pstart, bsum64);
     dscan<uint64_t>(st, tot + Dt, Dt, pstart + (Dt + 1), bsum64);
-    page_place_atomic<<<dim3(G, 2), 256, 0, st>>>(a, fill, fill + Dt);
-    part_rslots<<<(Dt + 7) / 8, 256, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, kChunkW, kSPages, rch,
-                                             sch);
-    items_per_part<<<(Dt + 255) / 256, 256, 0, st>>>(rch, sch, Dt, items);
-    dscan<uint32_t>(st, items, Dt, items_off, bsum32);
-    dscan<uint32_t>(st, rch, Dt, chunk_off, bsum32);
-    copy_last_u32<<<1, 1, 0, st>>>(items_off + Dt, ctr);
-    part_rchunks<<<(Dt + 7) / 8, 256, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, kChunkW, chunk_off,
-                                              cstart);
+    page_place<<<dim3(G, 2), kPlaceThreads, 0, st>>>(a, 0u, nullptr, nullptr);
+    part_chunks<<<(Dt + 31) / 32, 1024, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, kChunkW, kSPages, wl,
+                                                 false);
+    dscan<uint32_t>(st, wl.items, Dt, wl.items_off, bsum32);
+    copy_last_u32<<<1, 1, 0, st>>>(wl.items_off + Dt, wl.ctr);
     ADB_CK(cudaGetLastError());
     JoinArgs ja;
     ja.Rpages = a.out[0].pages; ja.Spages = a.out[1].pages;
     ja.Rcount = a.out[0].pcount; ja.Scount = a.out[1].pcount;
     ja.Rlist = a.out[0].plist; ja.Slist = a.out[1].plist;
-    ja.pstart = pstart; ja.items_off = items_off;
-    ja.chunk_off = chunk_off; ja.cstart = cstart;
-    ja.n_items = ctr; ja.work_counter = ctr + 1;
+    ja.pstart = pstart; ja.wl = wl;
     ja.acc = acc; ja.err = reinterpret_cast<int *>(acc + 2);
     ja.waits_run_out = 0;
     ja.F = Dt;

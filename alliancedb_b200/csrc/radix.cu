@@ -6,7 +6,7 @@
 // pass-2 partitioning, then a task-queued join per partition pair.  Here:
 //   pass 1        partition_pass (flat input)  + page lists
 //   pass 2        partition_pass (paged input, work units) + page lists  [fan-out > 2^9]
-//   R chunks      part_rslots, make_items_paged, part_rchunks
+//   R chunks      part_chunks
 //   join          radix_join_items: persistent, work-stealing build + probe
 // The fan-out 2^bits is chosen so an R partition fills about one CTA's
 // shared-memory table (8704 tuples).
@@ -97,19 +97,18 @@ uint64_t paged_final_pool_pages(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t 
     return p.passes == 2 ? p.pages2 : p.pages1;
 }
 
-static size_t pageset_bytes(uint64_t pages, uint32_t G, uint32_t Fout) {
-    return Workspace::need(pages * kPageTuples, 8) + Workspace::need(pages, 4) + Workspace::need(pages, 1) +
-           Workspace::need(G, 4) + Workspace::need(pages, 4);
+static size_t pageset_bytes(uint64_t pages, uint32_t G) {
+    return Workspace::need(pages * kPageTuples, 8) + 3 * Workspace::need(pages, 4) + Workspace::need(pages, 1) +
+           Workspace::need(G, 4) + Workspace::need(G, 8);
 }
 
 size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
     const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
-    size_t s = 2 * pageset_bytes(p.pages1, p.G1, p.F1) + Workspace::need(2ull * p.F1 * p.G1, 4) +
-               Workspace::need(2ull * p.F1, 4) * 2 + Workspace::need(2ull * (p.F1 + 1), 8);
+    size_t s = 2 * pageset_bytes(p.pages1, p.G1) + Workspace::need(2ull * (p.F1 + p.Fout), 4) +
+               Workspace::need(2ull * (p.F1 + 1), 8);
     if (p.passes == 2)
-        s += 2 * pageset_bytes(p.pages2, p.G2, p.Fout) + Workspace::need(2ull * p.F2 * p.G2, 4) +
-             Workspace::need(2ull * p.F2, 4) + Workspace::need(2ull * p.Fout, 4) +
-             Workspace::need(2ull * (p.Fout + 1), 8) + 2 * Workspace::need(p.F1 + 1, 4);
+        s += 2 * pageset_bytes(p.pages2, p.G2) + Workspace::need(2ull * (p.Fout + 1), 8) +
+             2 * Workspace::need(p.F1 + 1, 4);
     return s;
 }
 
@@ -118,6 +117,8 @@ static void take_pageset(Context *ctx, PageSet &ps, uint64_t pages, int G) {
     ps.log = ctx->ws.take<uint32_t>(pages);
     ps.pcount = ctx->ws.take<uint8_t>(pages);
     ps.nlog = ctx->ws.take<uint32_t>(G);
+    ps.doff = ctx->ws.take<uint32_t>(pages);
+    ps.udesc = ctx->ws.take<uint2>(G);
     ps.plist = ctx->ws.take<uint32_t>(pages);
 }
 
@@ -148,23 +149,25 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     a1.G = p.G1;
     a1.pool_cap = p.pool1;
     a1.paged = 0;
-    a1.npd = ctx->ws.take<uint32_t>(2ull * p.F1 * p.G1);
     a1.err = err;
-    uint32_t *rowtot1 = ctx->ws.take<uint32_t>(2ull * p.F1);
-    uint32_t *totals1 = ctx->ws.take<uint32_t>(2ull * p.F1);
+    uint32_t *totals1 = ctx->ws.take<uint32_t>(2ull * (p.F1 + p.Fout)), *totals2 = totals1 + 2ull * p.F1;
+    ADB_CK(cudaMemsetAsync(totals1, 0, 8ull * (p.F1 + (p.passes == 2 ? p.Fout : 0)), st));
+    a1.totals = totals1;
+    a1.Dtot = p.F1;
     uint64_t *pstart1 = ctx->ws.take<uint64_t>(2ull * (p.F1 + 1));
     a1.out[0].pstart = pstart1;
     a1.out[1].pstart = pstart1 + (p.F1 + 1);
 
     launch_pass(a1, p.F1, p.G1, false, st);
-    part_scan_rows<<<(2 * p.F1 + 7) / 8, 256, 0, st>>>(a1.npd, rowtot1, p.F1, p.G1);
-    pass_totals<<<dim3((p.F1 + 255) / 256, 2), 256, 0, st>>>(a1.npd, rowtot1, nullptr, nullptr, p.F1, 1, p.G1,
-                                                             totals1);
-    part_scan_totals<<<2, 1024, 0, st>>>(totals1, pstart1, p.F1);
-    page_place<<<dim3(p.G1, 2), 1024, p.F1 * 4, st>>>(a1, a1.npd, nullptr, nullptr);
+    uint32_t *uoff0 = nullptr, *uoff1 = nullptr;
+    if (p.passes == 2) {
+        uoff0 = ctx->ws.take<uint32_t>(p.F1 + 1);
+        uoff1 = ctx->ws.take<uint32_t>(p.F1 + 1);
+    }
+    page_place<<<dim3(p.G1, 2), kPlaceThreads, 0, st>>>(a1, p.passes == 2 ? p.unit_pages : 0u, uoff0, uoff1);
     ADB_CK(cudaGetLastError());
     ADB_CK(mark(ctx, 1));   // end of pass 1
-    ctx->kernels += 5;
+    ctx->kernels += 2;
     if (p.passes == 1) {
         out->R = a1.out[0];
         out->S = a1.out[1];
@@ -176,9 +179,6 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
 
     // ---- pass 2: work units over pass-1 partitions
     PassArgs a2{};
-    uint32_t *uoff0 = ctx->ws.take<uint32_t>(p.F1 + 1);
-    uint32_t *uoff1 = ctx->ws.take<uint32_t>(p.F1 + 1);
-    make_units<<<2, 1024, 0, st>>>(pstart1, pstart1 + (p.F1 + 1), p.F1, p.unit_pages, uoff0, uoff1);
     for (int r = 0; r < 2; r++) {
         PassIn &in = a2.in[r];
         in.pages = a1.out[r].pages;
@@ -194,22 +194,18 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     a2.pool_cap = p.pool2;
     a2.unit_pages = p.unit_pages;
     a2.paged = 1;
-    a2.npd = ctx->ws.take<uint32_t>(2ull * p.F2 * p.G2);
     a2.err = err;
-    uint32_t *rowtot2 = ctx->ws.take<uint32_t>(2ull * p.F2);
-    uint32_t *totals2 = ctx->ws.take<uint32_t>(2ull * p.Fout);
+    a2.totals = totals2;
+    a2.Dtot = p.Fout;
     uint64_t *pstart2 = ctx->ws.take<uint64_t>(2ull * (p.Fout + 1));
     a2.out[0].pstart = pstart2;
     a2.out[1].pstart = pstart2 + (p.Fout + 1);
 
     launch_pass(a2, p.F2, p.G2, true, st);
-    part_scan_rows<<<(2 * p.F2 + 7) / 8, 256, 0, st>>>(a2.npd, rowtot2, p.F2, p.G2);
-    pass_totals<<<dim3((p.Fout + 255) / 256, 2), 256, 0, st>>>(a2.npd, rowtot2, uoff0, uoff1, p.F2, p.F1, p.G2,
-                                                               totals2);
-    part_scan_totals<<<2, 1024, 0, st>>>(totals2, pstart2, p.Fout);
-    page_place<<<dim3(p.G2, 2), 1024, p.F2 * 4, st>>>(a2, a2.npd, uoff0, uoff1);
+    list_starts<<<dim3((p.Fout + kScanThreads - 1) / kScanThreads, 2), kScanThreads, 0, st>>>(a2);
+    page_place<<<dim3(p.G2, 2), kPlaceThreads, 0, st>>>(a2, 0u, nullptr, nullptr);
     ADB_CK(cudaGetLastError());
-    ctx->kernels += 6;
+    ctx->kernels += 3;
     out->R = a2.out[0];
     out->S = a2.out[1];
     out->Fout = p.Fout;
@@ -238,9 +234,7 @@ size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms) {
     const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
     const uint64_t pagesR = p.passes == 2 ? p.pages2 : p.pages1;
     const uint64_t F = p.Fout;
-    return paged_partition_scratch(nR, nS, b1, b2, num_sms) + Workspace::need(F, 4) * 2 +
-           Workspace::need(F + 1, 4) * 2 + Workspace::need(pagesR * kPageTuples / kChunkW + F + 1, 8) +
-           Workspace::need(2, 4);
+    return paged_partition_scratch(nR, nS, b1, b2, num_sms) + WorkList::bytes(F, pagesR, kChunkW);
 }
 
 int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned long long *acc) {
@@ -255,16 +249,9 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned lo
     if (b2) ADB_CK(mark(ctx, 2));   // phases: pass 1 | pass 2 | work list | join
 
     const uint32_t F = po.Fout;
-    uint32_t *rch = ctx->ws.take<uint32_t>(F);
-    uint32_t *sch = ctx->ws.take<uint32_t>(F);
-    uint32_t *items_off = ctx->ws.take<uint32_t>(F + 1);
-    uint32_t *chunk_off = ctx->ws.take<uint32_t>(F + 1);
-    uint64_t *cstart = ctx->ws.take<uint64_t>(po.pool_pages * kPageTuples / kChunkW + F + 1);
-    uint32_t *ctr = ctx->ws.take<uint32_t>(2);   // [0] n_items, [1] work counter
-    ADB_CK(cudaMemsetAsync(ctr, 0, 2 * sizeof(uint32_t), st));
-    part_rslots<<<(F + 7) / 8, 256, 0, st>>>(po.pstart, po.R.plist, po.R.pcount, F, kChunkW, kSPages, rch, sch);
-    make_items_paged<<<1, 1024, 0, st>>>(rch, sch, F, items_off, chunk_off, ctr);
-    part_rchunks<<<(F + 7) / 8, 256, 0, st>>>(po.pstart, po.R.plist, po.R.pcount, F, kChunkW, chunk_off, cstart);
+    WorkList wl;
+    wl.take(ctx->ws, F, po.pool_pages, kChunkW);
+    ctx->kernels += make_work_list(st, po.pstart, po.R.plist, po.R.pcount, F, kChunkW, kSPages, wl);
     ADB_CK(cudaGetLastError());
     ADB_CK(mark(ctx, 3));
 
@@ -272,9 +259,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned lo
     a.Rpages = po.R.pages; a.Spages = po.S.pages;
     a.Rcount = po.R.pcount; a.Scount = po.S.pcount;
     a.Rlist = po.R.plist; a.Slist = po.S.plist;
-    a.pstart = po.pstart; a.items_off = items_off;
-    a.chunk_off = chunk_off; a.cstart = cstart;
-    a.n_items = ctr; a.work_counter = ctr + 1;
+    a.pstart = po.pstart; a.wl = wl;
     a.acc = acc; a.err = reinterpret_cast<int *>(acc + 2);
     a.waits_run_out = j.test_flags & ADB_TEST_WAITS_RUN_OUT;
     a.F = F; a.bits = (uint32_t)bits;
@@ -286,7 +271,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned lo
     else if (hashed) radix_join_items<false, true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
     else radix_join_items<false><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
     ADB_CK(cudaGetLastError());
-    ctx->kernels += 4;
+    ctx->kernels += 1;
     return ADB_OK;
 }
 

@@ -8,7 +8,7 @@
 // and the task-queue loop of prj_thread (:1409-1416) with a persistent kernel
 // that takes work items from a global counter (work stealing).  A work item is
 // (partition p, R chunk, S chunk): an R chunk is a run of R_p's pages packed
-// greedily up to kRSlots tuples (part_rchunks), read page by page and linked
+// greedily up to kRSlots tuples (part_chunks), read page by page and linked
 // into a chained table in shared memory, and up to kSPages pages of S_p are
 // streamed from global memory and probed, one warp per page.  Large R
 // partitions (duplicate or skewed build keys, or |R| beyond 2^15 * 8K) take
@@ -16,6 +16,7 @@
 #pragma once
 
 #include "adb_common.cuh"
+#include "engine.cuh"
 #include "paged.cuh"
 
 namespace adb {
@@ -35,102 +36,103 @@ __device__ __forceinline__ uint32_t page_weight(uint32_t cnt) {
     return e > kMinPageW ? e : kMinPageW;
 }
 
-// Per partition: R chunk count (greedy by page weight, chunk_w per chunk) and
-// S chunk count (s_pages pages per chunk).  One warp per partition.
-static __global__ void part_rslots(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount, uint32_t F,
-                            uint32_t chunk_w, uint32_t s_pages, uint32_t *rch, uint32_t *sch) {
+// The work items of a join: partition p's items are (R chunk, S chunk) pairs
+// items_off[p] .. items_off[p + 1); its R chunks start at pages
+// cstart[chunk_off[p]], +1, .. (page-list indexes), rch[p] of them.
+struct WorkList {
+    uint32_t *rch, *chunk_off, *items, *items_off;   // [F], [F], [F], [F + 1]
+    uint64_t *cstart;
+    uint32_t *ctr;                                   // items, work counter, blocks done (zeroed before part_chunks)
+    // A partition's chunks weigh more than chunk_w but for the last, so at
+    // most 64 x pages / chunk_w + 1 of them: chunk_off needs no scan.
+    static size_t chunks(uint64_t F, uint64_t pages, uint32_t chunk_w) { return pages * kPageTuples / chunk_w + F + 1; }
+    static size_t bytes(uint64_t F, uint64_t pages, uint32_t chunk_w) {
+        return 3 * Workspace::need(F, 4) + Workspace::need(F + 1, 4) + Workspace::need(chunks(F, pages, chunk_w), 8) +
+               Workspace::need(3, 4);
+    }
+    void take(Workspace &ws, uint64_t F, uint64_t pages, uint32_t chunk_w) {
+        rch = ws.take<uint32_t>(F);
+        chunk_off = ws.take<uint32_t>(F);
+        items = ws.take<uint32_t>(F);
+        items_off = ws.take<uint32_t>(F + 1);
+        cstart = ws.take<uint64_t>(chunks(F, pages, chunk_w));
+        ctr = ws.take<uint32_t>(3);
+    }
+};
+
+// R chunks and item counts, one warp per partition: chunk c of a partition
+// starts at the first page whose preceding weight reaches c * chunk_w (greedy
+// by page weight); S chunks are s_pages pages each.  With `scan` (F <= 1024) the
+// last block to finish also makes items_off and the item count, so that one
+// launch stands between the passes and the join.
+static __global__ void __launch_bounds__(1024)
+part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount, uint32_t F, uint32_t chunk_w,
+            uint32_t s_pages, WorkList wl, bool scan) {
     const int lane = threadIdx.x & 31;
     const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (p >= F) return;
-    const uint64_t *pR = pstart, *pS = pstart + (F + 1);
-    const uint64_t r0 = pR[p], r1 = pR[p + 1];
-    uint64_t wsum = 0, wlast = 0;
-    for (uint64_t k = r0 + lane; k < r1; k += 32) {
-        const uint32_t w = page_weight(Rcount[Rlist[k]]);
-        wsum += w;
-        if (k == r1 - 1) wlast = w;
-    }
-    wsum = warp_sum_u64(wsum);
-    wlast = warp_sum_u64(wlast);
-    if (lane == 0) {
-        const uint64_t nS = pS[p + 1] - pS[p];
-        rch[p] = r1 > r0 ? (uint32_t)((wsum - wlast) / chunk_w + 1) : 0u;
-        sch[p] = (uint32_t)((nS + s_pages - 1) / s_pages);
-    }
-}
-
-// Work items (R chunk x S chunk) and R chunk offsets: items_off[p], chunk_off[p].
-static __global__ void make_items_paged(const uint32_t *rch, const uint32_t *sch, uint32_t F, uint32_t *items_off,
-                                 uint32_t *chunk_off, uint32_t *n_items) {
-    __shared__ uint32_t tmp[32];
-    __shared__ uint32_t carry[2];
-    if (threadIdx.x == 0) carry[0] = carry[1] = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < F; base += blockDim.x) {
-        const uint32_t p = base + threadIdx.x;
-        uint32_t vi = 0, vc = 0;
-        if (p < F) {
-            vc = rch[p];
-            vi = (vc && sch[p]) ? vc * sch[p] : 0u;
-        }
-        uint32_t ti, tc;
-        const uint32_t ei = block_exclusive_scan(vi, tmp, &ti);
-        const uint32_t ec = block_exclusive_scan(vc, tmp, &tc);
-        if (p < F) {
-            items_off[p] = carry[0] + ei;
-            chunk_off[p] = carry[1] + ec;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) { carry[0] += ti; carry[1] += tc; }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        items_off[F] = carry[0];
-        chunk_off[F] = carry[1];
-        *n_items = carry[0];
-    }
-}
-
-// First page (page-list index) of every R chunk: chunk c of partition p starts
-// at the first page whose preceding weight in p reaches c * chunk_w.  One warp
-// per partition.
-static __global__ void part_rchunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount, uint32_t F,
-                             uint32_t chunk_w, const uint32_t *chunk_off, uint64_t *cstart) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (p >= F) return;
-    const uint64_t r0 = pstart[p], r1 = pstart[p + 1];
-    uint64_t carry = 0;                 // weight before this round
-    uint32_t prev_chunk = 0xFFFFFFFFu;  // chunk of the page before this round
-    for (uint64_t base = r0; base < r1; base += 32) {
-        const uint64_t k = base + lane;
-        const uint32_t w = k < r1 ? page_weight(Rcount[Rlist[k]]) : 0u;
-        uint32_t x = w;                 // inclusive warp scan
+    if (p < F) {
+        const uint64_t *pS = pstart + (F + 1);
+        const uint64_t r0 = pstart[p], r1 = pstart[p + 1];
+        const uint64_t cid = r0 * kPageTuples / chunk_w + p;
+        uint64_t carry = 0;                 // weight before this round
+        uint32_t prev_chunk = 0xFFFFFFFFu;  // chunk of the page before this round
+        constexpr int U = 4;                // rounds of 32 pages loaded together
+        for (uint64_t base = r0; base < r1; base += 32 * U) {
+            uint32_t w[U];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+            for (int u = 0; u < U; u++) w[u] = base + 32 * u + lane < r1 ? Rlist[base + 32 * u + lane] : kNone;
+#pragma unroll
+            for (int u = 0; u < U; u++) w[u] = w[u] != kNone ? page_weight(Rcount[w[u]]) : 0u;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint64_t k = base + 32 * u + lane;
+                const uint32_t x = warp_incl_scan(w[u], lane);
+                const uint32_t ch = (uint32_t)((carry + x - w[u]) / chunk_w);
+                uint32_t before = __shfl_up_sync(0xffffffffu, ch, 1);
+                if (lane == 0) before = prev_chunk;
+                if (k < r1 && ch != before) wl.cstart[cid + ch] = k;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+                // the chunk of the last page so far (pages past the end weigh nothing and do not move it)
+                const uint32_t last = __ballot_sync(0xffffffffu, k < r1);
+                if (last) prev_chunk = __shfl_sync(0xffffffffu, ch, 31 - __clz(last));
+            }
         }
-        const uint64_t before = carry + x - w;
-        const uint32_t c = (uint32_t)(before / chunk_w);
-        uint32_t cprev = __shfl_up_sync(0xffffffffu, c, 1);
-        if (lane == 0) cprev = prev_chunk;
-        if (k < r1 && c != cprev) cstart[chunk_off[p] + c] = k;
-        carry += __shfl_sync(0xffffffffu, x, 31);
-        prev_chunk = __shfl_sync(0xffffffffu, c, 31);
+        if (lane == 0) {
+            const uint32_t rc = r1 > r0 ? prev_chunk + 1 : 0u;
+            const uint32_t sc = (uint32_t)((pS[p + 1] - pS[p] + s_pages - 1) / s_pages);
+            wl.rch[p] = rc;
+            wl.chunk_off[p] = (uint32_t)cid;
+            wl.items[p] = rc * sc;
+        }
     }
+    if (!scan) return;
+    __shared__ uint32_t tmp[32];
+    __shared__ bool last_block;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last_block = atomicAdd(&wl.ctr[2], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last_block) return;
+    __threadfence();
+    scan_list(wl.items, F, 0, wl.items_off, &wl.ctr[0], tmp);
 }
 
-__device__ __forceinline__ uint32_t find_part(const uint32_t *items_off, uint32_t F, uint32_t item) {
-    uint32_t lo = 0, hi = F;   // largest p with items_off[p] <= item
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (items_off[mid] <= item) lo = mid; else hi = mid;
-    }
-    return lo;
+static __global__ void __launch_bounds__(kScanThreads) items_scan(WorkList wl, uint32_t F) {
+    __shared__ uint32_t tmp[32];
+    scan_list(wl.items, F, blockIdx.x, wl.items_off, &wl.ctr[0], tmp);
 }
 
-// The same search by one warp, 32 probes per round: the largest i in [0, n)
+// The work list of F partitions; returns the launches it took.
+static int make_work_list(cudaStream_t st, const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount,
+                          uint32_t F, uint32_t chunk_w, uint32_t s_pages, const WorkList &wl) {
+    cudaMemsetAsync(wl.ctr, 0, 3 * sizeof(uint32_t), st);
+    part_chunks<<<(F + 31) / 32, 1024, 0, st>>>(pstart, Rlist, Rcount, F, chunk_w, s_pages, wl, F <= kScanThreads);
+    if (F <= kScanThreads) return 1;
+    items_scan<<<(F + kScanThreads - 1) / kScanThreads, kScanThreads, 0, st>>>(wl, F);
+    return 2;
+}
+
+// Search by one warp, 32 probes per round: the largest i in [0, n)
 // with off[i] <= v (off non-decreasing, off[0] <= v).  Three dependent rounds
 // for 2^14 entries instead of fourteen.
 __device__ __forceinline__ uint32_t warp_find(const uint32_t *off, uint32_t n, uint32_t v, int lane) {
@@ -144,26 +146,6 @@ __device__ __forceinline__ uint32_t warp_find(const uint32_t *off, uint32_t n, u
         hi = min(hi, lo + step);
     }
     return lo;
-}
-
-// Warp 0 takes the next work item: slots[0] = item, slots[1] = its partition,
-// slots[2] = the window of that partition (batched windows, else 0).
-__device__ __forceinline__ void take_item(uint32_t *work_counter, const uint32_t *items_off, uint32_t F,
-                                          uint32_t n_items, const uint32_t *wbase, uint32_t nwin,
-                                          volatile uint32_t *slots, int lane) {
-    uint32_t item = 0;
-    if (lane == 0) item = atomicAdd(work_counter, 1u);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    uint32_t p = 0, w = 0;
-    if (item < n_items) {
-        p = warp_find(items_off, F, item, lane);
-        if (wbase) w = warp_find(wbase, nwin, p, lane);
-    }
-    if (lane == 0) {
-        slots[0] = item;
-        slots[1] = p;
-        slots[2] = w;
-    }
 }
 
 // Page ranges of one work item (R chunk pages [rb, rb + nrpg) and S pages
@@ -180,12 +162,12 @@ __device__ __forceinline__ ItemGeo item_geo(const Args &a, uint32_t item, uint32
     const uint64_t r0 = pR[p], nrp = pR[p + 1] - r0;
     const uint64_t s0 = pS[p], nsp = pS[p + 1] - s0;
     const uint32_t sch = (uint32_t)((nsp + s_pages - 1) / s_pages);
-    const uint32_t local = item - a.items_off[p];
+    const uint32_t local = item - a.wl.items_off[p], rch = a.wl.rch[p];
     const uint32_t rc = local / sch, sc = local % sch;
-    const uint32_t cid = a.chunk_off[p] + rc;
+    const uint32_t cid = a.wl.chunk_off[p] + rc;
     ItemGeo g;
-    g.rb = a.cstart[cid];
-    const uint64_t re = rc + 1 < a.chunk_off[p + 1] - a.chunk_off[p] ? a.cstart[cid + 1] : r0 + nrp;
+    g.rb = a.wl.cstart[cid];
+    const uint64_t re = rc + 1 < rch ? a.wl.cstart[cid + 1] : r0 + nrp;
     g.nrpg = (uint32_t)(re - g.rb);
     g.sb = s0 + (uint64_t)sc * s_pages;
     g.nspg = (uint32_t)min((uint64_t)s_pages, nsp - (uint64_t)sc * s_pages);
@@ -238,11 +220,7 @@ struct JoinArgs {
     const uint8_t *Rcount, *Scount;
     const uint32_t *Rlist, *Slist;   // page lists grouped by digit
     const uint64_t *pstart;          // [2][F+1] page-list starts
-    const uint32_t *items_off;
-    const uint32_t *chunk_off;       // [F+1] first R chunk of each partition
-    const uint64_t *cstart;          // first page-list index of each R chunk
-    const uint32_t *n_items;
-    uint32_t *work_counter;
+    WorkList wl;
     unsigned long long *acc;         // [0] count, [1] checksum
     int *err;
     int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report a wait that ran out
@@ -307,7 +285,7 @@ radix_join_items(JoinArgs a) {
     uint64_t *red = reinterpret_cast<uint64_t *>(ptab + 4 * (kRMaxPages + 1));
     ItemRec *rec = reinterpret_cast<ItemRec *>(red + 64);                // [2]
 
-    const uint32_t n_items = *a.n_items;
+    const uint32_t n_items = a.wl.ctr[0];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kJoinThreads / 32;
     constexpr int kCtl = kWarps - 1;
@@ -316,11 +294,11 @@ radix_join_items(JoinArgs a) {
     // control warp: take the next item from the work counter into r
     auto take = [&](ItemRec *r) {
         uint32_t item = 0;
-        if (lane == 0) item = atomicAdd(a.work_counter, 1u);
+        if (lane == 0) item = atomicAdd(&a.wl.ctr[1], 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         uint32_t p = 0, w = 0;
         if (item < n_items) {
-            p = warp_find(a.items_off, F, item, lane);
+            p = warp_find(a.wl.items_off, F, item, lane);
             if (a.wacc) w = warp_find(a.wbase, a.nwin, p, lane);
         }
         if (lane == 0) {

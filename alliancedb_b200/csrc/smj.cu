@@ -50,10 +50,7 @@ struct SmjArgs {
     const uint8_t *Rcount, *Scount;
     const uint32_t *Rlist, *Slist;
     const uint64_t *pstart;          // [2][F+1]
-    const uint32_t *items_off, *chunk_off;
-    const uint64_t *cstart;
-    const uint32_t *n_items;
-    uint32_t *work_counter;
+    WorkList wl;
     unsigned long long *acc;
     int *err;
     int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report completed waits as run out
@@ -91,7 +88,7 @@ smj_items(SmjArgs a) {
     SmjRec *rec = reinterpret_cast<SmjRec *>(red + 112);     // [2]
     __shared__ uint32_t runn[2];   // length of R's run of a single S key, per item parity
 
-    const uint32_t n_items = *a.n_items;
+    const uint32_t n_items = a.wl.ctr[0];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kSmjThreads / 32;
     constexpr int kCtl = kWarps - 1;
@@ -101,10 +98,10 @@ smj_items(SmjArgs a) {
     // control warp: take the next item into r
     auto take = [&](SmjRec *r) {
         uint32_t item = 0;
-        if (lane == 0) item = atomicAdd(a.work_counter, 1u);
+        if (lane == 0) item = atomicAdd(&a.wl.ctr[1], 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         uint32_t p = 0;
-        if (item < n_items) p = warp_find(a.items_off, F, item, lane);
+        if (item < n_items) p = warp_find(a.wl.items_off, F, item, lane);
         if (lane == 0) {
             r->item = item;
             if (item < n_items) {
@@ -341,9 +338,7 @@ size_t smj_scratch(uint64_t nR, uint64_t nS, int part_fanout, int num_sms) {
     smj_bits(nR, part_fanout, &b1, &b2);
     const uint64_t F = 1ull << (b1 + b2);
     const uint64_t pages = paged_final_pool_pages(nR, nS, b1, b2, num_sms);
-    return paged_partition_scratch(nR, nS, b1, b2, num_sms) + Workspace::need(F, 4) * 2 +
-           Workspace::need(F + 1, 4) * 2 + Workspace::need(pages * kPageTuples / kSmjChunkW + F + 1, 8) +
-           Workspace::need(2, 4);
+    return paged_partition_scratch(nR, nS, b1, b2, num_sms) + WorkList::bytes(F, pages, kSmjChunkW);
 }
 
 int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool /*multipass*/, unsigned long long *acc) {
@@ -357,17 +352,9 @@ int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool /*multipass*/,
     ADB_CK(mark(ctx, 1));
 
     const uint32_t F = po.Fout;
-    uint32_t *rch = ctx->ws.take<uint32_t>(F);
-    uint32_t *sch = ctx->ws.take<uint32_t>(F);
-    uint32_t *items_off = ctx->ws.take<uint32_t>(F + 1);
-    uint32_t *chunk_off = ctx->ws.take<uint32_t>(F + 1);
-    uint64_t *cstart = ctx->ws.take<uint64_t>(po.pool_pages * kPageTuples / kSmjChunkW + F + 1);
-    uint32_t *ctr = ctx->ws.take<uint32_t>(2);
-    ADB_CK(cudaMemsetAsync(ctr, 0, 2 * sizeof(uint32_t), st));
-    part_rslots<<<(F + 7) / 8, 256, 0, st>>>(po.pstart, po.R.plist, po.R.pcount, F, kSmjChunkW, kSmjSPages, rch,
-                                             sch);
-    make_items_paged<<<1, 1024, 0, st>>>(rch, sch, F, items_off, chunk_off, ctr);
-    part_rchunks<<<(F + 7) / 8, 256, 0, st>>>(po.pstart, po.R.plist, po.R.pcount, F, kSmjChunkW, chunk_off, cstart);
+    WorkList wl;
+    wl.take(ctx->ws, F, po.pool_pages, kSmjChunkW);
+    ctx->kernels += make_work_list(st, po.pstart, po.R.plist, po.R.pcount, F, kSmjChunkW, kSmjSPages, wl);
     ADB_CK(cudaGetLastError());
     ADB_CK(mark(ctx, 2));
 
@@ -375,15 +362,14 @@ int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool /*multipass*/,
     a.Rpages = po.R.pages; a.Spages = po.S.pages;
     a.Rcount = po.R.pcount; a.Scount = po.S.pcount;
     a.Rlist = po.R.plist; a.Slist = po.S.plist;
-    a.pstart = po.pstart; a.items_off = items_off; a.chunk_off = chunk_off; a.cstart = cstart;
-    a.n_items = ctr; a.work_counter = ctr + 1;
+    a.pstart = po.pstart; a.wl = wl;
     a.acc = acc; a.err = reinterpret_cast<int *>(acc + 2);
     a.waits_run_out = j.test_flags & ADB_TEST_WAITS_RUN_OUT;
     a.F = F;
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;
     smj_items<<<ctx->num_sms * kSmjBlocks, kSmjThreads, kSmjSmem, st>>>(a);
     ADB_CK(cudaGetLastError());
-    ctx->kernels += 4;
+    ctx->kernels += 1;
     return ADB_OK;
 }
 
