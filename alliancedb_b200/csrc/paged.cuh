@@ -113,10 +113,11 @@ __host__ __device__ __forceinline__ uint32_t unit_pages_for(uint64_t pages1_both
 }
 
 // Shared memory of one pass:
-//   stage[kPTile] u64 | cnt[2][F] | toff[F] | lim[F] | b1[F] | b2[F] | npos[F] u32 | misc[48] u32
+//   stage[kPTile] u64 | cnt[2][F] | toff[F] | lim[F] | b1[F] | b2[F] | npos[F] | npages[F] u32 | misc[48] u32
 //   | paged input only: upage[kMaxUnitPages] u32 | ucnt[kMaxUnitPages] u8
 __host__ __device__ __forceinline__ size_t pass_smem(uint32_t F, bool paged) {
-    return (size_t)kPTile * 8 + (size_t)F * 4 * 7 + 48 * 4 + (paged ? (size_t)kMaxUnitPages * 5 : 0);
+    return (size_t)kPTile * 8 + (size_t)F * 4 * 8 + 48 * 4 +
+           (paged ? (size_t)kMaxUnitPages * 5 : 0);
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(kThreads, kPassMinBlocks)
 partition_pass(PassArgs a) {
     constexpr bool kPaged = kMode == 1;
     constexpr int kPer = kPTile / kThreads;
+    constexpr uint32_t kAll = (1u << kPer) - 1u;
     static_assert(kPer % 2 == 0 && kThreads % 32 == 0 && (kPTile / kPageTuples) % (kThreads / 32) == 0, "tile shape");
     static_assert((1u << kMaxPassBits) <= (uint32_t)kThreads, "one digit per thread in step B");
     extern __shared__ __align__(16) unsigned char smem[];
@@ -193,7 +195,8 @@ partition_pass(PassArgs a) {
     uint32_t *b1 = lim + F;
     uint32_t *b2 = b1 + F;
     uint32_t *npos = b2 + F;
-    uint32_t *misc = npos + F;          // [0] pool pages taken, [1] tuples in the tile,
+    uint32_t *npages = npos + F;        // pages the digit has taken
+    uint32_t *misc = npages + F;        // [0] pool pages taken, [1] tuples in the tile,
                                         // [8..24) per-warp totals of the digit scan,
                                         // [kHotWord] hot digit
     uint32_t *upage = misc + 48;        // paged input: this unit's pages
@@ -209,6 +212,7 @@ partition_pass(PassArgs a) {
         cnt[d] = 0;
         cnt[F + d] = 0;
         npos[d] = kNone;
+        npages[d] = 0;
     }
     if (tid == 0) {
         misc[0] = 0;
@@ -222,15 +226,18 @@ partition_pass(PassArgs a) {
         }
     __syncthreads();
 
-    // ---- tiles: kPTile flat tuples, or kPTile / 64 input pages
+    // ---- tiles: kPTile flat tuples, or kPTile / 64 input pages.  Whole flat
+    // tiles take loads, ranks and staging without bounds checks (pass 1 at 2^27:
+    // 1.033 -> 0.988 ms; the same for paged tiles, by whole pages of a warp, made
+    // pass 2 2 % slower).
     constexpr uint64_t kStep = kPaged ? (uint64_t)(kPTile / kPageTuples) : (uint64_t)kPTile;
     const bool vec = !kPaged && ((reinterpret_cast<uintptr_t>(in.in + b) & 15) == 0);
     uint64_t w[kPer];
     uint32_t valid = 0;   // bit k: w[k] holds a tuple
     auto load_tile = [&](uint64_t t0) {
-        valid = 0;
         if (kPaged) {
             // tuple pair k of this thread: slots 2 (tid % 32), +1 of the tile's page k * (kThreads / 32) + tid / 32
+            valid = 0;
             const uint32_t slot = 2 * (tid & 31);
 #pragma unroll
             for (int k = 0; k < kPer / 2; k++) {
@@ -249,22 +256,17 @@ partition_pass(PassArgs a) {
                     valid |= (ok ? 1u : 0u) << (2 * k);
                 }
             }
-        } else if (vec) {
+        } else if (vec && t0 + kStep <= e) {
+            valid = kAll;
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(in.in + t0) + tid;
 #pragma unroll
             for (int k = 0; k < kPer / 2; k++) {
-                const uint64_t i = t0 + 2 * ((uint64_t)k * kThreads + tid);
-                if (i + 1 < e) {
-                    const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(in.in + i));
-                    w[2 * k] = v.x;
-                    w[2 * k + 1] = v.y;
-                    valid |= 3u << (2 * k);
-                } else {
-                    w[2 * k] = i < e ? ld_stream(in.in + i) : 0;
-                    w[2 * k + 1] = 0;
-                    valid |= (i < e ? 1u : 0u) << (2 * k);
-                }
+                const ulonglong2 v = __ldcs(src + k * kThreads);
+                w[2 * k] = v.x;
+                w[2 * k + 1] = v.y;
             }
         } else {
+            valid = 0;
 #pragma unroll
             for (int k = 0; k < kPer; k++) {
                 const uint64_t i = t0 + (uint64_t)k * kThreads + tid;
@@ -306,7 +308,13 @@ partition_pass(PassArgs a) {
         //    would otherwise serialise on one shared counter.
         uint32_t rk[kPer / 2];   // two 16-bit ranks per word
         const uint32_t hot = misc[kHotWord];   // block-uniform
-        if (hot == kNone) {
+        if (!kPaged && hot == kNone && valid == kAll) {
+#pragma unroll
+            for (int k = 0; k < kPer; k++) {
+                const uint32_t r = atomicAdd(&c[dig(w[k])], 1u);
+                if (k & 1) rk[k / 2] |= r << 16; else rk[k / 2] = r;
+            }
+        } else if (hot == kNone) {
 #pragma unroll
             for (int k = 0; k < kPer; k++) {
                 const uint32_t r = (valid >> k) & 1 ? atomicAdd(&c[dig(w[k])], 1u) : 0u;
@@ -357,6 +365,7 @@ partition_pass(PassArgs a) {
                 const uint32_t nx = (pool_base + first) * kPageTuples - room;
                 b2[d] = nx - off;
                 np = nx + L;
+                npages[d] += need;
             }
             if (L && (np & (kPageTuples - 1)) == 0) np = kNone;   // page exactly full
             npos[d] = np;
@@ -444,10 +453,16 @@ partition_pass(PassArgs a) {
         }
         __syncthreads();
         // C. stage the tile grouped by digit
+        if (!kPaged && valid == kAll) {
 #pragma unroll
-        for (int k = 0; k < kPer; k++)
-            if ((valid >> k) & 1)
+            for (int k = 0; k < kPer; k++)
                 stage[toff[dig(w[k])] + ((rk[k / 2] >> ((k & 1) * 16)) & 0xFFFFu)] = w[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < kPer; k++)
+                if ((valid >> k) & 1)
+                    stage[toff[dig(w[k])] + ((rk[k / 2] >> ((k & 1) * 16)) & 0xFFFFu)] = w[k];
+        }
         const uint32_t tile_n = misc[1];
         if (t0 + kStep < e) {   // in flight during D; the tile after that into L2
             prefetch_tile(t0 + 2 * kStep);
@@ -479,17 +494,12 @@ partition_pass(PassArgs a) {
             if (p & 1) o.pages[p] = ~0ULL;
         }
     }
-    // F. pages per digit of this CTA (its log was written by this block)
-    const uint32_t used = misc[0];
-    for (uint32_t d = tid; d < F; d += kThreads) toff[d] = 0;
-    __syncthreads();
-    for (uint32_t k = tid; k < used; k += kThreads) atomicAdd(&toff[o.log[pool_base + k] - dbase], 1u);
-    __syncthreads();
+    // F. pages per digit of this CTA
     uint32_t *tot = a.totals + (size_t)relidx * a.Dtot;
     for (uint32_t d = tid; d < F; d += kThreads)
-        if (toff[d]) o.doff[pool_base + d] = atomicAdd(&tot[dbase + d], toff[d]);
+        if (npages[d]) o.doff[pool_base + d] = atomicAdd(&tot[dbase + d], npages[d]);
     if (tid == 0) {
-        o.nlog[g] = used;
+        o.nlog[g] = misc[0];
         o.udesc[g] = make_uint2(dbase, F);
     }
 }
