@@ -17,7 +17,6 @@
 namespace adb {
 
 int radix_set_attrs();
-int smj_set_attrs();
 int eager_set_attrs();
 int batch_set_attrs();
 int small_set_attrs();
@@ -178,7 +177,6 @@ Context *ctx_create(int dev, int *status) {
     if (cudaDeviceSynchronize() != cudaSuccess) goto fail;   // the library's stream does not wait for the clear
     {
         int s = radix_set_attrs();
-        if (s == ADB_OK) s = smj_set_attrs();
         if (s == ADB_OK) s = eager_set_attrs();
         if (s == ADB_OK) s = batch_set_attrs();
         if (s == ADB_OK) s = small_set_attrs();
@@ -336,7 +334,7 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
             if (npo_partitioned(nR, nS, p ? p->radix_bits : 0))
                 return radix_scratch(nR, nS, radix_bits_for(nR, 0), num_sms);
             return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
-        case Family::SortMerge: return smj_scratch(nR, nS, p ? p->part_fanout : 0, num_sms);
+        case Family::SortMerge: return radix_scratch(nR, nS, sort_bits_for(nR, p ? p->part_fanout : 0), num_sms);
         case Family::Shj:
         case Family::Pmj:
             return eager_scratch(nR, nS, a->fam, a->model, p && p->nthreads ? (int)p->nthreads : 1,
@@ -350,12 +348,13 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), false, acc);
+            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), PartJoin::Chain, acc);
         case Family::Npo:
             if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0))
-                return run_radix(ctx, j, radix_bits_for(j.nR, 0), true, acc);
+                return run_radix(ctx, j, radix_bits_for(j.nR, 0), PartJoin::HashedChain, acc);
             return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
-        case Family::SortMerge: return run_smj(ctx, j, p ? p->part_fanout : 0, a->model == 1, acc);
+        case Family::SortMerge:
+            return run_radix(ctx, j, sort_bits_for(j.nR, p ? p->part_fanout : 0), PartJoin::Sorted, acc);
         case Family::Shj:
         case Family::Pmj:
             return run_eager(ctx, j, a->fam, a->model, eager_batch(p), p && p->nthreads ? (int)p->nthreads : 0,

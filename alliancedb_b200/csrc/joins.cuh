@@ -38,20 +38,20 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
 bool small_fits(uint64_t nR, uint64_t nS);
 int run_small(Context *ctx, const DevJoin &j);
 
-// ---- radix (PRO / RJ_st / PRH / PRHO) ----
+// ---- partitioned joins (PRO / RJ_st / PRH / PRHO, large NPO, m-way / m-pass / m-way+skew) ----
 int radix_bits_for(uint64_t nR, int requested);
+int sort_bits_for(uint64_t nR, int part_fanout);   // m-way / m-pass: joinconfig_t.PARTFANOUT, 0 = chosen
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
-int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned long long *acc);
+// How a partition is joined: a chained table over digits of the key's low bits
+// or of its hash, or a counting sort (the sort-merge names).
+enum class PartJoin { Chain, HashedChain, Sorted };
+int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned long long *acc);
 
 // ---- NPO / NPO_st ----
 bool npo_partitioned(uint64_t nR, uint64_t nS, int requested);
 uint32_t npo_region_bits(uint64_t nR, int requested);
 size_t npo_scratch(uint64_t nR, uint64_t nS, int region_bits, int num_sms);
 int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long *acc);
-
-// ---- m-way / m-pass ----
-size_t smj_scratch(uint64_t nR, uint64_t nS, int part_fanout, int num_sms);
-int run_smj(Context *ctx, const DevJoin &j, int part_fanout, bool multipass, unsigned long long *acc);
 
 // ---- eager SHJ / PMJ over one window given as arrival-ordered relations ----
 size_t eager_scratch(uint64_t nR, uint64_t nS, Family fam, int model, int nthreads, int group_size);

@@ -35,7 +35,6 @@ constexpr int kPTile = 4096;                    // tuples per tile
 constexpr int kPassThreads = 512;               // threads per CTA of a pass
 constexpr int kPassMinBlocks = 2;               // CTAs per SM the registers are sized for
 constexpr uint32_t kMaxPassBits = 9;            // <= 512 partitions per pass
-constexpr uint32_t kSmallPassBits = 8;          // sort-merge: one pass up to 2^8 partitions
 constexpr uint32_t kMaxUnitPages = 2048;        // pass-2 work unit: <= 128K tuples
 constexpr uint32_t kMinUnitPages = kPTile / 64;  // one tile
 constexpr uint32_t kNone = 0xFFFFFFFFu;

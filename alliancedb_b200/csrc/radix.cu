@@ -1,5 +1,5 @@
-// radix.cu -- paged partitioning front end and the partitioned hash joins
-// (PRO, RJ_st, PRH, PRHO).
+// radix.cu -- paged partitioning front end and the partitioned joins (PRO, RJ_st,
+// PRH, PRHO; NPO beyond L2; m-way, m-pass, m-way+skew).
 //
 // Reference flow: join_init_run (hashing/joins/parallel_radix_join.cpp:1488-1701)
 // spawns prj_thread (:981-1473): parallel pass-1 partitioning, task-queued
@@ -45,16 +45,26 @@ static void launch_pass(const PassArgs &a, uint32_t F, int G, bool paged, cudaSt
     else partition_pass<0, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
 }
 
+// Fan-out bits: partitions of at most 2^13 tuples (one R chunk), and below that
+// size up to 2^8 partitions, down to 256 tuples each, so that the join's items
+// fill the SMs.  Device time of PRO / m-way, us, four of each key on both sides,
+// at these bits (and at 2^12 tuples a partition, or one bit less): 2^16 - / 53
+// (4 bits 72), 2^18 64 / 71 (6 bits 73 / 83), 2^20 102 / 110 (7 bits 108 / 118), 2^21 133 /
+// 167 (9 bits 166 / 186), 2^22 228 / 256 (8 bits 223 / 273), 2^23 - / 410 (9 bits 450).
 int radix_bits_for(uint64_t nR, int requested) {
     if (requested > 0) return requested > 15 ? 15 : requested;
-    // one pass (<= 9 bits) leaves up to one partial page per CTA in every
-    // partition, so it aims at half a join chunk; two passes at a full chunk
-    constexpr uint64_t kTarget = kRSlots >= 16384 ? 16384 : 8192;   // power of two <= kRSlots
-    int b = (int)ceil_log2_u64((nR + kTarget / 2 - 1) / (kTarget / 2));
-    if (b > (int)kMaxPassBits) b = (int)ceil_log2_u64((nR + kTarget - 1) / kTarget);
+    const int full = (int)ceil_log2_u64((nR + 8191) / 8192), fill = (int)ceil_log2_u64((nR + 255) / 256);
+    int b = fill > 8 ? 8 : fill;
+    if (full > b) b = full;
     if (b < 1) b = 1;
     if (b > 15) b = 15;
     return b;
+}
+
+// m-way / m-pass: the fan-out joinconfig_t.PARTFANOUT asks for, rounded up to a
+// power of two (at most 2^15), else as above.
+int sort_bits_for(uint64_t nR, int part_fanout) {
+    return radix_bits_for(nR, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -237,7 +247,8 @@ size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms) {
     return paged_partition_scratch(nR, nS, b1, b2, num_sms) + WorkList::bytes(F, pagesR, kChunkW);
 }
 
-int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned long long *acc) {
+int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned long long *acc) {
+    const bool hashed = kind != PartJoin::Chain;
     cudaStream_t st = ctx->stream;
     uint32_t b1, b2;
     split_bits(bits, &b1, &b2);
@@ -266,10 +277,16 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, bool hashed, unsigned lo
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;
     a.wbase = nullptr; a.wbits = nullptr; a.nwin = 0; a.wacc = nullptr;
     const int grid = ctx->num_sms * kJoinMinBlocks;
-    if (j.mat && hashed) radix_join_items<true, true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
-    else if (j.mat) radix_join_items<true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
-    else if (hashed) radix_join_items<false, true><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
-    else radix_join_items<false><<<grid, kJoinThreads, kJoinSmem, st>>>(a);
+    auto launch = [&](auto kernel) { kernel<<<grid, kJoinThreads, kJoinSmem, st>>>(a); };
+    switch (kind) {
+        case PartJoin::Chain: j.mat ? launch(radix_join_items<true>) : launch(radix_join_items<false>); break;
+        case PartJoin::HashedChain:
+            j.mat ? launch(radix_join_items<true, true>) : launch(radix_join_items<false, true>);
+            break;
+        case PartJoin::Sorted:
+            j.mat ? launch(radix_join_items<true, true, true>) : launch(radix_join_items<false, true, true>);
+            break;
+    }
     ADB_CK(cudaGetLastError());
     ctx->kernels += 1;
     return ADB_OK;
@@ -286,6 +303,8 @@ int radix_set_attrs() {
     ADB_CK(cudaFuncSetAttribute(radix_join_items<true>, attr, (int)kJoinSmem));
     ADB_CK(cudaFuncSetAttribute(radix_join_items<false, true>, attr, (int)kJoinSmem));
     ADB_CK(cudaFuncSetAttribute(radix_join_items<true, true>, attr, (int)kJoinSmem));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<false, true, true>, attr, (int)kJoinSmem));
+    ADB_CK(cudaFuncSetAttribute(radix_join_items<true, true, true>, attr, (int)kJoinSmem));
     return ADB_OK;
 }
 

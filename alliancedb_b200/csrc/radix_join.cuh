@@ -3,6 +3,8 @@
 // Replaces, per partition pair (R_p, S_p) produced by paged.cuh:
 //   bucket_chaining_join   hashing/joins/parallel_radix_join.cpp:291-354   (PRO, RJ_st)
 //   histogram_join         hashing/joins/parallel_radix_join.cpp:373-432   (PRH, PRHO)
+//   sorting and merge phases  sorting/joins/sortmergejoin_multiway.cpp:499-660, merge_join
+//                          sorting/joins/common_functions.cpp:298-372      (m-way, m-pass, m-way+skew)
 // (one chained table for all four: a histogram table, built with two passes
 // over R and a scan, took 0.35 ms where the chained one took 0.15 at 2^24)
 // and the task-queue loop of prj_thread (:1409-1416) with a persistent kernel
@@ -174,38 +176,6 @@ __device__ __forceinline__ ItemGeo item_geo(const Args &a, uint32_t item, uint32
     return g;
 }
 
-// --- bulk async copy helpers (sm_90+ PTX) -----------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, uint32_t bytes, uint64_t *bar) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst_smem);
-    const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-        "l"(src_gmem), "r"(bytes), "r"(b)
-        : "memory");
-}
-// Bounded wait on an mbarrier phase; false when the bound runs out.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    for (uint32_t it = 0; it < (1u << 22); it++) {
-        uint32_t done;
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(done)
-            : "r"(a), "r"(phase)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
 // Shared memory: tup[kRSlots] u64 | heads[2^kMaxHeadsLog2] u32 | two page tables
 // {pg[kRMaxPages + 1] u32, dst << 8 | count [kRMaxPages + 1] u32} | reduction and
 // two item records.
@@ -275,7 +245,7 @@ struct ItemRec {
 // whole call 7.86 -> 6.01 ms.  Adding a warp's matches together after the walk
 // instead of as they are found: 0.83 / 1.14, and 1.27 instead of 1.23 ms with
 // every key four times in both relations (2^26), so not kept.
-template <bool kMat, bool kHashed = false>
+template <bool kMat, bool kHashed = false, bool kSorted = false>
 __global__ void __launch_bounds__(kJoinThreads, kJoinMinBlocks)
 radix_join_items(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -416,7 +386,7 @@ radix_join_items(JoinArgs a) {
         auto next_of = [&](uint32_t w) { return kHashed ? w >> (32 - link) : w & lmask; };
         auto same = [&](uint32_t w, uint32_t x) { return kHashed ? (w ^ x) << link == 0 : (w ^ x) < lim; };
         for (uint32_t i = threadIdx.x; i < ((1u << lnb) + 3) / 4; i += kJoinThreads)
-            reinterpret_cast<uint4 *>(heads)[i] = make_uint4(kNone, kNone, kNone, kNone);
+            reinterpret_cast<uint4 *>(heads)[i] = kSorted ? make_uint4(0, 0, 0, 0) : make_uint4(kNone, kNone, kNone, kNone);
         if (a.waits_run_out && threadIdx.x == 0) atomicExch(a.err, 1);
         __syncthreads();
 
@@ -426,25 +396,57 @@ radix_join_items(JoinArgs a) {
             return tword(linked(x, old == kNone ? s : old), tpay(t));
         };
         constexpr int kB = 4;
-        for (uint32_t k0 = warp; k0 < nrpg; k0 += kB * kWarps) {
-            ulonglong2 r[kB];
-            uint32_t v[kB];
+        // f(slot, the lane's two tuples, whether the second is one) for every page of the chunk
+        auto each_page = [&](auto f) {
+            for (uint32_t k0 = warp; k0 < nrpg; k0 += kB * kWarps) {
+                ulonglong2 r[kB];
+                uint32_t v[kB];
 #pragma unroll
-            for (int j = 0; j < kB; j++) {
-                const uint32_t k = k0 + j * kWarps;
-                v[j] = k < nrpg ? tpk[k] : 0u;
-                if (2 * lane < (int)(v[j] & 0xFFu))
-                    r[j] = __ldcs(reinterpret_cast<const ulonglong2 *>(a.Rpages + (uint64_t)tpg[k] * kPageTuples) + lane);
+                for (int j = 0; j < kB; j++) {
+                    const uint32_t k = k0 + j * kWarps;
+                    v[j] = k < nrpg ? tpk[k] : 0u;
+                    if (2 * lane < (int)(v[j] & 0xFFu))
+                        r[j] = __ldcs(reinterpret_cast<const ulonglong2 *>(a.Rpages + (uint64_t)tpg[k] * kPageTuples) +
+                                      lane);
+                }
+#pragma unroll
+                for (int j = 0; j < kB; j++)
+                    if (2 * lane < (int)(v[j] & 0xFFu))
+                        f((v[j] >> 8) + 2 * lane, r[j], 2 * lane + 1 < (int)(v[j] & 0xFFu));
             }
-#pragma unroll
-            for (int j = 0; j < kB; j++) {
-                const uint32_t s = (v[j] >> 8) + 2 * lane;
-                if (2 * lane < (int)(v[j] & 0xFFu)) {
-                    r[j].x = enter(s, r[j].x);
-                    if (2 * lane + 1 < (int)(v[j] & 0xFFu)) r[j].y = enter(s + 1, r[j].y);
-                    *reinterpret_cast<ulonglong2 *>(tup + s) = r[j];
+        };
+        if (kSorted) {
+            each_page([&](uint32_t, const ulonglong2 &r, bool two) {
+                atomicAdd(&heads[bucket(hash(r.x))], 1u);
+                if (two) atomicAdd(&heads[bucket(hash(r.y))], 1u);
+            });
+            __syncthreads();
+            {   // bucket starts << 16: thread t's buckets t, t + 512, .. follow one another (any
+                // order of the buckets will do, and this one has no bank conflicts)
+                uint32_t loc = 0, tot;
+                for (uint32_t d = threadIdx.x; d <= bmask; d += kJoinThreads) loc += heads[d];
+                uint32_t at = block_exclusive_scan(loc, reinterpret_cast<uint32_t *>(red), &tot);
+                for (uint32_t d = threadIdx.x; d <= bmask; d += kJoinThreads) {
+                    const uint32_t n = heads[d];
+                    heads[d] = at << 16;
+                    at += n;
                 }
             }
+            __syncthreads();
+            each_page([&](uint32_t, const ulonglong2 &r, bool two) {
+                auto place = [&](uint64_t t) {
+                    const uint32_t h = atomicAdd(&heads[bucket(hash(t))], 1u);   // start << 16 | placed
+                    tup[(h >> 16) + (h & 0xFFFFu)] = t;
+                };
+                place(r.x);
+                if (two) place(r.y);
+            });
+        } else {
+            each_page([&](uint32_t s, ulonglong2 &r, bool two) {
+                r.x = enter(s, r.x);
+                if (two) r.y = enter(s + 1, r.y);
+                *reinterpret_cast<ulonglong2 *>(tup + s) = r;
+            });
         }
         __syncthreads();
 
@@ -460,20 +462,28 @@ radix_join_items(JoinArgs a) {
             auto probe = [&](uint64_t s) {
                 const uint32_t key = tkey(s), x = hash(s);
                 uint32_t at = heads[bucket(x)];
-                if (at == kNone) return;
+                if (at == (kSorted ? 0u : kNone)) return;
                 const uint64_t sh = s_half(key, tpay(s));
+                auto add = [&](uint64_t r) {
+                    acc.sum += pair_hash_pre(key, tpay(r), sh);
+                    matches++;
+                    if (kMat) {
+                        const unsigned long long m = atomicAdd(a.mat_n, 1ull);
+                        if (m < a.mat_cap) a.mat[m] = s;
+                    }
+                };
+                if (kSorted) {
+                    uint32_t n = at & 0xFFFFu;
+                    for (at >>= 16; n; n--, at++) {
+                        const uint64_t r = tup[at];
+                        if (tkey(r) == key) add(r);
+                    }
+                    return;
+                }
                 while (true) {
                     const uint64_t r = tup[at];
                     const uint32_t nx = next_of(tkey(r));
-                    if (same(tkey(r), x)) {
-                        
-                        acc.sum += pair_hash_pre(key, tpay(r), sh);
-                        matches++;
-                        if (kMat) {
-                            const unsigned long long m = atomicAdd(a.mat_n, 1ull);
-                            if (m < a.mat_cap) a.mat[m] = s;
-                        }
-                    }
+                    if (same(tkey(r), x)) add(r);
                     if (nx == at) break;
                     at = nx;
                 }

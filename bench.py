@@ -61,9 +61,9 @@ KERNELS = {
               1: ("partition_pass<1,512> (pass 2)", 16, (276288768 + 214363648) / 2**25),
               3: ("radix_join_items", 8, (273622272 + 3668736) / 2**25)},
     "npo": {1: ("npo_build", 8, None), 3: ("npo_probe", 8, None)},
-    "smj": {0: ("partition_pass (both passes)", 32,
-                (271074048 + 215111680 + 279591680 + 219554048) / 2**25),
-            3: ("smj_items", 8, (282003456 + 3525376) / 2**25)},
+    "smj": {0: ("partition_pass<0,512,hashed> (pass 1)", 16, None),
+            1: ("partition_pass<1,512,hashed> (pass 2)", 16, None),
+            3: ("radix_join_items (sort + merge)", 8, None)},
 }
 
 
