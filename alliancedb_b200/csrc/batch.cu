@@ -251,7 +251,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ADB_CK(cudaMemsetAsync(wacc, 0, (2 * W + 8) * 8, st));
     ADB_CK(cudaMemsetAsync(tot, 0, 2ull * Dt * 4, st));
     ADB_CK(cudaMemsetAsync(wl.ctr, 0, 12, st));
-    partition_pass<2, kPassThreads><<<dim3(G, 2), kPassThreads, pass_smem(1u << kMaxPassBits, false), st>>>(a);
+    partition_pass<2, kPassThreads, kSegTile><<<dim3(G, 2), kPassThreads, pass_smem(kSegTile, 1u << kMaxPassBits, false), st>>>(a);
     ADB_CK(cudaGetLastError());
     dscan<uint64_t>(st, tot, Dt, pstart, bsum64);
     dscan<uint64_t>(st, tot + Dt, Dt, pstart + (Dt + 1), bsum64);
@@ -303,8 +303,8 @@ static int batch_join_all(Context *ctx, const uint64_t *dR, const uint64_t *r_of
 }
 
 int batch_set_attrs() {
-    ADB_CK(cudaFuncSetAttribute(partition_pass<2, kPassThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)pass_smem(1u << kMaxPassBits, false)));
+    ADB_CK(cudaFuncSetAttribute(partition_pass<2, kPassThreads, kSegTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)pass_smem(kSegTile, 1u << kMaxPassBits, false)));
     return ADB_OK;
 }
 

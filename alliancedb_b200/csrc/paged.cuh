@@ -11,7 +11,7 @@
 //   * output goes to 512-byte pages (64 tuples) taken from a per-CTA pool, a
 //     partition's pages chained through the CTA's page log, so partitions
 //     need not be contiguous and their sizes need not be known in advance;
-//   * each tile of 4096 tuples is counting-sorted by digit in shared memory
+//   * each tile of 6144 or 8192 tuples is counting-sorted by digit in shared memory
 //     (the role of the reference's software write-combining buffers, its
 //     _optimized partitioner), then copied out so that each partition's
 //     tuples form one contiguous stream through its pages: warps store
@@ -31,14 +31,17 @@
 namespace adb {
 
 constexpr int kPageTuples = 64;                 // 512-byte pages
-constexpr int kPTile = 4096;                    // tuples per tile
-constexpr int kPassThreads = 512;               // threads per CTA of a pass
-constexpr int kPassMinBlocks = 2;               // CTAs per SM the registers are sized for
+constexpr int kPassThreads = 512;               // threads per CTA of a pass, two CTAs per SM
+constexpr int kPassMinBlocks = 2;
+constexpr int kFlatTile = 6144;                 // tuples per tile: flat input with a second pass to follow,
+constexpr int kPagedTile = 8192;                //   paged input,
+constexpr int kSegTile = 8192;                  //   segmented input,
+constexpr int kWideThreads = 1024;              //   flat input in a single pass (one CTA per SM)
+constexpr int kWideTile = 8192;
 constexpr uint32_t kMaxPassBits = 9;            // <= 512 partitions per pass
 constexpr uint32_t kMaxUnitPages = 2048;        // pass-2 work unit: <= 128K tuples
-constexpr uint32_t kMinUnitPages = kPTile / 64;  // one tile
+constexpr uint32_t kMinUnitPages = kPagedTile / 64;  // one tile
 constexpr uint32_t kNone = 0xFFFFFFFFu;
-constexpr uint32_t kHotRun = kPTile / 2;        // a digit above this many tuples of a tile is hot
 constexpr uint32_t kHotWord = 40;               // misc[] word of the hot digit
 
 // Pages written by one pass for one relation.
@@ -112,10 +115,10 @@ __host__ __device__ __forceinline__ uint32_t unit_pages_for(uint64_t pages1_both
 }
 
 // Shared memory of one pass:
-//   stage[kPTile] u64 | cnt[2][F] | toff[F] | lim[F] | b1[F] | b2[F] | npos[F] | npages[F] u32 | misc[48] u32
+//   stage[tile] u64 | cnt[2][F] | toff[F] | lim[F] | b1[F] | b2[F] | npos[F] | npages[F] u32 | misc[48] u32
 //   | paged input only: upage[kMaxUnitPages] u32 | ucnt[kMaxUnitPages] u8
-__host__ __device__ __forceinline__ size_t pass_smem(uint32_t F, bool paged) {
-    return (size_t)kPTile * 8 + (size_t)F * 4 * 8 + 48 * 4 +
+__host__ __device__ __forceinline__ size_t pass_smem(int tile, uint32_t F, bool paged) {
+    return (size_t)tile * 8 + (size_t)F * 4 * 8 + 48 * 4 +
            (paged ? (size_t)kMaxUnitPages * 5 : 0);
 }
 
@@ -129,7 +132,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
 }
 
 // One pass over one input unit (a flat chunk, a unit of input pages, or a
-// unit of a segment).  Per tile of up to kPTile tuples:
+// unit of a segment).  Per tile of up to kTile tuples:
 //   A  every thread ranks its tuples within their digit (shared atomics on
 //      cnt[tile parity][d]);
 //   B  warp 0 (up to 32 digits, one per lane) or warps 0 .. F/32 - 1 (one
@@ -148,14 +151,24 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
 // still in L2.  Three barriers per tile (four above 32 digits); the next
 // tile's loads are in flight during D.  kMode: 0 flat input, 1 paged input
 // (pass 2), 2 segmented flat input (batched windows).  kHashed: the digit is
-// taken from key * kFibMul instead of the key (the table regions of NPO).
-template <int kMode, int kThreads, bool kHashed = false>
-__global__ void __launch_bounds__(kThreads, kPassMinBlocks)
+// taken from key * kFibMul instead of the key.
+//
+// Bound: shared-memory data wavefronts (about 23 per 32 tuples, the pipe 73 %
+// busy in pass 1 with 4096-tuple tiles) and, between them, the barriers around
+// B.  Larger tiles give B more tuples to share and D longer runs, so each kind
+// takes the largest tile whose tuples, kTile / kThreads 64-bit registers, leave
+// 64 registers enough for the rest.  Two passes of 2^7 digits, 2^27 x 2^27, ms
+// at tiles of 4096 / 6144 / 8192: pass 1 0.991 / 0.953 / 0.966, pass 2 1.162 /
+// 1.096 / 1.069 (10240: 1.186, spills); 512 batched windows of 2^10 .. 2^22
+// tuples, whole call 5.94 / 5.67 / 5.51 (10240: 5.78).
+template <int kMode, int kThreads, int kTile, bool kHashed = false>
+__global__ void __launch_bounds__(kThreads, kThreads == kWideThreads ? 1 : kPassMinBlocks)
 partition_pass(PassArgs a) {
     constexpr bool kPaged = kMode == 1;
-    constexpr int kPer = kPTile / kThreads;
+    constexpr int kPer = kTile / kThreads;
+    constexpr uint32_t kHotRun = kTile / 2;   // a digit above this many tuples of a tile is hot
     constexpr uint32_t kAll = (1u << kPer) - 1u;
-    static_assert(kPer % 2 == 0 && kThreads % 32 == 0 && (kPTile / kPageTuples) % (kThreads / 32) == 0, "tile shape");
+    static_assert(kPer % 2 == 0 && kThreads % 32 == 0 && (kTile / kPageTuples) % (kThreads / 32) == 0, "tile shape");
     static_assert((1u << kMaxPassBits) <= (uint32_t)kThreads, "one digit per thread in step B");
     extern __shared__ __align__(16) unsigned char smem[];
     const int relidx = blockIdx.y, g = blockIdx.x;
@@ -188,7 +201,7 @@ partition_pass(PassArgs a) {
     const uint32_t F = df.mask + 1;
     auto dig = [&](uint64_t w) { return df(kHashed ? tkey(w) * kFibMul : tkey(w)); };
     uint64_t *stage = reinterpret_cast<uint64_t *>(smem);
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + kPTile);   // [2][F]
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + kTile);   // [2][F]
     uint32_t *toff = cnt + 2 * F;
     uint32_t *lim = toff + F;
     uint32_t *b1 = lim + F;
@@ -225,11 +238,11 @@ partition_pass(PassArgs a) {
         }
     __syncthreads();
 
-    // ---- tiles: kPTile flat tuples, or kPTile / 64 input pages.  Whole flat
+    // ---- tiles: kTile flat tuples, or kTile / 64 input pages.  Whole flat
     // tiles take loads, ranks and staging without bounds checks (pass 1 at 2^27:
     // 1.033 -> 0.988 ms; the same for paged tiles, by whole pages of a warp, made
     // pass 2 2 % slower).
-    constexpr uint64_t kStep = kPaged ? (uint64_t)(kPTile / kPageTuples) : (uint64_t)kPTile;
+    constexpr uint64_t kStep = kPaged ? (uint64_t)(kTile / kPageTuples) : (uint64_t)kTile;
     const bool vec = !kPaged && ((reinterpret_cast<uintptr_t>(in.in + b) & 15) == 0);
     uint64_t w[kPer];
     uint32_t valid = 0;   // bit k: w[k] holds a tuple
@@ -265,12 +278,14 @@ partition_pass(PassArgs a) {
                 w[2 * k + 1] = v.y;
             }
         } else {
+            const uint64_t *src = in.in + t0 + tid;
+            const int left = (int)min(kStep, e - t0) - tid;
             valid = 0;
 #pragma unroll
             for (int k = 0; k < kPer; k++) {
-                const uint64_t i = t0 + (uint64_t)k * kThreads + tid;
-                w[k] = i < e ? ld_stream(in.in + i) : 0;
-                valid |= (i < e ? 1u : 0u) << k;
+                const bool ok = k * kThreads < left;
+                w[k] = ok ? ld_stream(src + k * kThreads) : 0;
+                valid |= (ok ? 1u : 0u) << k;
             }
         }
     };
@@ -390,7 +405,7 @@ partition_pass(PassArgs a) {
                         sumN += pages_for(Ls[j], Ps[j]);
                     }
                 }
-                const uint32_t v = sumL | (sumN << 16);   // L <= kPTile, pages < 2^16
+                const uint32_t v = sumL | (sumN << 16);   // L <= kTile, pages < 2^16
                 const uint32_t inc = warp_incl_scan(v, lane);
                 const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
                 const uint32_t pool0 = misc[0];
@@ -424,7 +439,7 @@ partition_pass(PassArgs a) {
                     p = npos[d];
                     need = pages_for(L, p);
                 }
-                inc = warp_incl_scan(L | (need << 16), lane);   // L <= kPTile, pages of 32 digits < 2^16
+                inc = warp_incl_scan(L | (need << 16), lane);   // L <= kTile, pages of 32 digits < 2^16
                 mx = __reduce_max_sync(0xffffffffu, (L << 16) | d);   // this warp's largest run, its digit
                 pool0 = misc[0];
                 if (lane == 31) misc[8 + bw] = inc;

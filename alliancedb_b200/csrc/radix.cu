@@ -18,31 +18,45 @@ namespace adb {
 
 // CTAs of a flat pass, split over the relations by size, at most one per tile.
 // Every (CTA, digit) stream ends in a partial page, which the join reads and
-// copies like a full one, so smaller inputs get one wave of resident CTAs
-// (2^22 x 2^22, 512 digits: pass 87 -> 79 us, join kernel 122 -> 60 us against two
-// waves, whose pages are half empty and overfill the join's R chunks).  From
-// 2^27 tuples on the partial pages no longer count and a second wave evens out
-// skewed digits (2^27 x 2^27, pass 1: theta 0 1.057 -> 1.046 ms, theta 1.5 1.154 ->
-// 1.088 ms).
-static void flat_ctas(uint64_t nR, uint64_t nS, int num_sms, int G[2]) {
-    const uint64_t all = (uint64_t)num_sms * kPassMinBlocks * (nR + nS >= (1ull << 27) ? 2 : 1);
-    const uint64_t n[2] = {nR, nS};
+// copies like a full one, so the fewer streams the better where they are short:
+//   * inputs below 2^27 tuples get one wave of CTAs (2^22 x 2^22, two waves of
+//     1024-thread CTAs: 138 us instead of 118).  From 2^27 on the partial pages
+//     no longer count and a second wave evens out skewed digits (2^27 x 2^27,
+//     pass 1: theta 0 1.057 -> 1.046 ms, theta 1.5 1.154 -> 1.088 ms);
+//   * wide: a single pass, whose pages go to the join, runs as one 1024-thread
+//     CTA per SM, so half as many streams as two of 512 threads.  PRO, us, two
+//     CTAs / one: 2^20 x 2^20 68 / 59, 2^22 x 2^22 134 / 117, the same with four of
+//     each key 101 / 80 and 223 / 193, 2^22 x 2^26 (512 digits) 1669 / 1570; 2^20 x
+//     2^25 854 / 867 (0.99, the one size where it was slower).  A first pass with
+//     a second to follow keeps two CTAs, one of which loads and stores while
+//     the other waits at a barrier (2^27 x 2^27: 0.953 ms, one CTA 1.033).
+static void flat_ctas(uint64_t nR, uint64_t nS, int num_sms, bool wide, int G[2]) {
+    const uint64_t all = (uint64_t)num_sms * (wide ? 1 : kPassMinBlocks) * (nR + nS >= (1ull << 27) ? 2 : 1);
+    const uint64_t n[2] = {nR, nS}, tile = wide ? kWideTile : kFlatTile;
+    uint64_t left = all;   // not more than all together: one CTA over would be a wave of its own
     for (int r = 0; r < 2; r++) {
-        uint64_t g = nR + nS ? (all * n[r] + (nR + nS) / 2) / (nR + nS) : 1;
-        const uint64_t tiles = (n[r] + kPTile - 1) / kPTile;
+        uint64_t g = r ? left : nR + nS ? (all * nR + (nR + nS) / 2) / (nR + nS) : 1;
+        if (!r && g >= all) g = all - 1;
+        const uint64_t tiles = (n[r] + tile - 1) / tile;
         if (g > tiles) g = tiles;
         G[r] = (int)(g < 1 ? 1 : g);
+        left -= G[r];
     }
 }
 
 // Launches one partition pass (both relations: grid.y = relation).
-static void launch_pass(const PassArgs &a, uint32_t F, int G, bool paged, cudaStream_t st) {
+static void launch_pass(const PassArgs &a, uint32_t F, int G, bool wide, cudaStream_t st) {
     const dim3 grid(G, 2);
-    const size_t smem = pass_smem(F, paged);
-    if (paged && a.df.hashed) partition_pass<1, kPassThreads, true><<<grid, kPassThreads, smem, st>>>(a);
-    else if (paged) partition_pass<1, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
-    else if (a.df.hashed) partition_pass<0, kPassThreads, true><<<grid, kPassThreads, smem, st>>>(a);
-    else partition_pass<0, kPassThreads><<<grid, kPassThreads, smem, st>>>(a);
+    const bool h = a.df.hashed;
+    auto go = [&](auto kernel, int threads, int tile) {
+        kernel<<<grid, threads, pass_smem(tile, F, a.paged == 1), st>>>(a);
+    };
+    if (a.paged) go(h ? partition_pass<1, kPassThreads, kPagedTile, true> : partition_pass<1, kPassThreads, kPagedTile>,
+                    kPassThreads, kPagedTile);
+    else if (wide) go(h ? partition_pass<0, kWideThreads, kWideTile, true> : partition_pass<0, kWideThreads, kWideTile>,
+                      kWideThreads, kWideTile);
+    else go(h ? partition_pass<0, kPassThreads, kFlatTile, true> : partition_pass<0, kPassThreads, kFlatTile>,
+            kPassThreads, kFlatTile);
 }
 
 // Fan-out bits: partitions of at most 2^13 tuples (one R chunk), and below that
@@ -72,6 +86,7 @@ int sort_bits_for(uint64_t nR, int part_fanout) {
 // ---------------------------------------------------------------------------
 struct PartPlan {
     int passes;
+    bool wide;                 // pass 1 in 1024-thread CTAs
     uint32_t F1, F2, Fout;
     int g1[2];                 // pass 1: CTAs of R, S
     int G1, G2;                // CTAs per relation (pass 1: the larger of g1)
@@ -86,7 +101,8 @@ static PartPlan plan_partition(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b
     p.F1 = 1u << b1;
     p.F2 = b2 ? 1u << b2 : 1u;
     p.Fout = p.F1 * p.F2;
-    flat_ctas(nR, nS, num_sms, p.g1);
+    p.wide = !b2;
+    flat_ctas(nR, nS, num_sms, p.wide, p.g1);
     p.G1 = p.g1[0] > p.g1[1] ? p.g1[0] : p.g1[1];
     const uint32_t a = flat_pool_cap(nR, p.g1[0], p.F1), b = flat_pool_cap(nS, p.g1[1], p.F1);
     p.pool1 = a > b ? a : b;
@@ -168,7 +184,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     a1.out[0].pstart = pstart1;
     a1.out[1].pstart = pstart1 + (p.F1 + 1);
 
-    launch_pass(a1, p.F1, p.G1, false, st);
+    launch_pass(a1, p.F1, p.G1, p.wide, st);
     uint32_t *uoff0 = nullptr, *uoff1 = nullptr;
     if (p.passes == 2) {
         uoff0 = ctx->ws.take<uint32_t>(p.F1 + 1);
@@ -211,7 +227,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     a2.out[0].pstart = pstart2;
     a2.out[1].pstart = pstart2 + (p.Fout + 1);
 
-    launch_pass(a2, p.F2, p.G2, true, st);
+    launch_pass(a2, p.F2, p.G2, false, st);
     list_starts<<<dim3((p.Fout + kScanThreads - 1) / kScanThreads, 2), kScanThreads, 0, st>>>(a2);
     page_place<<<dim3(p.G2, 2), kPlaceThreads, 0, st>>>(a2, 0u, nullptr, nullptr);
     ADB_CK(cudaGetLastError());
@@ -293,12 +309,16 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
 }
 
 int radix_set_attrs() {
-    const int flat = (int)pass_smem(1u << kMaxPassBits, false), paged = (int)pass_smem(1u << kMaxPassBits, true);
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads>, attr, flat));
-    ADB_CK(cudaFuncSetAttribute(partition_pass<0, kPassThreads, true>, attr, flat));
-    ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads>, attr, paged));
-    ADB_CK(cudaFuncSetAttribute(partition_pass<1, kPassThreads, true>, attr, paged));
+    auto pass_attr = [&](auto kernel, int tile, bool paged) {
+        return cudaFuncSetAttribute(kernel, attr, (int)pass_smem(tile, 1u << kMaxPassBits, paged));
+    };
+    ADB_CK(pass_attr(partition_pass<0, kPassThreads, kFlatTile>, kFlatTile, false));
+    ADB_CK(pass_attr(partition_pass<0, kPassThreads, kFlatTile, true>, kFlatTile, false));
+    ADB_CK(pass_attr(partition_pass<0, kWideThreads, kWideTile>, kWideTile, false));
+    ADB_CK(pass_attr(partition_pass<0, kWideThreads, kWideTile, true>, kWideTile, false));
+    ADB_CK(pass_attr(partition_pass<1, kPassThreads, kPagedTile>, kPagedTile, true));
+    ADB_CK(pass_attr(partition_pass<1, kPassThreads, kPagedTile, true>, kPagedTile, true));
     ADB_CK(cudaFuncSetAttribute(radix_join_items<false>, attr, (int)kJoinSmem));
     ADB_CK(cudaFuncSetAttribute(radix_join_items<true>, attr, (int)kJoinSmem));
     ADB_CK(cudaFuncSetAttribute(radix_join_items<false, true>, attr, (int)kJoinSmem));
