@@ -25,6 +25,8 @@
 // bytes of page-list and count metadata per 64 tuples.
 #pragma once
 
+#include <type_traits>
+
 #include "adb_common.cuh"
 #include "partition.cuh"
 
@@ -116,10 +118,10 @@ __host__ __device__ __forceinline__ uint32_t unit_pages_for(uint64_t pages1_both
 
 // Shared memory of one pass:
 //   stage[tile] u64 | cnt[2][F] | toff[F] | lim[F] | b1[F] | b2[F] | npos[F] | npages[F] u32 | misc[48] u32
-//   | paged input only: upage[kMaxUnitPages] u32 | ucnt[kMaxUnitPages] u8
+//   | paged input only: upage[kMaxUnitPages] u32
 __host__ __device__ __forceinline__ size_t pass_smem(int tile, uint32_t F, bool paged) {
     return (size_t)tile * 8 + (size_t)F * 4 * 8 + 48 * 4 +
-           (paged ? (size_t)kMaxUnitPages * 5 : 0);
+           (paged ? (size_t)kMaxUnitPages * 4 : 0);
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
@@ -211,8 +213,7 @@ partition_pass(PassArgs a) {
     uint32_t *misc = npages + F;        // [0] pool pages taken, [1] tuples in the tile,
                                         // [8..24) per-warp totals of the digit scan,
                                         // [kHotWord] hot digit
-    uint32_t *upage = misc + 48;        // paged input: this unit's pages
-    uint8_t *ucnt = reinterpret_cast<uint8_t *>(upage + kMaxUnitPages);
+    uint32_t *upage = misc + 48;        // paged input: this unit's pages, id << 6 | tuples - 1
 
     const PageSet &o = relidx ? a.out[1] : a.out[0];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -233,15 +234,13 @@ partition_pass(PassArgs a) {
     if (kPaged)
         for (uint64_t i = b + tid; i < e; i += kThreads) {
             const uint32_t pg = in.plist[i];
-            upage[i - b] = pg;
-            ucnt[i - b] = in.pcount[pg];
+            upage[i - b] = pg << 6 | (in.pcount[pg] - 1u);
         }
     __syncthreads();
 
     // ---- tiles: kTile flat tuples, or kTile / 64 input pages.  Whole flat
     // tiles take loads, ranks and staging without bounds checks (pass 1 at 2^27:
-    // 1.033 -> 0.988 ms; the same for paged tiles, by whole pages of a warp, made
-    // pass 2 2 % slower).
+    // 1.033 -> 0.988 ms; the same for paged tiles made pass 2 slower, 1.059 -> 1.124).
     constexpr uint64_t kStep = kPaged ? (uint64_t)(kTile / kPageTuples) : (uint64_t)kTile;
     const bool vec = !kPaged && ((reinterpret_cast<uintptr_t>(in.in + b) & 15) == 0);
     uint64_t w[kPer];
@@ -254,16 +253,17 @@ partition_pass(PassArgs a) {
 #pragma unroll
             for (int k = 0; k < kPer / 2; k++) {
                 const uint64_t li = t0 + (uint64_t)k * (kThreads / 32) + tid / 32;
-                const uint32_t c = li < e ? ucnt[li - b] : 0u;
+                const uint32_t v = li < e ? upage[li - b] : 0u;
+                const uint32_t c = li < e ? (v & 63u) + 1u : 0u;
+                const uint64_t *src = in.pages + (uint64_t)(v >> 6) * kPageTuples + slot;
                 if (slot + 1 < c) {
-                    const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(
-                        in.pages + (uint64_t)upage[li - b] * kPageTuples + slot));
-                    w[2 * k] = v.x;
-                    w[2 * k + 1] = v.y;
+                    const ulonglong2 x = __ldcs(reinterpret_cast<const ulonglong2 *>(src));
+                    w[2 * k] = x.x;
+                    w[2 * k + 1] = x.y;
                     valid |= 3u << (2 * k);
                 } else {
                     const bool ok = slot < c;
-                    w[2 * k] = ok ? ld_stream(in.pages + (uint64_t)upage[li - b] * kPageTuples + slot) : 0;
+                    w[2 * k] = ok ? ld_stream(src) : 0;
                     w[2 * k + 1] = 0;
                     valid |= (ok ? 1u : 0u) << (2 * k);
                 }
@@ -303,7 +303,7 @@ partition_pass(PassArgs a) {
         if (kPaged && tid < (int)(kStep * 4)) {
             const uint64_t li = t0 + (uint64_t)(tid >> 2);
             if (li < e) {
-                const uint64_t *line = in.pages + (uint64_t)upage[li - b] * kPageTuples + (tid & 3) * 16;
+                const uint64_t *line = in.pages + (uint64_t)(upage[li - b] >> 6) * kPageTuples + (tid & 3) * 16;
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
             }
         }
@@ -484,16 +484,33 @@ partition_pass(PassArgs a) {
         }
         __syncthreads();
         // D. stage slots to their pages
-        for (uint32_t i = tid; i < tile_n; i += kThreads) {
-            const uint64_t v = stage[i];
-            const uint32_t d = dig(v);
-            const uint32_t dst = i + (i < lim[d] ? b1[d] : b2[d]);
-            o.pages[dst] = v;
-            if ((dst & (kPageTuples - 1)) == 0) {   // first slot of a page taken in B
-                o.log[dst / kPageTuples] = dbase + d;
-                o.pcount[dst / kPageTuples] = kPageTuples;
+        auto copy = [&](uint32_t i0, auto n) {   // slots i0, i0 + kThreads, ..: n of them
+            constexpr int U = decltype(n)::value;
+            uint64_t v[U];
+            uint32_t d[U], dst[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = stage[i0 + u * kThreads];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t i = i0 + u * kThreads;
+                d[u] = dig(v[u]);
+                dst[u] = i + (i < lim[d[u]] ? b1 : b2)[d[u]];
             }
-        }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                o.pages[dst[u]] = v[u];
+                if ((dst[u] & (kPageTuples - 1)) == 0) {   // first slot of a page taken in B
+                    o.log[dst[u] / kPageTuples] = dbase + d[u];
+                    o.pcount[dst[u] / kPageTuples] = kPageTuples;
+                }
+            }
+        };
+        // two at a time, so that one's look-ups overlap the other's (2^27 x 2^27,
+        // ms, one / two / four / eight: pass 1 0.954 / 0.948 / 0.946 / 1.085, pass 2
+        // 1.068 / 1.065 / 1.073 / 1.514)
+        uint32_t i = tid;
+        for (; i + kThreads < tile_n; i += 2 * kThreads) copy(i, std::integral_constant<int, 2>());
+        if (i < tile_n) copy(i, std::integral_constant<int, 1>());
         // the next tile's A uses the other counter array and registers only;
         // its B / C run after the next barrier, when every thread is past D
     }
