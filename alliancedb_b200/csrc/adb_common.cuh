@@ -78,6 +78,21 @@ __device__ __forceinline__ void block_flush(Acc a, unsigned long long *out, uint
     __syncthreads();
 }
 
+// One thread per CTA of a call's last kernel, after the CTA's sums are in acc:
+// the last of them hands acc[0 .. 3] to the host (out: pinned memory) and
+// leaves the accumulators at 0 for the next call, so that neither a clear nor a
+// copy back is launched.  acc[5] counts the CTAs.
+__device__ __forceinline__ void finish_call(unsigned long long *acc, unsigned long long *out) {
+    __threadfence();
+    if (atomicAdd(acc + 5, 1ull) != (unsigned long long)gridDim.x * gridDim.y - 1) return;
+    __threadfence();
+    ulonglong2 *a2 = reinterpret_cast<ulonglong2 *>(acc), *o2 = reinterpret_cast<ulonglong2 *>(out);
+    const ulonglong2 lo = __ldcg(a2), hi = __ldcg(a2 + 1);
+    o2[0] = lo;
+    o2[1] = hi;
+    for (int k = 0; k < 3; k++) a2[k] = make_ulonglong2(0, 0);
+}
+
 // Exclusive scan of one value per thread across the block; returns the prefix
 // and writes the block total to *total.  `tmp` needs 32 u32 of shared memory.
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *tmp, uint32_t *total) {

@@ -256,7 +256,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     dscan<uint64_t>(st, tot, Dt, pstart, bsum64);
     dscan<uint64_t>(st, tot + Dt, Dt, pstart + (Dt + 1), bsum64);
     page_place<<<dim3(G, 2), kPlaceThreads, 0, st>>>(a, 0u, nullptr, nullptr);
-    part_chunks<<<(Dt + 31) / 32, 1024, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, kChunkW, kSPages, wl,
+    part_chunks<<<(Dt + 31) / 32, 1024, 0, st>>>(pstart, a.out[0].plist, a.out[0].pcount, Dt, wl,
                                                  false);
     dscan<uint32_t>(st, wl.items, Dt, wl.items_off, bsum32);
     copy_last_u32<<<1, 1, 0, st>>>(wl.items_off + Dt, wl.ctr);
@@ -266,7 +266,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ja.Rcount = a.out[0].pcount; ja.Scount = a.out[1].pcount;
     ja.Rlist = a.out[0].plist; ja.Slist = a.out[1].plist;
     ja.pstart = pstart; ja.wl = wl;
-    ja.acc = acc; ja.err = reinterpret_cast<int *>(acc + 2);
+    ja.acc = acc; ja.out = nullptr; ja.err = reinterpret_cast<int *>(acc + 2);
     ja.waits_run_out = 0;
     ja.F = Dt;
     ja.bits = 0;   // per-window fan-out: the kernel reads each window's bits

@@ -173,7 +173,7 @@ Context *ctx_create(int dev, int *status) {
     for (auto &e : c->ev)
         if (cudaEventCreate(&e) != cudaSuccess) goto fail;
     if (cudaMallocHost(&c->h_res, 64 * sizeof(unsigned long long)) != cudaSuccess) goto fail;
-    if (cudaMalloc(&c->d_small, 64) != cudaSuccess || cudaMemset(c->d_small, 0, 64) != cudaSuccess) goto fail;
+    if (cudaMalloc(&c->d_acc, 64) != cudaSuccess || cudaMemset(c->d_acc, 0, 64) != cudaSuccess) goto fail;
     if (cudaDeviceSynchronize() != cudaSuccess) goto fail;   // the library's stream does not wait for the clear
     {
         int s = radix_set_attrs();
@@ -202,7 +202,7 @@ void ctx_destroy(Context *c) {
     for (auto &e : c->ev)
         if (e) cudaEventDestroy(e);
     if (c->h_res) cudaFreeHost(c->h_res);
-    if (c->d_small) cudaFree(c->d_small);
+    if (c->d_acc) cudaFree(c->d_acc);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_out) cudaFreeHost(c->h_out);
     for (int t = 0; t < Context::kCopyWorkers; t++) {
@@ -375,16 +375,26 @@ static int join_device_core(Context *ctx, const AlgoEntry *a, DevJoin j, const a
     // events: ev[0] start, ev[6] end, and the phase boundaries ev[1..3] that the
     // driver marks; a boundary it does not mark falls onto the one before it
     ADB_CK(cudaEventRecord(ctx->ev[0], st));
-    if (use_small(a, j.nR, j.nS, p)) {
+    const bool eager = a->fam == Family::Shj || a->fam == Family::Pmj;
+    unsigned long long *acc = ctx->d_acc;
+    if (!j.nR || !j.nS) {
+        for (int k = 0; k < 4; k++) ctx->h_res[k] = 0;
+    } else if (use_small(a, j.nR, j.nS, p)) {
         ADB_TRY(run_small(ctx, j));
-        ADB_CK(cudaEventRecord(ctx->ev[6], st));
     } else {
-        unsigned long long *acc = ctx->ws.take<unsigned long long>(8);
-        ADB_CK(cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st));
-        if (j.nR && j.nS) ADB_TRY(dispatch(ctx, a, j, p, acc));
-        ADB_CK(cudaEventRecord(ctx->ev[6], st));
-        ADB_CK(cudaMemcpyAsync(ctx->h_res, acc, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        if (eager) {
+            acc = ctx->ws.take<unsigned long long>(8);
+            ADB_CK(cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st));
+        }
+        const int rc = dispatch(ctx, a, j, p, acc);
+        if (rc != ADB_OK) {
+            if (!eager) cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st);   // 0 between calls
+            return rc;
+        }
     }
+    ADB_CK(cudaEventRecord(ctx->ev[6], st));
+    if (j.nR && j.nS && eager)
+        ADB_CK(cudaMemcpyAsync(ctx->h_res, acc, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     ADB_CK(cudaStreamSynchronize(st));
     float at[5] = {0, 0, 0, 0, 0}, t[4];   // boundaries, ms after the start
     ADB_CK(cudaEventElapsedTime(&at[4], ctx->ev[0], ctx->ev[6]));

@@ -73,7 +73,7 @@ struct Context {
     cudaEvent_t ev[12] = {};
     Workspace ws;
     unsigned long long *h_res = nullptr;   // pinned: [0] count [1] checksum [2] err [3] mat_n ...
-    unsigned long long *d_small = nullptr; // device accumulators of the single-launch joins, 0 between calls
+    unsigned long long *d_acc = nullptr;   // device accumulators (8 words), 0 between calls
     unsigned marks = 0;                    // phase events recorded by the current call (bit k: ev[k])
     // pinned, grow-only host buffers of the batched path: the per-call plan (one
     // host -> device copy) and the per-window results (one copy back); growing

@@ -1,9 +1,11 @@
 // joins.cuh -- device-resident join drivers shared by the C ABI and the
 // batched/served paths.  Each driver: scratch size for a call, then the
 // launch sequence on ctx->stream.  Results land in acc[0] (count) and acc[1]
-// (checksum) of a device accumulator the caller zeroed; acc[2] is the error
+// (checksum) of a device accumulator that is 0 at the start; acc[2] is the error
 // word (a timed-out device wait sets it), acc[3] the materialised count, acc[4]
-// NPO's build tuples equal to its empty marker.
+// NPO's build tuples equal to its empty marker, acc[5] the CTAs done.  All but
+// the eager drivers end with a kernel that moves acc[0 .. 3] to ctx->h_res and
+// clears acc (finish_call); run_eager leaves that to its caller.
 #pragma once
 
 #include "engine.cuh"
@@ -32,7 +34,7 @@ struct DigitFn;
 size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms);
 uint64_t paged_final_pool_pages(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms);
 int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitFn *d2, PartOut *out,
-                        unsigned long long *acc);
+                        unsigned long long *acc, uint32_t **ctr = nullptr);
 
 // ---- hash joins of a small build side, small.cu ----
 bool small_fits(uint64_t nR, uint64_t nS);

@@ -171,7 +171,7 @@ template <bool kMaterialize>
 __global__ void __launch_bounds__(kNpoThreads, 4)
 npo_probe_pages(NpoPages P, const uint64_t *__restrict__ table, uint32_t log2n,
                 const unsigned long long *sentinel_cnt, unsigned long long *acc, uint64_t *mat,
-                unsigned long long *mat_n, uint64_t mat_cap) {
+                unsigned long long *mat_n, uint64_t mat_cap, unsigned long long *out) {
     __shared__ uint64_t red[64];
     const uint64_t mask = (1ULL << log2n) - 1;
     const int lane = threadIdx.x & 31;
@@ -209,6 +209,7 @@ npo_probe_pages(NpoPages P, const uint64_t *__restrict__ table, uint32_t log2n,
             if (ok[u]) npo_probe_one(sink, table, mask, s[u], slot[u], lo[u], hi[u], nsent);
     }
     block_flush(sink.a, acc, red);
+    if (threadIdx.x == 0) finish_call(acc, out);
 }
 
 // Phases (ms_phase): 0 grouping by region (0 without), 1 build (with the
@@ -241,10 +242,10 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
         ADB_CK(mark(ctx, 2));
         if (j.mat)
             npo_probe_pages<true><<<ctx->num_sms * np, kNpoThreads, 0, st>>>(PS, table, l2, sent, acc, j.mat,
-                                                                              acc + 3, j.mat_cap);
+                                                                              acc + 3, j.mat_cap, ctx->h_res);
         else
             npo_probe_pages<false><<<ctx->num_sms * np, kNpoThreads, 0, st>>>(PS, table, l2, sent, acc, nullptr,
-                                                                               nullptr, 0);
+                                                                               nullptr, 0, ctx->h_res);
     } else {
         const int threads = 256;
         // every CTA resident at once: one grid-stride sweep without a second wave
@@ -260,10 +261,10 @@ int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long 
         ADB_CK(mark(ctx, 2));
         if (j.mat)
             npo_probe<true><<<blocks(j.nS, rp_sm), threads, 0, st>>>(j.S, j.nS, table, (uint32_t)nb, sent, acc, j.mat,
-                                                                     acc + 3, j.mat_cap);
+                                                                     acc + 3, j.mat_cap, ctx->h_res);
         else
             npo_probe<false><<<blocks(j.nS, rp_sm), threads, 0, st>>>(j.S, j.nS, table, (uint32_t)nb, sent, acc,
-                                                                      nullptr, nullptr, 0);
+                                                                      nullptr, nullptr, 0, ctx->h_res);
     }
     ADB_CK(cudaGetLastError());
     ctx->kernels += 2;

@@ -228,7 +228,7 @@ template <bool kMaterialize>
 __global__ void __launch_bounds__(256)
 npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restrict__ table, uint32_t nb,
           const unsigned long long *sentinel_cnt, unsigned long long *acc, uint64_t *mat, unsigned long long *mat_n,
-          uint64_t mat_cap) {
+          uint64_t mat_cap, unsigned long long *out) {
     __shared__ uint64_t red[64];
     const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t nsent = *sentinel_cnt;
@@ -278,6 +278,7 @@ npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restric
             if (found[u]) sink.match(s[u], tkey(s[u]), pay[u], sh[u]);
     }
     block_flush(sink.a, acc, red);
+    if (out && threadIdx.x == 0) finish_call(acc, out);
 }
 
 }  // namespace adb

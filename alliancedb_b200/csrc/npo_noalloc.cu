@@ -118,7 +118,7 @@ extern "C" int adb_npo_join_noalloc(const adb_tuple *dR, uint64_t nR, const adb_
         npo_build<<<blocks(nR), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dR), nR, table, (uint32_t)nb, acc + 3,
                                                   reinterpret_cast<int *>(acc + 2));
         npo_probe<false><<<blocks(nS), threads, 0, st>>>(reinterpret_cast<const uint64_t *>(dS), nS, table, (uint32_t)nb,
-                                                         acc + 3, acc, nullptr, nullptr, 0);
+                                                         acc + 3, acc, nullptr, nullptr, 0, nullptr);
     }
     noalloc_emit<<<1, 32, 0, st>>>(acc, d_out);
     ADB_CK(cudaGetLastError());

@@ -130,7 +130,7 @@ static size_t pageset_bytes(uint64_t pages, uint32_t G) {
 
 size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
     const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
-    size_t s = 2 * pageset_bytes(p.pages1, p.G1) + Workspace::need(2ull * (p.F1 + p.Fout), 4) +
+    size_t s = 2 * pageset_bytes(p.pages1, p.G1) + Workspace::need(2ull * (p.F1 + p.Fout) + 4, 4) +
                Workspace::need(2ull * (p.F1 + 1), 8);
     if (p.passes == 2)
         s += 2 * pageset_bytes(p.pages2, p.G2) + Workspace::need(2ull * (p.Fout + 1), 8) +
@@ -151,7 +151,7 @@ static void take_pageset(Context *ctx, PageSet &ps, uint64_t pages, int G) {
 // Partitions R and S by d1 (and then d2) into page lists per output partition
 // D = p1 * F2 + p2.  out->pstart = [2][Fout + 1] page-list starts.
 int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitFn *d2, PartOut *out,
-                        unsigned long long *acc) {
+                        unsigned long long *acc, uint32_t **ctr) {
     cudaStream_t st = ctx->stream;
     const uint32_t b1 = ceil_log2_u64((uint64_t)d1.mask + 1), b2 = d2 ? ceil_log2_u64((uint64_t)d2->mask + 1) : 0;
     const PartPlan p = plan_partition(j.nR, j.nS, b1, b2, ctx->num_sms);
@@ -176,8 +176,11 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     a1.pool_cap = p.pool1;
     a1.paged = 0;
     a1.err = err;
-    uint32_t *totals1 = ctx->ws.take<uint32_t>(2ull * (p.F1 + p.Fout)), *totals2 = totals1 + 2ull * p.F1;
-    ADB_CK(cudaMemsetAsync(totals1, 0, 8ull * (p.F1 + (p.passes == 2 ? p.Fout : 0)), st));
+    // the work counters and both passes' totals, cleared by one launch
+    uint32_t *zeros = ctx->ws.take<uint32_t>(2ull * (p.F1 + p.Fout) + 4);
+    uint32_t *totals1 = zeros + 4, *totals2 = totals1 + 2ull * p.F1;
+    ADB_CK(cudaMemsetAsync(zeros, 0, 16 + 8ull * (p.F1 + (p.passes == 2 ? p.Fout : 0)), st));
+    if (ctr) *ctr = zeros;
     a1.totals = totals1;
     a1.Dtot = p.F1;
     uint64_t *pstart1 = ctx->ws.take<uint64_t>(2ull * (p.F1 + 1));
@@ -272,13 +275,14 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
     const DigitFn d1{hashed ? 32u - b1 : 0u, (1u << b1) - 1, hashed};
     const DigitFn d2{hashed ? 32u - b1 - b2 : b1, (1u << b2) - 1, hashed};
     PartOut po;
-    ADB_TRY(run_paged_partition(ctx, j, d1, b2 ? &d2 : nullptr, &po, acc));
+    uint32_t *ctr;
+    ADB_TRY(run_paged_partition(ctx, j, d1, b2 ? &d2 : nullptr, &po, acc, &ctr));
     if (b2) ADB_CK(mark(ctx, 2));   // phases: pass 1 | pass 2 | work list | join
 
     const uint32_t F = po.Fout;
     WorkList wl;
-    wl.take(ctx->ws, F, po.pool_pages, kChunkW);
-    ctx->kernels += make_work_list(st, po.pstart, po.R.plist, po.R.pcount, F, kChunkW, kSPages, wl);
+    wl.take(ctx->ws, F, po.pool_pages, kChunkW, ctr);
+    ctx->kernels += make_work_list(st, po.pstart, po.R.plist, po.R.pcount, F, wl);
     ADB_CK(cudaGetLastError());
     ADB_CK(mark(ctx, 3));
 
@@ -287,7 +291,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
     a.Rcount = po.R.pcount; a.Scount = po.S.pcount;
     a.Rlist = po.R.plist; a.Slist = po.S.plist;
     a.pstart = po.pstart; a.wl = wl;
-    a.acc = acc; a.err = reinterpret_cast<int *>(acc + 2);
+    a.acc = acc; a.out = ctx->h_res; a.err = reinterpret_cast<int *>(acc + 2);
     a.waits_run_out = j.test_flags & ADB_TEST_WAITS_RUN_OUT;
     a.F = F; a.bits = (uint32_t)bits;
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;

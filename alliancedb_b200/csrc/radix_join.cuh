@@ -52,30 +52,30 @@ struct WorkList {
         return 3 * Workspace::need(F, 4) + Workspace::need(F + 1, 4) + Workspace::need(chunks(F, pages, chunk_w), 8) +
                Workspace::need(3, 4);
     }
-    void take(Workspace &ws, uint64_t F, uint64_t pages, uint32_t chunk_w) {
+    void take(Workspace &ws, uint64_t F, uint64_t pages, uint32_t chunk_w, uint32_t *counters = nullptr) {
         rch = ws.take<uint32_t>(F);
         chunk_off = ws.take<uint32_t>(F);
         items = ws.take<uint32_t>(F);
         items_off = ws.take<uint32_t>(F + 1);
         cstart = ws.take<uint64_t>(chunks(F, pages, chunk_w));
-        ctr = ws.take<uint32_t>(3);
+        ctr = counters ? counters : ws.take<uint32_t>(3);
     }
 };
 
 // R chunks and item counts, one warp per partition: chunk c of a partition
-// starts at the first page whose preceding weight reaches c * chunk_w (greedy
-// by page weight); S chunks are s_pages pages each.  With `scan` (F <= 1024) the
+// starts at the first page whose preceding weight reaches c * kChunkW (greedy
+// by page weight); S chunks are kSPages pages each.  With `scan` (F <= 1024) the
 // last block to finish also makes items_off and the item count, so that one
 // launch stands between the passes and the join.
 static __global__ void __launch_bounds__(1024)
-part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount, uint32_t F, uint32_t chunk_w,
-            uint32_t s_pages, WorkList wl, bool scan) {
+part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount, uint32_t F, WorkList wl,
+            bool scan) {
     const int lane = threadIdx.x & 31;
     const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (p < F) {
         const uint64_t *pS = pstart + (F + 1);
         const uint64_t r0 = pstart[p], r1 = pstart[p + 1];
-        const uint64_t cid = r0 * kPageTuples / chunk_w + p;
+        const uint64_t cid = r0 * kPageTuples / kChunkW + p;
         uint64_t carry = 0;                 // weight before this round
         uint32_t prev_chunk = 0xFFFFFFFFu;  // chunk of the page before this round
         constexpr int U = 4;                // rounds of 32 pages loaded together
@@ -89,7 +89,7 @@ part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount
             for (int u = 0; u < U; u++) {
                 const uint64_t k = base + 32 * u + lane;
                 const uint32_t x = warp_incl_scan(w[u], lane);
-                const uint32_t ch = (uint32_t)((carry + x - w[u]) / chunk_w);
+                const uint32_t ch = (uint32_t)((carry + x - w[u]) / kChunkW);
                 uint32_t before = __shfl_up_sync(0xffffffffu, ch, 1);
                 if (lane == 0) before = prev_chunk;
                 if (k < r1 && ch != before) wl.cstart[cid + ch] = k;
@@ -101,7 +101,7 @@ part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount
         }
         if (lane == 0) {
             const uint32_t rc = r1 > r0 ? prev_chunk + 1 : 0u;
-            const uint32_t sc = (uint32_t)((pS[p + 1] - pS[p] + s_pages - 1) / s_pages);
+            const uint32_t sc = (uint32_t)((pS[p + 1] - pS[p] + kSPages - 1) / kSPages);
             wl.rch[p] = rc;
             wl.chunk_off[p] = (uint32_t)cid;
             wl.items[p] = rc * sc;
@@ -126,9 +126,8 @@ static __global__ void __launch_bounds__(kScanThreads) items_scan(WorkList wl, u
 
 // The work list of F partitions; returns the launches it took.
 static int make_work_list(cudaStream_t st, const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount,
-                          uint32_t F, uint32_t chunk_w, uint32_t s_pages, const WorkList &wl) {
-    cudaMemsetAsync(wl.ctr, 0, 3 * sizeof(uint32_t), st);
-    part_chunks<<<(F + 31) / 32, 1024, 0, st>>>(pstart, Rlist, Rcount, F, chunk_w, s_pages, wl, F <= kScanThreads);
+                          uint32_t F, const WorkList &wl) {
+    part_chunks<<<(F + 31) / 32, 1024, 0, st>>>(pstart, Rlist, Rcount, F, wl, F <= kScanThreads);
     if (F <= kScanThreads) return 1;
     items_scan<<<(F + kScanThreads - 1) / kScanThreads, kScanThreads, 0, st>>>(wl, F);
     return 2;
@@ -192,6 +191,7 @@ struct JoinArgs {
     const uint64_t *pstart;          // [2][F+1] page-list starts
     WorkList wl;
     unsigned long long *acc;         // [0] count, [1] checksum
+    unsigned long long *out;         // pinned host copy of acc[0 .. 3], written by the last CTA (null: none)
     int *err;
     int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report a wait that ran out
     uint32_t F;
@@ -516,6 +516,7 @@ radix_join_items(JoinArgs a) {
         cur ^= 1;
     }
     block_flush(acc, a.acc, red);
+    if (a.out && threadIdx.x == 0) finish_call(a.acc, a.out);
 }
 
 }  // namespace adb

@@ -28,8 +28,7 @@ constexpr uint32_t kSmallNone = 0xFFFFFFFFu;
 constexpr size_t kSmallSmem = ((size_t)12 << kSmallLog2) + 64 * 8;
 static_assert(kSmallBlocks * (kSmallSmem + 1024) <= 233472, "small_join CTAs exceed the SM's shared memory");
 
-// acc: [0] count, [1] checksum, [3] materialised tuples, [4] CTAs done; all 0
-// before and after.  out: the same first four words for the host.
+// acc: [0] count, [1] checksum, [3] materialised tuples; out: the host's copy.
 template <bool kMat>
 __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks)
 small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const uint64_t *__restrict__ S, uint64_t nS,
@@ -106,15 +105,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
         i0 = i1;
     }
     block_flush(a, acc, red);
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(acc + 4, 1ull) == gridDim.x * gridDim.y - 1) {   // every CTA's sums are in
-            __threadfence();
-            for (int k = 0; k < 4; k++) out[k] = atomicExch(acc + k, 0ull);
-            acc[4] = 0;
-            __threadfence_system();
-        }
-    }
+    if (threadIdx.x == 0) finish_call(acc, out);
 }
 
 // One chunk of R at any |S|; several while the probes, one per S tuple and
@@ -140,10 +131,10 @@ int run_small(Context *ctx, const DevJoin &j) {
     const dim3 grid((unsigned)gx, (unsigned)chunks);
     if (j.mat)
         small_join<true><<<grid, kSmallThreads, kSmallSmem, ctx->stream>>>(
-            j.R, j.nR, lnb, j.S, j.nS, per, ctx->d_small, ctx->h_res, j.mat, j.mat_cap);
+            j.R, j.nR, lnb, j.S, j.nS, per, ctx->d_acc, ctx->h_res, j.mat, j.mat_cap);
     else
         small_join<false><<<grid, kSmallThreads, kSmallSmem, ctx->stream>>>(
-            j.R, j.nR, lnb, j.S, j.nS, per, ctx->d_small, ctx->h_res, nullptr, 0);
+            j.R, j.nR, lnb, j.S, j.nS, per, ctx->d_acc, ctx->h_res, nullptr, 0);
     ADB_CK(cudaGetLastError());
     ctx->kernels++;
     return ADB_OK;
