@@ -223,8 +223,8 @@ struct ItemRec {
 //   i + 2 from the work counter and prefetches item i + 1's R pages to L2; the
 //   probing warps load their S page ids of item i + 1.
 // Per item: the table build by all warps (a page per warp, kB pages' loads in
-// flight), then the probe by warps 0 .. kProbeWarps - 1, each holding two S
-// pages in flight ahead of the one it probes.
+// flight), then the probe by warps 0 .. kProbeWarps - 1, each with one S page
+// in flight ahead of the one it probes.
 //
 // The table: bucket heads indexed by the lnb key bits above the b bits the
 // partitioning consumed (kHashed: the lnb bits of key * kFibMul below the b
@@ -235,17 +235,23 @@ struct ItemRec {
 // visited tuple gives payload, comparison bits and link.
 //
 // Bound: instruction issue and the ALU pipe (60 % busy), not DRAM.  |R| = |S| =
-// 2^27, ms: one 1024-thread CTA per SM with two slots per head, separate next
-// array and bulk-copied pages 1.05 dense keys / 1.74 keys spread over 32 bits;
-// this form 0.76 / 1.34 (two CTAs, so that one builds while the other probes:
-// -0.08 / -0.05; one head per slot and links in the tuples: -0.13 / -0.5; pages
-// read straight into the build, without the copy's per-page issue cost of
-// about 58 cycles and its wait: -0.03; the probe's half of the checksum before
-// the walk: -0.05 / -0.07; the next item's R pages in L2 before its build:
-// 0.776 -> 0.740 / 1.350 -> 1.315).  Batched windows (512, 2^10 .. 2^22 tuples): the
-// whole call 7.86 -> 6.01 ms.  Adding a warp's matches together after the walk
-// instead of as they are found: 0.83 / 1.14, and 1.27 instead of 1.23 ms with
-// every key four times in both relations (2^26), so not kept.
+// 2^27, ms, dense keys / keys spread over 32 bits:
+//   one 1024-thread CTA per SM, two slots per head, a
+//   separate next array, bulk-copied pages                  1.05  / 1.74
+//   two CTAs, so that one builds while the other probes    -0.08  / -0.05
+//   one head per slot, links in the tuples                 -0.13  / -0.5
+//   pages read straight into the build, without the copy's
+//   issue cost of about 58 cycles a page and its wait      -0.03
+//   the probe's half of the checksum before the walk       -0.05  / -0.07
+//   the next item's R pages in L2 before its build          0.740 / 1.315
+//   one S page in flight instead of two and three R pages
+//   instead of four: room within 64 registers               0.678 / 1.230
+// The sorted form, with two R pages in flight (four spilled), 1.308 -> 1.168;
+// 512 batched windows (2^10 .. 2^22 tuples), the whole call 5.50 -> 5.29 ms.
+// Not kept: adding a warp's matches together after the walk instead of as they
+// are found, 0.744 / 1.013, and batched windows 3 % slower; choosing between
+// the two by item, by the tuples that share a bucket, 0.694 / 1.025, windows
+// 2 % slower.
 template <bool kMat, bool kHashed = false, bool kSorted = false>
 __global__ void __launch_bounds__(kJoinThreads, kJoinMinBlocks)
 radix_join_items(JoinArgs a) {
@@ -355,7 +361,7 @@ radix_join_items(JoinArgs a) {
         const uint32_t shift = C.shift;
         const uint32_t nrpg = C.nrpg, nspg = C.nspg;
 
-        // --- the probing warp's first two S pages (ids loaded during the
+        // --- the probing warp's first S page (ids loaded during the
         //     previous item): lane l holds tuples 2l, 2l + 1 of a page, cn the
         //     page's count (0: none)
         const uint32_t npw = warp < kProbeWarps && (uint32_t)warp < nspg
@@ -367,11 +373,10 @@ radix_join_items(JoinArgs a) {
             if (2 * lane < (int)cn)
                 x = __ldcs(reinterpret_cast<const ulonglong2 *>(a.Spages + (uint64_t)(v >> 6) * kPageTuples) + lane);
         };
-        ulonglong2 x0 = make_ulonglong2(0, 0), x1 = x0, x2 = x0;
-        uint32_t n0 = 0, n1 = 0, n2 = 0;
+        ulonglong2 x0 = make_ulonglong2(0, 0);
+        uint32_t n0 = 0;
         if (warp < kProbeWarps) {
             load_page(0, x0, n0);
-            load_page(1, x1, n1);
         }
 
         // the bits of x (the key, or its hash) that a bucket shares: the lowest
@@ -396,7 +401,7 @@ radix_join_items(JoinArgs a) {
             const uint32_t x = hash(t), old = atomicExch(&heads[bucket(x)], s);
             return tword(linked(x, old == kNone ? s : old), tpay(t));
         };
-        constexpr int kB = 4;
+        constexpr int kB = kSorted ? 2 : 3;
         // f(slot, the lane's two tuples, whether the second is one) for every page of the chunk
         auto each_page = [&](auto f) {
             for (uint32_t k0 = warp; k0 < nrpg; k0 += kB * kWarps) {
@@ -496,14 +501,14 @@ radix_join_items(JoinArgs a) {
                 }
             };
             for (uint32_t i = 0; i < npw; i++) {
-                n2 = 0;
-                if (i + 2 < npw) load_page(i + 2, x2, n2);
-                if (2 * lane < (int)n0) probe(x0.x);
+                const ulonglong2 c = x0;
+                const uint32_t n = n0;
+                n0 = 0;
+                if (i + 1 < npw) load_page(i + 1, x0, n0);
+                if (2 * lane < (int)n) probe(c.x);
                 __syncwarp();
-                if (2 * lane + 1 < (int)n0) probe(x0.y);
+                if (2 * lane + 1 < (int)n) probe(c.y);
                 __syncwarp();
-                x0 = x1; n0 = n1;
-                x1 = x2; n1 = n2;
             }
             acc.count += matches;
             my_pg = nx_pg;
