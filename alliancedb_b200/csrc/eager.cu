@@ -234,6 +234,8 @@ static uint32_t shj_log2sub(uint64_t n, uint32_t log2parts) {
 // ---------------------------------------------------------------------------
 // PMJ helpers: sort a run, accumulate sorted runs
 // ---------------------------------------------------------------------------
+static unsigned merge_tiles(uint64_t n) { return (unsigned)((n + kMergeTile - 1) / kMergeTile); }
+
 // Sorts n tuples of `in` (stride words per element, tuple last) into out, using
 // tmp (n words) as the ping-pong buffer.  Returns the buffer holding the result.
 __global__ void gather_tuples(const uint64_t *in, uint32_t stride, uint64_t n, uint64_t *out) {
@@ -248,8 +250,7 @@ static uint64_t *device_sort(Context *ctx, uint64_t *a, uint64_t *b, uint64_t n)
     ctx->kernels++;
     uint64_t *src = b, *dst = a;
     for (uint64_t run = kSortBlock; run < n; run *= 2) {
-        const uint64_t threads = (n + kMergeSeg - 1) / kMergeSeg;
-        merge_pass_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(src, n, run, dst);
+        merge_pass_kernel<<<merge_tiles(n), kMergeThreads, 0, st>>>(src, n, run, dst);
         ctx->kernels++;
         std::swap(src, dst);
     }
@@ -259,15 +260,13 @@ static uint64_t *device_sort(Context *ctx, uint64_t *a, uint64_t *b, uint64_t n)
 static void launch_merge_join(Context *ctx, const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb,
                               int a_is_r, unsigned long long *acc) {
     if (!na || !nb) return;
-    const uint64_t threads = (na + nb + kMergeSeg - 1) / kMergeSeg;
-    merge_join_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(A, na, B, nb, a_is_r, acc);
+    merge_join_kernel<<<merge_tiles(na + nb), kMergeThreads, 0, ctx->stream>>>(A, na, B, nb, a_is_r, acc);
     ctx->kernels++;
 }
 
 static void launch_merge(Context *ctx, const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb, uint64_t *out) {
-    const uint64_t threads = (na + nb + kMergeSeg - 1) / kMergeSeg;
-    if (!threads) return;
-    merge_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(A, na, B, nb, out);
+    if (!na && !nb) return;
+    merge_kernel<<<merge_tiles(na + nb), kMergeThreads, 0, ctx->stream>>>(A, na, B, nb, out);
     ctx->kernels++;
 }
 

@@ -147,77 +147,127 @@ static __global__ void __launch_bounds__(1024, 1) block_sort_kernel(const uint64
     for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) out[b + i] = Y[i];
 }
 
+// ---------------------------------------------------------------------------
+// Merges, merge-path tiled: a CTA produces kMergeTile merged elements.  Two warps
+// find where the tile begins and ends in A and in B, the CTA copies both parts to
+// shared memory, and each thread merges kMergePer elements there, from where its
+// own diagonal cuts the tile.  Bound by latency: the searches, the loads and the
+// local merges of one wave of CTAs follow one another.  Runs of 1.6M tuples, us:
+// a merge pass 28 with one thread per 64 elements, which read and wrote global
+// memory element by element, 12 in this form; the join of two runs 82 / 40.  Tiles
+// of 1024 to 2048 tuples by 128 to 512 threads: 12 to 13.6.
+// ---------------------------------------------------------------------------
+constexpr int kMergeThreads = 256;
+constexpr uint32_t kMergePer = 8;
+constexpr uint32_t kMergeTile = kMergeThreads * kMergePer;
+static_assert(2 * kSortBlock % kMergeTile == 0, "a tile lies within one pair of runs");
+
+struct MergeTile {
+    uint64_t v[kMergeTile];                        // A's part, then B's
+    uint64_t cut[2];                               // A elements before the tile, and before its end
+};
+
 // Number of A elements among the first k elements of merge(A, B), A first on
-// equal keys.
-__device__ __forceinline__ uint64_t merge_path(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb,
-                                               uint64_t k) {
+// equal keys; by one warp, 32 probes a round.
+__device__ __forceinline__ uint64_t warp_merge_path(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb,
+                                                    uint64_t k, int lane) {
     uint64_t lo = k > nb ? k - nb : 0, hi = k < na ? k : na;
     while (lo < hi) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (tkey(A[mid]) <= tkey(B[k - mid - 1])) lo = mid + 1; else hi = mid;
+        const uint64_t step = (hi - lo + 31) / 32, mid = lo + lane * step;
+        const bool before = mid < hi && tkey(A[mid]) <= tkey(B[k - mid - 1]);   // true up to the answer
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, before));
+        if (c == 0) break;
+        hi = min(hi, lo + c * step);
+        lo += (c - 1) * step + 1;
     }
     return lo;
 }
 
-constexpr uint32_t kMergeSeg = 64;   // merged elements per thread
+// Elements k0 .. k0 + kMergeTile - 1 of merge(A, B): f(o, i, v, from_b) for each of
+// the calling thread's, in order, o its place in the tile and i the number of A
+// elements of the tile before it.  Every thread of the CTA calls it.
+template <class F>
+__device__ __forceinline__ void merge_tile(MergeTile &t, const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb,
+                                           uint64_t k0, F f) {
+    const uint64_t k1 = min(na + nb, k0 + kMergeTile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 2) {
+        const uint64_t c = warp_merge_path(A, na, B, nb, warp ? k1 : k0, lane);
+        if (lane == 0) t.cut[warp] = c;
+    }
+    __syncthreads();
+    const uint64_t i0 = t.cut[0], j0 = k0 - i0;
+    const uint32_t n = (uint32_t)(k1 - k0), ta = (uint32_t)(t.cut[1] - i0), tb = n - ta;
+    for (uint32_t x = threadIdx.x; x < n; x += kMergeThreads) t.v[x] = x < ta ? A[i0 + x] : B[j0 + (x - ta)];
+    __syncthreads();
+    const uint64_t *a = t.v, *b = t.v + ta;
+    const uint32_t d = min(n, threadIdx.x * kMergePer), e = min(n, d + kMergePer);
+    uint32_t lo = d > tb ? d - tb : 0, hi = d < ta ? d : ta;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (tkey(a[mid]) <= tkey(b[d - mid - 1])) lo = mid + 1; else hi = mid;
+    }
+    uint32_t i = lo, j = d - lo;
+    for (uint32_t o = d; o < e; o++) {
+        const bool from_b = i >= ta || (j < tb && tkey(b[j]) < tkey(a[i]));
+        const uint64_t v = from_b ? b[j] : a[i];
+        f(o, i, v, from_b);
+        if (from_b) j++; else i++;
+    }
+}
+
+// The tile's elements k0 .. of merge(A, B) to out[0 ..), through shared memory
+// (a pad word per thread: no bank conflicts), so that the stores are coalesced.
+__device__ __forceinline__ void merge_tile_out(MergeTile &t, uint64_t *stage, const uint64_t *A, uint64_t na,
+                                               const uint64_t *B, uint64_t nb, uint64_t k0, uint64_t *out) {
+    merge_tile(t, A, na, B, nb, k0, [&](uint32_t o, uint32_t, uint64_t v, bool) { stage[o + o / kMergePer] = v; });
+    __syncthreads();
+    const uint32_t n = (uint32_t)(min(na + nb, k0 + kMergeTile) - k0);
+    for (uint32_t x = threadIdx.x; x < n; x += kMergeThreads) out[x] = stage[x + x / kMergePer];
+}
 
 // Merges sorted pairs of runs: run pair q covers in[q * 2 * run .. ) as
 // A = [q*2*run, q*2*run + run) and B = the next run (shorter at the end).
-static __global__ void merge_pass_kernel(const uint64_t *in, uint64_t n, uint64_t run, uint64_t *out) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t k0 = t * kMergeSeg;
-    if (k0 >= n) return;
-    const uint64_t pair = k0 / (2 * run);
-    const uint64_t base = pair * 2 * run;
-    const uint64_t na = min(run, n - base);
-    const uint64_t nb = min(run, n - base - na);
-    const uint64_t *A = in + base, *B = A + na;
-    const uint64_t kk0 = k0 - base, kk1 = min(na + nb, kk0 + kMergeSeg);
-    uint64_t i = merge_path(A, na, B, nb, kk0), j = kk0 - i;
-    for (uint64_t k = kk0; k < kk1; k++) {
-        if (j >= nb || (i < na && tkey(A[i]) <= tkey(B[j]))) out[base + k] = A[i++];
-        else out[base + k] = B[j++];
-    }
+static __global__ void __launch_bounds__(kMergeThreads)
+merge_pass_kernel(const uint64_t *in, uint64_t n, uint64_t run, uint64_t *out) {
+    __shared__ MergeTile t;
+    __shared__ uint64_t stage[kMergeTile + kMergeThreads];
+    const uint64_t k0 = (uint64_t)blockIdx.x * kMergeTile;
+    const uint64_t base = k0 / (2 * run) * (2 * run);
+    const uint64_t na = min(run, n - base), nb = min(run, n - base - na);
+    merge_tile_out(t, stage, in + base, na, in + base + na, nb, k0 - base, out + k0);
 }
 
 // Merges two sorted arrays into out.
-static __global__ void merge_kernel(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb, uint64_t *out) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t k0 = t * kMergeSeg;
-    if (k0 >= na + nb) return;
-    const uint64_t k1 = min(na + nb, k0 + kMergeSeg);
-    uint64_t i = merge_path(A, na, B, nb, k0), j = k0 - i;
-    for (uint64_t k = k0; k < k1; k++) {
-        if (j >= nb || (i < na && tkey(A[i]) <= tkey(B[j]))) out[k] = A[i++];
-        else out[k] = B[j++];
-    }
+static __global__ void __launch_bounds__(kMergeThreads)
+merge_kernel(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb, uint64_t *out) {
+    __shared__ MergeTile t;
+    __shared__ uint64_t stage[kMergeTile + kMergeThreads];
+    const uint64_t k0 = (uint64_t)blockIdx.x * kMergeTile;
+    merge_tile_out(t, stage, A, na, B, nb, k0, out + k0);
 }
 
 // Joins sorted R (A) with sorted S (B): every S tuple meets the run of equal
-// R keys just before its merge position.  r_is_a selects which side A is,
-// for the checksum's (r_payload, s_payload) order.
-static __global__ void merge_join_kernel(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb, int a_is_r,
-                                  unsigned long long *acc) {
+// R keys just before its merge position (in the tile, and before it where the
+// run began earlier).  r_is_a selects which side A is, for the checksum's
+// (r_payload, s_payload) order.
+static __global__ void __launch_bounds__(kMergeThreads)
+merge_join_kernel(const uint64_t *A, uint64_t na, const uint64_t *B, uint64_t nb, int a_is_r, unsigned long long *acc) {
+    __shared__ MergeTile t;
     __shared__ uint64_t red[64];
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t k0 = t * kMergeSeg;
     Acc ac;
-    if (k0 < na + nb) {
-        const uint64_t k1 = min(na + nb, k0 + kMergeSeg);
-        uint64_t i = merge_path(A, na, B, nb, k0), j = k0 - i;
-        for (uint64_t k = k0; k < k1; k++) {
-            if (j >= nb || (i < na && tkey(A[i]) <= tkey(B[j]))) {
-                i++;
-            } else {
-                const uint64_t b = B[j++];
-                const uint32_t key = tkey(b);
-                for (int64_t q = (int64_t)i - 1; q >= 0 && tkey(A[q]) == key; q--) {
-                    ac.count++;
-                    ac.sum += a_is_r ? pair_hash(key, tpay(A[q]), tpay(b)) : pair_hash(key, tpay(b), tpay(A[q]));
-                }
-            }
-        }
-    }
+    merge_tile(t, A, na, B, nb, (uint64_t)blockIdx.x * kMergeTile, [&](uint32_t, uint32_t i, uint64_t b, bool from_b) {
+        if (!from_b) return;
+        const uint32_t key = tkey(b);
+        auto add = [&](uint64_t x) {
+            ac.count++;
+            ac.sum += a_is_r ? pair_hash(key, tpay(x), tpay(b)) : pair_hash(key, tpay(b), tpay(x));
+        };
+        int64_t q = (int64_t)i - 1;
+        for (; q >= 0 && tkey(t.v[q]) == key; q--) add(t.v[q]);
+        if (q < 0)
+            for (q = (int64_t)t.cut[0] - 1; q >= 0 && tkey(A[q]) == key; q--) add(A[q]);
+    });
     block_flush(ac, acc, red);
 }
 
