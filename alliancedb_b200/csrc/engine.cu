@@ -329,12 +329,12 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return radix_scratch(nR, nS, radix_bits_for(nR, p ? p->radix_bits : 0), num_sms);
+            return radix_scratch(nR, nS, radix_bits_for(nR, nS, p ? p->radix_bits : 0), num_sms);
         case Family::Npo:
             if (npo_partitioned(nR, nS, p ? p->radix_bits : 0))
-                return radix_scratch(nR, nS, radix_bits_for(nR, 0), num_sms);
+                return radix_scratch(nR, nS, radix_bits_for(nR, nS, 0), num_sms);
             return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
-        case Family::SortMerge: return radix_scratch(nR, nS, sort_bits_for(nR, p ? p->part_fanout : 0), num_sms);
+        case Family::SortMerge: return radix_scratch(nR, nS, sort_bits_for(nR, nS, p ? p->part_fanout : 0), num_sms);
         case Family::Shj:
         case Family::Pmj:
             return eager_scratch(nR, nS, a->fam, a->model, p && p->nthreads ? (int)p->nthreads : 1,
@@ -343,18 +343,34 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
     }
 }
 
+// Reserves the workspace of one join and `extra` bytes before it.  Where the
+// partitioned NPO's pages do not fit the device's free memory, its one table may:
+// *p then becomes *alt, which asks for that.
+static int reserve_for(Context *ctx, const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params **p,
+                       adb_join_params *alt, size_t extra) {
+    int s = ctx->ws.reserve(extra + scratch_for(a, nR, nS, *p, ctx->num_sms) + 4096);
+    if (s == ADB_ERR_OOM && a->fam == Family::Npo && !use_small(a, nR, nS, *p) &&
+        npo_partitioned(nR, nS, *p ? (*p)->radix_bits : 0)) {
+        if (*p) *alt = **p; else adb_params_default(alt);
+        alt->radix_bits = -1;
+        *p = alt;
+        s = ctx->ws.reserve(extra + scratch_for(a, nR, nS, *p, ctx->num_sms) + 4096);
+    }
+    return s;
+}
+
 static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const adb_join_params *p,
                     unsigned long long *acc) {
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return run_radix(ctx, j, radix_bits_for(j.nR, p ? p->radix_bits : 0), PartJoin::Chain, acc);
+            return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, p ? p->radix_bits : 0), PartJoin::Chain, acc);
         case Family::Npo:
             if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0))
-                return run_radix(ctx, j, radix_bits_for(j.nR, 0), PartJoin::HashedChain, acc);
+                return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, 0), PartJoin::HashedChain, acc);
             return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
         case Family::SortMerge:
-            return run_radix(ctx, j, sort_bits_for(j.nR, p ? p->part_fanout : 0), PartJoin::Sorted, acc);
+            return run_radix(ctx, j, sort_bits_for(j.nR, j.nS, p ? p->part_fanout : 0), PartJoin::Sorted, acc);
         case Family::Shj:
         case Family::Pmj:
             return run_eager(ctx, j, a->fam, a->model, eager_batch(p), p && p->nthreads ? (int)p->nthreads : 0,
@@ -475,7 +491,8 @@ int adb_join_device(const char *algo, const adb_tuple *dR, uint64_t nR, const ad
     if (!ctx) return out->status = s;
     cudaStream_t saved = ctx->stream;
     if (stream) ctx->stream = (cudaStream_t)stream;
-    s = ctx->ws.reserve(scratch_for(a, nR, nS, p, ctx->num_sms) + 4096);
+    adb_join_params alt;
+    s = reserve_for(ctx, a, nR, nS, &p, &alt, 0);
     if (s == ADB_OK) {
         DevJoin j{reinterpret_cast<const uint64_t *>(dR), nR, reinterpret_cast<const uint64_t *>(dS), nS};
         j.test_flags = p ? p->test_flags : 0;
@@ -505,7 +522,8 @@ int adb_join_materialize_device(const char *algo, const adb_tuple *dR, uint64_t 
     if (!ctx) return out->status = s;
     cudaStream_t saved = ctx->stream;
     if (stream) ctx->stream = (cudaStream_t)stream;
-    s = ctx->ws.reserve(scratch_for(a, nR, nS, p, ctx->num_sms) + 4096);
+    adb_join_params alt;
+    s = reserve_for(ctx, a, nR, nS, &p, &alt, 0);
     if (s == ADB_OK) {
         DevJoin j{reinterpret_cast<const uint64_t *>(dR), nR, reinterpret_cast<const uint64_t *>(dS), nS,
                   reinterpret_cast<uint64_t *>(dOut), cap};
@@ -530,7 +548,8 @@ int adb_join(const char *algo, const adb_tuple *R, uint64_t nR, const adb_tuple 
     Context *ctx = held_.ctx;
     if (!ctx) return out->status = s;
     const size_t in_bytes = Workspace::need(nR + 2, 8) + Workspace::need(nS + 2, 8);
-    s = ctx->ws.reserve(in_bytes + scratch_for(a, nR, nS, p, ctx->num_sms) + 4096);
+    adb_join_params alt;
+    s = reserve_for(ctx, a, nR, nS, &p, &alt, in_bytes);
     if (s) return out->status = s;
     uint64_t *dR = ctx->ws.take<uint64_t>(nR + 2);
     uint64_t *dS = ctx->ws.take<uint64_t>(nS + 2);

@@ -41,8 +41,8 @@ bool small_fits(uint64_t nR, uint64_t nS);
 int run_small(Context *ctx, const DevJoin &j);
 
 // ---- partitioned joins (PRO / RJ_st / PRH / PRHO, large NPO, m-way / m-pass / m-way+skew) ----
-int radix_bits_for(uint64_t nR, int requested);
-int sort_bits_for(uint64_t nR, int part_fanout);   // m-way / m-pass: joinconfig_t.PARTFANOUT, 0 = chosen
+int radix_bits_for(uint64_t nR, uint64_t nS, int requested);
+int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout);   // m-way / m-pass: joinconfig_t.PARTFANOUT, 0 = chosen
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
 // How a partition is joined: a chained table over digits of the key's low bits
 // or of its hash, or a counting sort (the sort-merge names).

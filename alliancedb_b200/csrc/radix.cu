@@ -65,20 +65,25 @@ static void launch_pass(const PassArgs &a, uint32_t F, int G, bool wide, cudaStr
 // at these bits (and at 2^12 tuples a partition, or one bit less): 2^16 - / 53
 // (4 bits 72), 2^18 64 / 71 (6 bits 73 / 83), 2^20 102 / 110 (7 bits 108 / 118), 2^21 133 /
 // 167 (9 bits 166 / 186), 2^22 228 / 256 (8 bits 223 / 273), 2^23 - / 410 (9 bits 450).
-int radix_bits_for(uint64_t nR, int requested) {
+// The largest relations leave 32-bit slot numbers less room for partial pages:
+// within 2^23 tuples of the limit no partitions beyond one R chunk each, above
+// 3 x 2^30 tuples at most 2^14.
+int radix_bits_for(uint64_t nR, uint64_t nS, int requested) {
     if (requested > 0) return requested > 15 ? 15 : requested;
     const int full = (int)ceil_log2_u64((nR + 8191) / 8192), fill = (int)ceil_log2_u64((nR + 255) / 256);
-    int b = fill > 8 ? 8 : fill;
+    const uint64_t larger = nR > nS ? nR : nS;
+    const int most = larger > 3ull << 30 ? 14 : 15;
+    int b = larger > (1ull << 32) - (1u << 23) ? 1 : fill > 8 ? 8 : fill;
     if (full > b) b = full;
     if (b < 1) b = 1;
-    if (b > 15) b = 15;
+    if (b > most) b = most;
     return b;
 }
 
 // m-way / m-pass: the fan-out joinconfig_t.PARTFANOUT asks for, rounded up to a
 // power of two (at most 2^15), else as above.
-int sort_bits_for(uint64_t nR, int part_fanout) {
-    return radix_bits_for(nR, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0);
+int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout) {
+    return radix_bits_for(nR, nS, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0);
 }
 
 // ---------------------------------------------------------------------------
