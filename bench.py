@@ -57,13 +57,13 @@ ALG_BYTES = {"PRO": 24, "RJ_st": 24, "PRH": 24, "PRHO": 24, "NPO": 16, "NPO_st":
 # launch is that figure times the launch's tuples: the kernels stream every
 # tuple once, so traffic grows in proportion.
 KERNELS = {
-    "radix": {0: ("partition_pass<0,512> (pass 1)", 16, (270247168 + 213934080) / 2**25),
-              1: ("partition_pass<1,512> (pass 2)", 16, (276288768 + 214363648) / 2**25),
-              3: ("radix_join_items", 8, (273622272 + 3668736) / 2**25)},
+    "radix": {0: ("partition_pass<0,512,6144> (pass 1)", 16, (269430016 + 214572288) / 2**25),
+              1: ("partition_pass<1,512,8192> (pass 2)", 16, (274856704 + 217763840) / 2**25),
+              3: ("radix_join_items", 8, (281964544 + 3466752) / 2**25)},
     "npo": {1: ("npo_build", 8, None), 3: ("npo_probe", 8, None)},
-    "smj": {0: ("partition_pass<0,512,hashed> (pass 1)", 16, None),
-            1: ("partition_pass<1,512,hashed> (pass 2)", 16, None),
-            3: ("radix_join_items (sort + merge)", 8, None)},
+    "smj": {0: ("partition_pass<0,512,6144,hashed> (pass 1)", 16, None),
+            1: ("partition_pass<1,512,8192,hashed> (pass 2)", 16, None),
+            3: ("radix_join_items<sorted>", 8, (282349568 + 3129088) / 2**25)},
 }
 
 
