@@ -614,7 +614,14 @@ int adb_host_alloc_pinned(void **ptr, size_t bytes) {
     return ADB_OK;
 }
 int adb_host_free_pinned(void *ptr) { ADB_CK(cudaFreeHost(ptr)); return ADB_OK; }
-int adb_memcpy_h2d(void *dst, const void *src, size_t bytes) { ADB_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice)); return ADB_OK; }
+// cudaMemcpy from pageable memory may return while the last staged part is still
+// on its way to the device, and the library's own stream does not wait for the
+// legacy one that carries it: so the copy is waited for here.
+int adb_memcpy_h2d(void *dst, const void *src, size_t bytes) {
+    ADB_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    ADB_CK(cudaStreamSynchronize(cudaStreamLegacy));
+    return ADB_OK;
+}
 int adb_memcpy_d2h(void *dst, const void *src, size_t bytes) { ADB_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost)); return ADB_OK; }
 int adb_device_sync(void) { ADB_CK(cudaDeviceSynchronize()); return ADB_OK; }
 int adb_release_workspace(void) {
