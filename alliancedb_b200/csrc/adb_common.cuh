@@ -78,6 +78,27 @@ __device__ __forceinline__ void block_flush(Acc a, unsigned long long *out, uint
     __syncthreads();
 }
 
+// Loads of words that other CTAs of the same launch wrote, after a ticket showed
+// that they are done: from L2, and not moved ahead of the ticket (volatile).
+__device__ __forceinline__ ulonglong2 ld_done(const ulonglong2 *p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 ld_done(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_done(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // One thread per CTA of a call's last kernel, after the CTA's sums are in acc:
 // the last of them hands acc[0 .. 3] to the host (out: pinned memory) and
 // leaves the accumulators at 0 for the next call, so that neither a clear nor a
@@ -87,7 +108,7 @@ __device__ __forceinline__ void finish_call(unsigned long long *acc, unsigned lo
     if (atomicAdd(acc + 5, 1ull) != (unsigned long long)gridDim.x * gridDim.y - 1) return;
     __threadfence();
     ulonglong2 *a2 = reinterpret_cast<ulonglong2 *>(acc), *o2 = reinterpret_cast<ulonglong2 *>(out);
-    const ulonglong2 lo = __ldcg(a2), hi = __ldcg(a2 + 1);
+    const ulonglong2 lo = ld_done(a2), hi = ld_done(a2 + 1);
     o2[0] = lo;
     o2[1] = hi;
     for (int k = 0; k < 3; k++) a2[k] = make_ulonglong2(0, 0);

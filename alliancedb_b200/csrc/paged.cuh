@@ -550,12 +550,12 @@ __device__ __forceinline__ void scan_list(const uint32_t *t, uint32_t n, uint32_
     const uint4 *t4 = reinterpret_cast<const uint4 *>(t);
     uint32_t before = 0, tot;
     for (uint32_t i = threadIdx.x; i < b * (kScanThreads / 4); i += kScanThreads) {
-        const uint4 v = __ldcg(t4 + i);
+        const uint4 v = ld_done(t4 + i);
         before += v.x + v.y + v.z + v.w;
     }
     block_exclusive_scan(before, tmp, &before);
     const uint32_t i = b * kScanThreads + threadIdx.x;
-    const uint32_t v = i < n ? __ldcg(t + i) : 0u;
+    const uint32_t v = i < n ? ld_done(t + i) : 0u;
     const uint32_t ex = block_exclusive_scan(v, tmp, &tot);
     if (i < n) out[i] = before + ex;
     if (i + 1 == n) {
