@@ -450,13 +450,27 @@ partition_pass(PassArgs a) {
             }
             __syncthreads();   // every B warp has read misc[0] and written its total
             if (bw < (int)nbw) {
-                // totals of the warps before this one, and of all of them
+                // totals of the warps before this one, and of all of them: by a
+                // shuffle scan, or where four warps are usual one by one (2^22 x
+                // 2^22, 16 warps: pass 1 58.6 -> 56.3 us; 512 batched windows 5.275 ->
+                // 5.255 ms; 2^27 x 2^27, four warps: pass 2 1.038 -> 1.057 ms)
                 uint32_t before_t = 0, before_p = 0, all_t = 0, all_p = 0;
-                for (uint32_t k = 0; k < nbw; k++) {
-                    const uint32_t tv = misc[8 + k];
-                    if ((int)k < bw) { before_t += tv & 0xFFFFu; before_p += tv >> 16; }
-                    all_t += tv & 0xFFFFu;
-                    all_p += tv >> 16;
+                if (!kPaged) {
+                    const uint32_t tv = lane < (int)nbw ? misc[8 + lane] : 0u;
+                    const uint32_t sums = warp_incl_scan(tv, lane);   // both halves stay below 2^16
+                    const uint32_t all = __shfl_sync(0xffffffffu, sums, 31);
+                    const uint32_t before = __shfl_sync(0xffffffffu, sums - tv, bw);
+                    before_t = before & 0xFFFFu;
+                    before_p = before >> 16;
+                    all_t = all & 0xFFFFu;
+                    all_p = all >> 16;
+                } else {
+                    for (uint32_t k = 0; k < nbw; k++) {
+                        const uint32_t tv = misc[8 + k];
+                        if ((int)k < bw) { before_t += tv & 0xFFFFu; before_p += tv >> 16; }
+                        all_t += tv & 0xFFFFu;
+                        all_p += tv >> 16;
+                    }
                 }
                 const uint32_t ex = inc - (L | (need << 16));
                 if (d < F) run_digit(d, L, p, before_t + (ex & 0xFFFFu), pool0 + before_p + (ex >> 16));
