@@ -173,7 +173,7 @@ Context *ctx_create(int dev, int *status) {
     for (auto &e : c->ev)
         if (cudaEventCreate(&e) != cudaSuccess) goto fail;
     if (cudaMallocHost(&c->h_res, 64 * sizeof(unsigned long long)) != cudaSuccess) goto fail;
-    if (cudaMalloc(&c->d_acc, 64) != cudaSuccess || cudaMemset(c->d_acc, 0, 64) != cudaSuccess) goto fail;
+    if (cudaMalloc(&c->d_acc, kAccBytes) != cudaSuccess || cudaMemset(c->d_acc, 0, kAccBytes) != cudaSuccess) goto fail;
     if (cudaDeviceSynchronize() != cudaSuccess) goto fail;   // the library's stream does not wait for the clear
     {
         int s = radix_set_attrs();
@@ -321,7 +321,7 @@ static uint64_t eager_batch(const adb_join_params *p) {
 // device time: PRO 72 us partitioned, NPO 33 us with a table in L2, 9 us here.
 static bool use_small(const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params *p) {
     return (a->fam == Family::Radix || a->fam == Family::RadixHist || a->fam == Family::Npo) && nR && nS &&
-           small_fits(nR, nS) && !(p && (p->radix_bits || p->test_flags));
+           small_fits(nR, nS) && !(p && (p->radix_bits || p->test_flags & ADB_TEST_WAITS_RUN_OUT));
 }
 
 static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params *p, int num_sms) {
@@ -380,10 +380,8 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
     }
 }
 
-// Runs one join on device-resident inputs; inputs may live inside the workspace
-// region [0, pre) that the caller already reserved.
-static int join_device_core(Context *ctx, const AlgoEntry *a, DevJoin j, const adb_join_params *p,
-                            adb_join_result *out, size_t pre_bytes) {
+static int join_device_run(Context *ctx, const AlgoEntry *a, const DevJoin &j, const adb_join_params *p,
+                           adb_join_result *out, size_t pre_bytes) {
     cudaStream_t st = ctx->stream;
     ctx->kernels = 0;
     ctx->marks = 0;
@@ -399,14 +397,14 @@ static int join_device_core(Context *ctx, const AlgoEntry *a, DevJoin j, const a
         ADB_TRY(run_small(ctx, j));
     } else {
         if (eager) {
-            acc = ctx->ws.take<unsigned long long>(8);
-            ADB_CK(cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st));
+            acc = ctx->ws.take<unsigned long long>(kAccBytes / sizeof(unsigned long long));
+            ADB_CK(cudaMemsetAsync(acc, 0, kAccBytes, st));
         }
-        const int rc = dispatch(ctx, a, j, p, acc);
-        if (rc != ADB_OK) {
-            if (!eager) cudaMemsetAsync(acc, 0, 8 * sizeof(unsigned long long), st);   // 0 between calls
-            return rc;
-        }
+        ADB_TRY(dispatch(ctx, a, j, p, acc));
+    }
+    if (j.test_flags & ADB_TEST_CALL_FAILS) {
+        set_error("ADB_TEST_CALL_FAILS: the call gives up with its kernels queued");
+        return ADB_ERR_DEVICE;
     }
     ADB_CK(cudaEventRecord(ctx->ev[6], st));
     if (j.nR && j.nS && eager)
@@ -431,6 +429,23 @@ static int join_device_core(Context *ctx, const AlgoEntry *a, DevJoin j, const a
         return ADB_ERR_TIMEOUT;
     }
     return ADB_OK;
+}
+
+// Runs one join on device-resident inputs; inputs may live inside the workspace
+// region [0, pre) that the caller already reserved.
+//
+// A call that fails may leave kernels queued that add to the accumulators and
+// use the workspace, and the next call may come on another stream: so they are
+// waited for, and the accumulators cleared, before the context is handed on.
+static int join_device_core(Context *ctx, const AlgoEntry *a, const DevJoin &j, const adb_join_params *p,
+                            adb_join_result *out, size_t pre_bytes) {
+    const int s = join_device_run(ctx, a, j, p, out, pre_bytes);
+    if (s != ADB_OK) {
+        cudaStreamSynchronize(ctx->stream);
+        if (cudaMemsetAsync(ctx->d_acc, 0, kAccBytes, ctx->stream) == cudaSuccess) cudaStreamSynchronize(ctx->stream);
+        cudaGetLastError();   // s and its message stand
+    }
+    return s;
 }
 
 static int check_sizes(uint64_t nR, uint64_t nS) {

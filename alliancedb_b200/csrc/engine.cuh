@@ -30,6 +30,7 @@ int h2d_copy(Context *ctx, void *dst, const void *src, size_t bytes, cudaStream_
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
         if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError();   /* reported here: not the next launch's error */        \
             ::adb::set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_),      \
                              __FILE__, __LINE__);                                         \
             return e_ == cudaErrorMemoryAllocation ? ADB_ERR_OOM : ADB_ERR_DEVICE;        \
@@ -66,6 +67,10 @@ struct Workspace {
 // host; longer streams are checked on the device after their copy.
 constexpr uint64_t kHostOrderCheck = 1ull << 16;
 
+// The accumulators of a join: count, checksum, error word, materialised count,
+// NPO's build tuples equal to its empty marker, CTAs done, two unused words.
+constexpr size_t kAccBytes = 8 * sizeof(unsigned long long);
+
 struct Context {
     int device = -1;
     int num_sms = kNumSMs;
@@ -73,7 +78,7 @@ struct Context {
     cudaEvent_t ev[12] = {};
     Workspace ws;
     unsigned long long *h_res = nullptr;   // pinned: [0] count [1] checksum [2] err [3] mat_n ...
-    unsigned long long *d_acc = nullptr;   // device accumulators (8 words), 0 between calls
+    unsigned long long *d_acc = nullptr;   // device accumulators (kAccBytes), 0 between calls
     unsigned marks = 0;                    // phase events recorded by the current call (bit k: ev[k])
     // pinned, grow-only host buffers of the batched path: the per-call plan (one
     // host -> device copy) and the per-window results (one copy back); growing

@@ -5,7 +5,8 @@
 // word (a timed-out device wait sets it), acc[3] the materialised count, acc[4]
 // NPO's build tuples equal to its empty marker, acc[5] the CTAs done.  All but
 // the eager drivers end with a kernel that moves acc[0 .. 3] to ctx->h_res and
-// clears acc (finish_call); run_eager leaves that to its caller.
+// clears acc (finish_call); run_eager leaves that to its caller.  After a driver
+// that failed half-way, the caller waits for the stream and clears acc.
 #pragma once
 
 #include "engine.cuh"

@@ -88,10 +88,13 @@ typedef struct adb_join_params {
     int32_t test_flags;         /* 0 in normal use.  ADB_TEST_WAITS_RUN_OUT: the partitioned and
                                    sort-merge joins do their work and then report that a bounded device
                                    wait ran out, so callers can test their ADB_ERR_TIMEOUT handling
-                                   without making a GPU wait for real */
+                                   without making a GPU wait for real.  ADB_TEST_CALL_FAILS: the call
+                                   returns ADB_ERR_DEVICE with its kernels queued, as after a CUDA call
+                                   that failed half-way */
 } adb_join_params;
 
 #define ADB_TEST_WAITS_RUN_OUT 1
+#define ADB_TEST_CALL_FAILS 2
 
 typedef struct adb_join_result {
     uint64_t count;             /* result_t.totalresults */
