@@ -44,6 +44,11 @@ __host__ __device__ __forceinline__ uint64_t pair_hash(uint32_t key, uint32_t r_
     return pair_hash_pre(key, r_pay, s_half(key, s_pay));
 }
 
+// Error words (acc[2]) of the kernels' own checks.  Neither can occur while the
+// host sizes tables and pools as it does.
+constexpr int kErrTableFull = 2;      // an insert found no free slot
+constexpr int kErrPagesUsedUp = 3;    // a partition pass ran past its page pool
+
 // Count + checksum accumulator; sums are exact mod 2^64 and order-independent.
 struct Acc {
     uint64_t count = 0;

@@ -266,8 +266,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     ja.Rcount = a.out[0].pcount; ja.Scount = a.out[1].pcount;
     ja.Rlist = a.out[0].plist; ja.Slist = a.out[1].plist;
     ja.pstart = pstart; ja.wl = wl;
-    ja.acc = acc; ja.out = nullptr; ja.err = reinterpret_cast<int *>(acc + 2);
-    ja.waits_run_out = 0;
+    ja.acc = acc; ja.out = nullptr;
     ja.F = Dt;
     ja.bits = 0;   // per-window fan-out: the kernel reads each window's bits
     ja.mat = nullptr; ja.mat_n = nullptr; ja.mat_cap = 0;

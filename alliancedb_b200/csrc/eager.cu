@@ -109,7 +109,7 @@ __device__ __forceinline__ void shj_insert(const ShjTables &t, int side, uint64_
             return;
         }
         slot = (slot + 1) & m;
-        if (tries > m) { atomicExch(err, 2); return; }   // table full: cannot happen at load <= 0.5
+        if (tries > m) { atomicExch(err, kErrTableFull); return; }   // table full: cannot happen at load <= 0.5
     }
 }
 

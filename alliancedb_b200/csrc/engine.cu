@@ -321,7 +321,7 @@ static uint64_t eager_batch(const adb_join_params *p) {
 // device time: PRO 72 us partitioned, NPO 33 us with a table in L2, 9 us here.
 static bool use_small(const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params *p) {
     return (a->fam == Family::Radix || a->fam == Family::RadixHist || a->fam == Family::Npo) && nR && nS &&
-           small_fits(nR, nS) && !(p && (p->radix_bits || p->test_flags & ADB_TEST_WAITS_RUN_OUT));
+           small_fits(nR, nS) && !(p && p->radix_bits);
 }
 
 static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params *p, int num_sms) {
@@ -380,6 +380,23 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
     }
 }
 
+// The status of a finished join's error word: 0, or a kernel's own check that
+// failed.  No join waits for anything on the device but its own launches' order,
+// so ADB_ERR_TIMEOUT comes from the test flag alone.
+static int check_error_word(const AlgoEntry *a, const DevJoin &j, unsigned long long word) {
+    const bool partitioned = a->fam == Family::Radix || a->fam == Family::RadixHist || a->fam == Family::SortMerge;
+    if (partitioned && j.nR && j.nS && j.test_flags & ADB_TEST_WAITS_RUN_OUT) {
+        set_error("a bounded device wait ran out (ADB_TEST_WAITS_RUN_OUT)");
+        return ADB_ERR_TIMEOUT;
+    }
+    if (const int test = j.test_flags >> ADB_TEST_ERROR_WORD_SHIFT) word = (unsigned long long)test;
+    if (!word) return ADB_OK;
+    set_error("a kernel's own check failed: %s (error word %llu); the result is not valid",
+              word == kErrTableFull ? "hash table full" : word == kErrPagesUsedUp ? "page pool used up" : "unknown",
+              word);
+    return ADB_ERR_DEVICE;
+}
+
 static int join_device_run(Context *ctx, const AlgoEntry *a, const DevJoin &j, const adb_join_params *p,
                            adb_join_result *out, size_t pre_bytes) {
     cudaStream_t st = ctx->stream;
@@ -424,11 +441,7 @@ static int join_device_run(Context *ctx, const AlgoEntry *a, const DevJoin &j, c
     for (int k = 0; k < 4; k++) out->ms_phase[k] = t[k];
     out->ms_device = tot;
     out->kernels = ctx->kernels;
-    if (ctx->h_res[2]) {
-        set_error("a bounded device wait ran out (error word %llu)", ctx->h_res[2]);
-        return ADB_ERR_TIMEOUT;
-    }
-    return ADB_OK;
+    return check_error_word(a, j, ctx->h_res[2]);
 }
 
 // Runs one join on device-resident inputs; inputs may live inside the workspace

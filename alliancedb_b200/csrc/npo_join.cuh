@@ -35,7 +35,7 @@ __device__ __forceinline__ void npo_insert_from(uint64_t *table, uint64_t mask, 
                                                   (unsigned long long)kEmpty, (unsigned long long)w);
         if (prev == kEmpty) return;
         slot = (slot + 1) & mask;
-        if (++tries > mask) { atomicExch(err, 2); return; }   // table full: cannot happen at load <= 0.5
+        if (++tries > mask) { atomicExch(err, kErrTableFull); return; }   // table full: cannot happen at load <= 0.5
     }
 }
 
@@ -193,7 +193,7 @@ npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ ta
             } else {
                 b = b + 1 == nb ? 0 : b + 1;
             }
-            if (tries > 8ull * nb) { atomicExch(err, 2); break; }   // table full: cannot happen at load <= 0.5
+            if (tries > 8ull * nb) { atomicExch(err, kErrTableFull); break; }   // table full: cannot happen at load <= 0.5
         }
     }
 }

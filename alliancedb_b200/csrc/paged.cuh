@@ -376,7 +376,7 @@ partition_pass(PassArgs a) {
             if (L > room) {
                 const uint32_t need = (L - room + kPageTuples - 1) / kPageTuples;
                 if (first + need > pool_cap) {   // cannot happen: the pool covers the input
-                    atomicExch(a.err, 3);
+                    atomicExch(a.err, kErrPagesUsedUp);
                     first = pool_cap - need;
                 }
                 const uint32_t nx = (pool_base + first) * kPageTuples - room;

@@ -296,8 +296,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
     a.Rcount = po.R.pcount; a.Scount = po.S.pcount;
     a.Rlist = po.R.plist; a.Slist = po.S.plist;
     a.pstart = po.pstart; a.wl = wl;
-    a.acc = acc; a.out = ctx->h_res; a.err = reinterpret_cast<int *>(acc + 2);
-    a.waits_run_out = j.test_flags & ADB_TEST_WAITS_RUN_OUT;
+    a.acc = acc; a.out = ctx->h_res;
     a.F = F; a.bits = (uint32_t)bits;
     a.mat = j.mat; a.mat_n = acc + 3; a.mat_cap = j.mat_cap;
     a.wbase = nullptr; a.wbits = nullptr; a.nwin = 0; a.wacc = nullptr;

@@ -192,8 +192,6 @@ struct JoinArgs {
     WorkList wl;
     unsigned long long *acc;         // [0] count, [1] checksum
     unsigned long long *out;         // pinned host copy of acc[0 .. 3], written by the last CTA (null: none)
-    int *err;
-    int waits_run_out;               // ADB_TEST_WAITS_RUN_OUT: report a wait that ran out
     uint32_t F;
     uint32_t bits;                   // bits the partitioning consumed (the hash skips them)
     uint64_t *mat;                   // optional <S-key, S-payload> output
@@ -393,7 +391,6 @@ radix_join_items(JoinArgs a) {
         auto same = [&](uint32_t w, uint32_t x) { return kHashed ? (w ^ x) << link == 0 : (w ^ x) < lim; };
         for (uint32_t i = threadIdx.x; i < ((1u << lnb) + 3) / 4; i += kJoinThreads)
             reinterpret_cast<uint4 *>(heads)[i] = kSorted ? make_uint4(0, 0, 0, 0) : make_uint4(kNone, kNone, kNone, kNone);
-        if (a.waits_run_out && threadIdx.x == 0) atomicExch(a.err, 1);
         __syncthreads();
 
         // --- build: a warp per page, two tuples per lane, kB pages in flight

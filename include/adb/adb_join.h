@@ -56,8 +56,8 @@ typedef enum adb_status {
     ADB_OK = 0,
     ADB_ERR_ARG = 1,         /* bad argument: NULL pointer, unknown algorithm, size out of range */
     ADB_ERR_OOM = 2,         /* device or pinned-host allocation failed */
-    ADB_ERR_DEVICE = 3,      /* a CUDA call failed; the message says which */
-    ADB_ERR_TIMEOUT = 4,     /* a bounded device wait ran out */
+    ADB_ERR_DEVICE = 3,      /* a CUDA call failed, or a kernel's own check; the message says which */
+    ADB_ERR_TIMEOUT = 4,     /* a bounded device wait ran out (no join has one: ADB_TEST_WAITS_RUN_OUT only) */
     ADB_ERR_UNSUPPORTED = 5, /* name known to the reference but not provided (adb_algo_name reports which) */
     ADB_ERR_BUSY = 6,        /* admission refused: over the device-memory budget */
     ADB_ERR_NO_DEVICE = 7    /* no CUDA device, or the kernels were not built for it */
@@ -85,16 +85,18 @@ typedef struct adb_join_params {
     uint64_t seed;              /* JBCR's random split of S */
     int32_t realtime;           /* adb_stream_join: 1 = release each micro-batch at its timestamp
                                    (wall clock, the reference's WAIT gating, fetcher.cpp:120-190) */
-    int32_t test_flags;         /* 0 in normal use.  ADB_TEST_WAITS_RUN_OUT: the partitioned and
-                                   sort-merge joins do their work and then report that a bounded device
-                                   wait ran out, so callers can test their ADB_ERR_TIMEOUT handling
-                                   without making a GPU wait for real.  ADB_TEST_CALL_FAILS: the call
-                                   returns ADB_ERR_DEVICE with its kernels queued, as after a CUDA call
-                                   that failed half-way */
+    int32_t test_flags;         /* 0 in normal use; for callers that test their error handling.  The host
+                                   injects the error, the kernels run as ever.  ADB_TEST_WAITS_RUN_OUT:
+                                   the PRO family and the sort-merge names return ADB_ERR_TIMEOUT after
+                                   their work.  ADB_TEST_CALL_FAILS: the call returns ADB_ERR_DEVICE with
+                                   its kernels queued, as after a CUDA call that failed half-way.
+                                   ADB_TEST_ERROR_WORD(w): as if a kernel's check had left error word w */
 } adb_join_params;
 
 #define ADB_TEST_WAITS_RUN_OUT 1
 #define ADB_TEST_CALL_FAILS 2
+#define ADB_TEST_ERROR_WORD_SHIFT 8
+#define ADB_TEST_ERROR_WORD(w) ((w) << ADB_TEST_ERROR_WORD_SHIFT)   /* 2: table full, 3: page pool used up */
 
 typedef struct adb_join_result {
     uint64_t count;             /* result_t.totalresults */

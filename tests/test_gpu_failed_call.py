@@ -44,3 +44,23 @@ def test_an_error_is_reported_once(oracle):
     assert adb.lib().adb_host_free_pinned(R.ctypes.data) == adb.ADB_ERR_DEVICE   # not pinned memory
     got = adb.join_device("PRO", dR.ptr, 3000, dS.ptr, 5000)
     assert (got.count, got.checksum) == oracle.truth(R, S)
+
+
+@pytest.mark.parametrize("algo", ["PRO", "NPO", "m-way", "SHJ_JM_NP"])
+@pytest.mark.parametrize("word,says", [(2, "table full"), (3, "page pool")])
+def test_a_kernels_check_is_not_a_timeout(oracle, algo, word, says):
+    R = adb.gen_pk(20000, 47)
+    S = adb.gen_fk(30000, R, 0.0, 48)
+    with pytest.raises(adb.AdbError) as e:
+        adb.join(algo, R, S, adb.default_params(test_flags=word << 8))
+    assert e.value.status == adb.ADB_ERR_DEVICE and says in str(e.value)
+    got = adb.join(algo, R, S)
+    assert (got.count, got.checksum) == oracle.pk_truth(R, S)
+
+
+@pytest.mark.parametrize("n", [1 << 14, (7 << 19) + 1])
+def test_npo_has_no_wait_to_run_out_at_any_size(oracle, n):
+    R = adb.gen_pk(n, 49)
+    S = adb.gen_fk(n, R, 0.0, 50)
+    got = adb.join("NPO", R, S, adb.default_params(test_flags=1))
+    assert (got.count, got.checksum) == oracle.pk_truth(R, S)
