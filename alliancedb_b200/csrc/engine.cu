@@ -329,12 +329,13 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return radix_scratch(nR, nS, radix_bits_for(nR, nS, p ? p->radix_bits : 0), num_sms);
+            return radix_scratch(nR, nS, radix_bits_for(nR, nS, p ? p->radix_bits : 0, num_sms), num_sms);
         case Family::Npo:
             if (npo_partitioned(nR, nS, p ? p->radix_bits : 0))
-                return radix_scratch(nR, nS, radix_bits_for(nR, nS, 0), num_sms);
+                return radix_scratch(nR, nS, radix_bits_for(nR, nS, 0, num_sms), num_sms);
             return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
-        case Family::SortMerge: return radix_scratch(nR, nS, sort_bits_for(nR, nS, p ? p->part_fanout : 0), num_sms);
+        case Family::SortMerge:
+            return radix_scratch(nR, nS, sort_bits_for(nR, nS, p ? p->part_fanout : 0, num_sms), num_sms);
         case Family::Shj:
         case Family::Pmj:
             return eager_scratch(nR, nS, a->fam, a->model, p && p->nthreads ? (int)p->nthreads : 1,
@@ -343,20 +344,29 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
     }
 }
 
-// Reserves the workspace of one join and `extra` bytes before it.  Where the
-// partitioned NPO's pages do not fit the device's free memory, its one table may:
-// *p then becomes *alt, which asks for that.
+// Reserves the workspace of one join and `extra` bytes before it.  Where that
+// does not fit the device's free memory, a form of the join that takes less may:
+// half the partitions (fewer partly filled pages, or one pass instead of two),
+// or NPO's one table instead of pages.  *p then becomes *alt, which asks for it.
 static int reserve_for(Context *ctx, const AlgoEntry *a, uint64_t nR, uint64_t nS, const adb_join_params **p,
                        adb_join_params *alt, size_t extra) {
-    int s = ctx->ws.reserve(extra + scratch_for(a, nR, nS, *p, ctx->num_sms) + 4096);
-    if (s == ADB_ERR_OOM && a->fam == Family::Npo && !use_small(a, nR, nS, *p) &&
-        npo_partitioned(nR, nS, *p ? (*p)->radix_bits : 0)) {
-        if (*p) *alt = **p; else adb_params_default(alt);
+    auto reserve = [&] { return ctx->ws.reserve(extra + scratch_for(a, nR, nS, *p, ctx->num_sms) + 4096); };
+    const int s = reserve();
+    if (s != ADB_ERR_OOM || !nR || !nS || use_small(a, nR, nS, *p)) return s;
+    if (*p) *alt = **p; else adb_params_default(alt);
+    if (a->fam == Family::Radix || a->fam == Family::RadixHist) {
+        alt->radix_bits = radix_bits_for(nR, nS, alt->radix_bits, ctx->num_sms) - 1;
+        if (!alt->radix_bits) return s;
+    } else if (a->fam == Family::SortMerge) {
+        alt->part_fanout = 1 << (sort_bits_for(nR, nS, alt->part_fanout, ctx->num_sms) - 1);
+        if (alt->part_fanout < 2) return s;
+    } else if (a->fam == Family::Npo && npo_partitioned(nR, nS, alt->radix_bits)) {
         alt->radix_bits = -1;
-        *p = alt;
-        s = ctx->ws.reserve(extra + scratch_for(a, nR, nS, *p, ctx->num_sms) + 4096);
+    } else {
+        return s;
     }
-    return s;
+    *p = alt;
+    return reserve();
 }
 
 static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const adb_join_params *p,
@@ -364,13 +374,15 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
     switch (a->fam) {
         case Family::Radix:
         case Family::RadixHist:
-            return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, p ? p->radix_bits : 0), PartJoin::Chain, acc);
+            return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, p ? p->radix_bits : 0, ctx->num_sms), PartJoin::Chain,
+                             acc);
         case Family::Npo:
             if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0))
-                return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, 0), PartJoin::HashedChain, acc);
+                return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, 0, ctx->num_sms), PartJoin::HashedChain, acc);
             return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
         case Family::SortMerge:
-            return run_radix(ctx, j, sort_bits_for(j.nR, j.nS, p ? p->part_fanout : 0), PartJoin::Sorted, acc);
+            return run_radix(ctx, j, sort_bits_for(j.nR, j.nS, p ? p->part_fanout : 0, ctx->num_sms), PartJoin::Sorted,
+                             acc);
         case Family::Shj:
         case Family::Pmj:
             return run_eager(ctx, j, a->fam, a->model, eager_batch(p), p && p->nthreads ? (int)p->nthreads : 0,

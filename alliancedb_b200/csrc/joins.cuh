@@ -33,7 +33,6 @@ enum class Family { Radix, RadixHist, Npo, SortMerge, Shj, Pmj, Unsupported };
 struct PartOut;
 struct DigitFn;
 size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms);
-uint64_t paged_final_pool_pages(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms);
 int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitFn *d2, PartOut *out,
                         unsigned long long *acc, uint32_t **ctr = nullptr);
 
@@ -42,8 +41,8 @@ bool small_fits(uint64_t nR, uint64_t nS);
 int run_small(Context *ctx, const DevJoin &j);
 
 // ---- partitioned joins (PRO / RJ_st / PRH / PRHO, large NPO, m-way / m-pass / m-way+skew) ----
-int radix_bits_for(uint64_t nR, uint64_t nS, int requested);
-int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout);   // m-way / m-pass: joinconfig_t.PARTFANOUT, 0 = chosen
+int radix_bits_for(uint64_t nR, uint64_t nS, int requested, int num_sms);
+int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout, int num_sms);   // joinconfig_t.PARTFANOUT, 0 = chosen
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
 // How a partition is joined: a chained table over digits of the key's low bits
 // or of its hash, or a counting sort (the sort-merge names).

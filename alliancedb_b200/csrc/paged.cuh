@@ -52,7 +52,7 @@ struct PageSet {
     uint32_t *log;       // output digit of each pool page
     uint8_t *pcount;     // tuples in each pool page
     uint32_t *nlog;      // [G] pages used by each CTA
-    uint32_t *doff;      // at the CTA's first pool page + d: its place among digit d's pages
+    uint32_t *doff;      // its place among digit d's pages at doff_at(CTA) + d
     uint2 *udesc;        // [G] each CTA's first output digit and digit count
     uint32_t *plist;     // page list grouped by output digit (filled by page_place)
     uint64_t *pstart;    // [Fout + 1] page-list starts
@@ -92,7 +92,7 @@ struct PassArgs {
     PageSet out[2];
     DigitFn df;          // this pass's digit (F = df.mask + 1 <= 512)
     uint32_t F1;         // input partitions (1 for flat input)
-    int G;               // CTAs per relation: flat chunks, or the bound on work units
+    int G;               // CTAs per relation, the larger bound: flat chunks, or work units
     uint32_t pool_cap;   // pages per CTA pool
     uint32_t unit_pages; // paged input: pages per work unit
     uint64_t unit_tuples;// segmented input: tuples per work unit
@@ -101,6 +101,12 @@ struct PassArgs {
     uint32_t Dtot;
     int *err;
 };
+
+// Where CTA g's doff entries begin: F per CTA, or for segmented input, where F
+// differs, at the CTA's first pool page (a pool has more pages than digits).
+__device__ __forceinline__ uint32_t doff_at(int mode, uint32_t g, uint32_t F, uint32_t pool_base) {
+    return mode == 2 ? pool_base : g * F;
+}
 
 __host__ __device__ __forceinline__ uint32_t flat_pool_cap(uint64_t n, int G, uint32_t F) {
     return (uint32_t)((chunk_of(n, G) + kPageTuples - 1) / kPageTuples + F + 1);
@@ -545,7 +551,7 @@ partition_pass(PassArgs a) {
     // F. pages per digit of this CTA
     uint32_t *tot = a.totals + (size_t)relidx * a.Dtot;
     for (uint32_t d = tid; d < F; d += kThreads)
-        if (npages[d]) o.doff[pool_base + d] = atomicAdd(&tot[dbase + d], npages[d]);
+        if (npages[d]) o.doff[doff_at(kMode, g, F, pool_base) + d] = atomicAdd(&tot[dbase + d], npages[d]);
     if (tid == 0) {
         o.nlog[g] = misc[0];
         o.udesc[g] = make_uint2(dbase, F);
@@ -608,7 +614,7 @@ page_place(PassArgs a, uint32_t unit_pages, uint32_t *uoff0, uint32_t *uoff1) {
         const uint32_t v = tid < F ? a.totals[(size_t)relidx * F + tid] : 0u;
         uint32_t tot;
         const uint32_t ex = block_exclusive_scan(v, tmp, &tot);
-        if (tid < F) base[tid] = ex + o.doff[pool_base + tid];   // (doff of an absent digit is not used)
+        if (tid < F) base[tid] = ex + o.doff[doff_at(0, g, F, pool_base) + tid];   // (an absent digit's is not used)
         if (g == 0) {
             if (tid < F) o.pstart[tid] = ex;
             if (tid == 0) o.pstart[F] = tot;
@@ -622,7 +628,7 @@ page_place(PassArgs a, uint32_t unit_pages, uint32_t *uoff0, uint32_t *uoff1) {
     } else {
         if (!used) return;
         for (uint32_t d = tid; d < ud.y; d += kPlaceThreads)
-            base[d] = (uint32_t)o.pstart[ud.x + d] + o.doff[pool_base + d];
+            base[d] = (uint32_t)o.pstart[ud.x + d] + o.doff[doff_at(a.paged, g, ud.y, pool_base) + d];
     }
     __syncthreads();
     for (uint32_t k = tid; k < used; k += kPlaceThreads)

@@ -10,6 +10,8 @@
 //   join          radix_join_items: persistent, work-stealing build + probe
 // The fan-out 2^bits is chosen so an R partition fills about one CTA's
 // shared-memory table (8704 tuples).
+#include <algorithm>
+
 #include "joins.cuh"
 #include "paged.cuh"
 #include "radix_join.cuh"
@@ -30,18 +32,17 @@ namespace adb {
 //     2^25 854 / 867 (0.99, the one size where it was slower).  A first pass with
 //     a second to follow keeps two CTAs, one of which loads and stores while
 //     the other waits at a barrier (2^27 x 2^27: 0.953 ms, one CTA 1.033).
+// The smaller relation's share is rounded up: rounded down, its chunks, and with
+// them every CTA's page pool, would be up to 1.5 times the larger one's.
 static void flat_ctas(uint64_t nR, uint64_t nS, int num_sms, bool wide, int G[2]) {
     const uint64_t all = (uint64_t)num_sms * (wide ? 1 : kPassMinBlocks) * (nR + nS >= (1ull << 27) ? 2 : 1);
     const uint64_t n[2] = {nR, nS}, tile = wide ? kWideTile : kFlatTile;
-    uint64_t left = all;   // not more than all together: one CTA over would be a wave of its own
-    for (int r = 0; r < 2; r++) {
-        uint64_t g = r ? left : nR + nS ? (all * nR + (nR + nS) / 2) / (nR + nS) : 1;
-        if (!r && g >= all) g = all - 1;
-        const uint64_t tiles = (n[r] + tile - 1) / tile;
-        if (g > tiles) g = tiles;
-        G[r] = (int)(g < 1 ? 1 : g);
-        left -= G[r];
-    }
+    const int small = nS < nR;
+    auto at_most = [](uint64_t g, uint64_t a, uint64_t b) { return std::max<uint64_t>(1, std::min({g, a, b})); };
+    const uint64_t share = nR + nS ? (all * n[small] + nR + nS - 1) / (nR + nS) : 1;
+    const uint64_t gs = at_most(share, all - 1, (n[small] + tile - 1) / tile);
+    G[small] = (int)gs;   // not more than all together: one CTA over would be a wave of its own
+    G[!small] = (int)at_most(all - gs, all - gs, (n[!small] + tile - 1) / tile);
 }
 
 // Launches one partition pass (both relations: grid.y = relation).
@@ -59,33 +60,6 @@ static void launch_pass(const PassArgs &a, uint32_t F, int G, bool wide, cudaStr
             kPassThreads, kFlatTile);
 }
 
-// Fan-out bits: partitions of at most 2^13 tuples (one R chunk), and below that
-// size up to 2^8 partitions, down to 256 tuples each, so that the join's items
-// fill the SMs.  Device time of PRO / m-way, us, four of each key on both sides,
-// at these bits (and at 2^12 tuples a partition, or one bit less): 2^16 - / 53
-// (4 bits 72), 2^18 64 / 71 (6 bits 73 / 83), 2^20 102 / 110 (7 bits 108 / 118), 2^21 133 /
-// 167 (9 bits 166 / 186), 2^22 228 / 256 (8 bits 223 / 273), 2^23 - / 410 (9 bits 450).
-// The largest relations leave 32-bit slot numbers less room for partial pages:
-// within 2^23 tuples of the limit no partitions beyond one R chunk each, above
-// 3 x 2^30 tuples at most 2^14.
-int radix_bits_for(uint64_t nR, uint64_t nS, int requested) {
-    if (requested > 0) return requested > 15 ? 15 : requested;
-    const int full = (int)ceil_log2_u64((nR + 8191) / 8192), fill = (int)ceil_log2_u64((nR + 255) / 256);
-    const uint64_t larger = nR > nS ? nR : nS;
-    const int most = larger > 3ull << 30 ? 14 : 15;
-    int b = larger > (1ull << 32) - (1u << 23) ? 1 : fill > 8 ? 8 : fill;
-    if (full > b) b = full;
-    if (b < 1) b = 1;
-    if (b > most) b = most;
-    return b;
-}
-
-// m-way / m-pass: the fan-out joinconfig_t.PARTFANOUT asks for, rounded up to a
-// power of two (at most 2^15), else as above.
-int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout) {
-    return radix_bits_for(nR, nS, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0);
-}
-
 // ---------------------------------------------------------------------------
 // Paged partitioning front end
 // ---------------------------------------------------------------------------
@@ -93,11 +67,16 @@ struct PartPlan {
     int passes;
     bool wide;                 // pass 1 in 1024-thread CTAs
     uint32_t F1, F2, Fout;
-    int g1[2];                 // pass 1: CTAs of R, S
-    int G1, G2;                // CTAs per relation (pass 1: the larger of g1)
+    int g1[2], g2[2];          // CTAs of R, S in pass 1, and in pass 2 (bounds)
+    int G1, G2;                // the larger of the two
     uint32_t pool1, pool2;
     uint32_t unit_pages;       // pass-2 work unit
-    uint64_t pages1, pages2;   // pool pages per relation
+    uint64_t pages1[2], pages2[2];   // pool pages of R, S
+    const uint64_t *pages() const { return passes == 2 ? pages2 : pages1; }   // of the output
+    // slot numbers (page x 64 + place) are 32 bits
+    bool fits() const {
+        return std::max({pages1[0], pages1[1], pages2[0], pages2[1]}) * kPageTuples < (uint64_t)kNone;
+    }
 };
 
 static PartPlan plan_partition(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
@@ -108,47 +87,98 @@ static PartPlan plan_partition(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b
     p.Fout = p.F1 * p.F2;
     p.wide = !b2;
     flat_ctas(nR, nS, num_sms, p.wide, p.g1);
-    p.G1 = p.g1[0] > p.g1[1] ? p.g1[0] : p.g1[1];
-    const uint32_t a = flat_pool_cap(nR, p.g1[0], p.F1), b = flat_pool_cap(nS, p.g1[1], p.F1);
-    p.pool1 = a > b ? a : b;
-    p.pages1 = (uint64_t)p.G1 * p.pool1;
-    if (b2) {
-        // units from the tuples actually present (the pass-1 pool has slack)
-        const uint64_t pages_in = (nR + kPageTuples - 1) / kPageTuples + (nS + kPageTuples - 1) / kPageTuples;
-        p.unit_pages = unit_pages_for(pages_in, num_sms);
-        p.G2 = (int)((p.pages1 + p.unit_pages - 1) / p.unit_pages + p.F1);
-        p.pool2 = unit_pool_cap(p.F2, p.unit_pages);
-        p.pages2 = (uint64_t)p.G2 * p.pool2;
+    p.pool1 = std::max(flat_pool_cap(nR, p.g1[0], p.F1), flat_pool_cap(nS, p.g1[1], p.F1));
+    // units from the tuples actually present (the pass-1 pool has slack)
+    const uint64_t pages_in = (nR + kPageTuples - 1) / kPageTuples + (nS + kPageTuples - 1) / kPageTuples;
+    p.unit_pages = unit_pages_for(pages_in, num_sms);
+    p.pool2 = unit_pool_cap(p.F2, p.unit_pages);
+    for (int r = 0; r < 2; r++) {
+        p.pages1[r] = (uint64_t)p.g1[r] * p.pool1;
+        if (b2) {
+            p.g2[r] = (int)((p.pages1[r] + p.unit_pages - 1) / p.unit_pages + p.F1);
+            p.pages2[r] = (uint64_t)p.g2[r] * p.pool2;
+        }
     }
+    p.G1 = std::max(p.g1[0], p.g1[1]);
+    p.G2 = std::max(p.g2[0], p.g2[1]);
     return p;
 }
 
-uint64_t paged_final_pool_pages(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
-    const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
-    return p.passes == 2 ? p.pages2 : p.pages1;
+static void split_bits(int bits, uint32_t *b1, uint32_t *b2) {
+    // one pass up to 2^9 partitions; two passes of at most 2^8 each above
+    if (bits <= (int)kMaxPassBits) {
+        *b1 = bits;
+        *b2 = 0;
+    } else {
+        *b1 = bits / 2;
+        *b2 = bits - bits / 2;
+    }
 }
 
-static size_t pageset_bytes(uint64_t pages, uint32_t G) {
-    return Workspace::need(pages * kPageTuples, 8) + 3 * Workspace::need(pages, 4) + Workspace::need(pages, 1) +
-           Workspace::need(G, 4) + Workspace::need(G, 8);
+// Fan-out bits: partitions of at most 2^13 tuples (one R chunk), and below that
+// size up to 2^8 partitions, down to 256 tuples each, so that the join's items
+// fill the SMs.  Device time of PRO / m-way, us, four of each key on both sides,
+// at these bits (and at 2^12 tuples a partition, or one bit less): 2^16 - / 53
+// (4 bits 72), 2^18 64 / 71 (6 bits 73 / 83), 2^20 102 / 110 (7 bits 108 / 118), 2^21 133 /
+// 167 (9 bits 166 / 186), 2^22 228 / 256 (8 bits 223 / 273), 2^23 - / 410 (9 bits 450).
+// The largest relations leave 32-bit slot numbers less room for partial pages:
+// where 2^b partitions do not fit them there are fewer, down to four R chunks per
+// partition (2^13 partitions above 2^27 tuples).
+static int bits_that_fit(uint64_t nR, uint64_t nS, int b, int least, int num_sms) {
+    for (;; b--) {
+        uint32_t b1, b2;
+        split_bits(b, &b1, &b2);
+        if (b <= least || plan_partition(nR, nS, b1, b2, num_sms).fits()) return b;
+    }
 }
 
-size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
-    const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
-    size_t s = 2 * pageset_bytes(p.pages1, p.G1) + Workspace::need(2ull * (p.F1 + p.Fout) + 4, 4) +
-               Workspace::need(2ull * (p.F1 + 1), 8);
-    if (p.passes == 2)
-        s += 2 * pageset_bytes(p.pages2, p.G2) + Workspace::need(2ull * (p.Fout + 1), 8) +
-             2 * Workspace::need(p.F1 + 1, 4);
+static int partition_bits(uint64_t nR, uint64_t nS, int requested, int most, int num_sms) {
+    int b = requested, least = requested;
+    if (requested <= 0) {
+        const int full = (int)ceil_log2_u64((nR + 8191) / 8192), fill = (int)ceil_log2_u64((nR + 255) / 256);
+        least = full;
+        b = std::max(full, std::min(fill, 8));
+        most = 15;
+    }
+    b = std::max(1, std::min(b, most));
+    return bits_that_fit(nR, nS, b, std::max(1, std::min(least, 15) - 2), num_sms);
+}
+
+int radix_bits_for(uint64_t nR, uint64_t nS, int requested, int num_sms) {
+    return partition_bits(nR, nS, requested, 15, num_sms);
+}
+
+// m-way / m-pass: the fan-out joinconfig_t.PARTFANOUT asks for, rounded up to a
+// power of two (at most 2^15), else as above.
+int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout, int num_sms) {
+    return partition_bits(nR, nS, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0, 15, num_sms);
+}
+
+static size_t pageset_bytes(uint64_t pages, uint32_t G, uint32_t F) {
+    return Workspace::need(pages * kPageTuples, 8) + 2 * Workspace::need(pages, 4) + Workspace::need(pages, 1) +
+           Workspace::need(G, 4) + Workspace::need((uint64_t)G * F, 4) + Workspace::need(G, 8);
+}
+
+static size_t partition_bytes(const PartPlan &p) {
+    size_t s = Workspace::need(2ull * (p.F1 + p.Fout) + 4, 4) + Workspace::need(2ull * (p.F1 + 1), 8);
+    for (int r = 0; r < 2; r++) s += pageset_bytes(p.pages1[r], p.G1, p.F1);
+    if (p.passes == 2) {
+        s += Workspace::need(2ull * (p.Fout + 1), 8) + 2 * Workspace::need(p.F1 + 1, 4);
+        for (int r = 0; r < 2; r++) s += pageset_bytes(p.pages2[r], p.G2, p.F2);
+    }
     return s;
 }
 
-static void take_pageset(Context *ctx, PageSet &ps, uint64_t pages, int G) {
+size_t paged_partition_scratch(uint64_t nR, uint64_t nS, uint32_t b1, uint32_t b2, int num_sms) {
+    return partition_bytes(plan_partition(nR, nS, b1, b2, num_sms));
+}
+
+static void take_pageset(Context *ctx, PageSet &ps, uint64_t pages, int G, uint32_t F) {
     ps.pages = ctx->ws.take<uint64_t>(pages * kPageTuples);
     ps.log = ctx->ws.take<uint32_t>(pages);
     ps.pcount = ctx->ws.take<uint8_t>(pages);
     ps.nlog = ctx->ws.take<uint32_t>(G);
-    ps.doff = ctx->ws.take<uint32_t>(pages);
+    ps.doff = ctx->ws.take<uint32_t>((uint64_t)G * F);
     ps.udesc = ctx->ws.take<uint2>(G);
     ps.plist = ctx->ws.take<uint32_t>(pages);
 }
@@ -160,9 +190,9 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     cudaStream_t st = ctx->stream;
     const uint32_t b1 = ceil_log2_u64((uint64_t)d1.mask + 1), b2 = d2 ? ceil_log2_u64((uint64_t)d2->mask + 1) : 0;
     const PartPlan p = plan_partition(j.nR, j.nS, b1, b2, ctx->num_sms);
-    const uint64_t maxpages = p.passes == 2 ? p.pages2 : p.pages1;
-    if (p.pages1 * kPageTuples >= (uint64_t)kNone || maxpages * kPageTuples >= (uint64_t)kNone) {
-        set_error("relation too large for one partitioned join (%llu pool pages)", (unsigned long long)maxpages);
+    if (!p.fits()) {
+        set_error("relations too large for one partitioned join (%llu and %llu pool pages)",
+                  (unsigned long long)p.pages()[0], (unsigned long long)p.pages()[1]);
         return ADB_ERR_ARG;
     }
     int *err = reinterpret_cast<int *>(acc + 2);
@@ -173,7 +203,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
         a1.in[r].in = r ? j.S : j.R;
         a1.in[r].n = r ? j.nS : j.nR;
         a1.in[r].G = p.g1[r];
-        take_pageset(ctx, a1.out[r], p.pages1, p.G1);
+        take_pageset(ctx, a1.out[r], p.pages1[r], p.G1, p.F1);
     }
     a1.df = d1;
     a1.F1 = 1;
@@ -207,7 +237,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
         out->S = a1.out[1];
         out->Fout = p.F1;
         out->pstart = pstart1;
-        out->pool_pages = p.pages1;
+        out->pool_pages = p.pages1[0];
         return ADB_OK;
     }
 
@@ -220,7 +250,7 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
         in.plist = a1.out[r].plist;
         in.pstart = a1.out[r].pstart;
         in.uoff = r ? uoff1 : uoff0;
-        take_pageset(ctx, a2.out[r], p.pages2, p.G2);
+        take_pageset(ctx, a2.out[r], p.pages2[r], p.G2, p.F2);
     }
     a2.df = *d2;
     a2.F1 = p.F1;
@@ -244,19 +274,8 @@ int run_paged_partition(Context *ctx, const DevJoin &j, DigitFn d1, const DigitF
     out->S = a2.out[1];
     out->Fout = p.Fout;
     out->pstart = pstart2;
-    out->pool_pages = p.pages2;
+    out->pool_pages = p.pages2[0];
     return ADB_OK;
-}
-
-static void split_bits(int bits, uint32_t *b1, uint32_t *b2) {
-    // one pass up to 2^9 partitions; two passes of at most 2^7 each above
-    if (bits <= (int)kMaxPassBits) {
-        *b1 = bits;
-        *b2 = 0;
-    } else {
-        *b1 = bits / 2;
-        *b2 = bits - bits / 2;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -266,9 +285,7 @@ size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms) {
     uint32_t b1, b2;
     split_bits(bits, &b1, &b2);
     const PartPlan p = plan_partition(nR, nS, b1, b2, num_sms);
-    const uint64_t pagesR = p.passes == 2 ? p.pages2 : p.pages1;
-    const uint64_t F = p.Fout;
-    return paged_partition_scratch(nR, nS, b1, b2, num_sms) + WorkList::bytes(F, pagesR, kChunkW);
+    return partition_bytes(p) + WorkList::bytes(p.Fout, p.pages()[0], kChunkW);
 }
 
 int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned long long *acc) {

@@ -1,0 +1,83 @@
+"""The partitioned joins' device workspace: its size for relations of unlike
+sizes, and what a join does where it does not fit.  Free memory is read around
+a call and cut down by holding a buffer; counts and checksums are exact."""
+import pytest
+import torch
+
+import alliancedb_b200 as adb
+
+pytestmark = pytest.mark.gpu
+
+
+def free_bytes():
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.fixture
+def relations():
+    kept = []
+
+    def make(n_r, n_s, seed):
+        R = adb.gen_pk(n_r, seed)
+        S = adb.gen_fk(n_s, R, 0.0, seed + 1)
+        kept.extend([adb.DeviceBuffer.from_host(R), adb.DeviceBuffer.from_host(S)])
+        return R, S, kept[-2].ptr, kept[-1].ptr
+
+    torch.cuda.empty_cache()
+    adb.lib().adb_release_workspace()
+    yield make
+    for b in kept:
+        b.close()
+    adb.lib().adb_release_workspace()
+
+
+@pytest.mark.parametrize("algo", ["PRO", "m-way"])
+@pytest.mark.parametrize("n_r,n_s,passes", [
+    (4_500_000, 1 << 25, 2),      # a small R, whose partitions ask for two passes over S
+    (1 << 25, 20_011, 2),         # an S of less than one CTA's share
+    (20_011, 1 << 25, 1),
+    (1 << 24, 1 << 24, 2),
+])
+def test_each_relation_has_its_own_pages(oracle, relations, algo, n_r, n_s, passes):
+    R, S, dR, dS = relations(n_r, n_s, 61)
+    before = free_bytes()
+    got = adb.join_device(algo, dR, n_r, dS, n_s)
+    took = before - free_bytes()
+    assert (got.count, got.checksum) == oracle.pk_truth(R, S)
+    # per pass 8 bytes a tuple in pages, a quarter for partly filled ones and the lists,
+    # an eighth that the workspace allocates beyond its need; 64 MiB of fixed tables
+    assert took <= passes * 8 * (n_r + n_s) * 1.25 * 1.125 + (64 << 20)
+
+
+@pytest.mark.parametrize("algo,n_r,n_s,room", [
+    ("PRO", 4_500_000, 1 << 26, 900 << 20),       # two passes take 1.2 GB, one 0.6
+    ("PRH", 4_500_000, 1 << 26, 900 << 20),
+    ("m-way", 4_500_000, 1 << 26, 900 << 20),
+    ("NPO", 1 << 25, 1 << 25, 1000 << 20),        # pages 1.15 GB, the one table 0.8
+])
+def test_a_join_that_does_not_fit_takes_less(oracle, relations, algo, n_r, n_s, room):
+    R, S, dR, dS = relations(n_r, n_s, 63)
+    want = oracle.pk_truth(R, S)
+    usual = adb.join_device(algo, dR, n_r, dS, n_s)
+    assert (usual.count, usual.checksum) == want
+    adb.lib().adb_release_workspace()
+    hold = adb.DeviceBuffer(free_bytes() - room)
+    try:
+        got = adb.join_device(algo, dR, n_r, dS, n_s)
+    finally:
+        hold.close()
+    assert (got.count, got.checksum) == want
+    assert got.kernels < usual.kernels      # one pass instead of two, or NPO's build and probe
+
+
+def test_a_join_that_fits_in_no_form_is_refused(relations):
+    _, _, dR, dS = relations(1 << 24, 1 << 24, 65)
+    hold = adb.DeviceBuffer(free_bytes() - (64 << 20))
+    try:
+        for algo in ("PRO", "NPO", "m-way"):
+            with pytest.raises(adb.AdbError) as e:
+                adb.join_device(algo, dR, 1 << 24, dS, 1 << 24)
+            assert e.value.status == adb.ADB_ERR_OOM
+    finally:
+        hold.close()
+    assert adb.join_device("PRO", dR, 1 << 24, dS, 1 << 24).count == 1 << 24
