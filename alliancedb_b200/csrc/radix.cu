@@ -149,9 +149,9 @@ int radix_bits_for(uint64_t nR, uint64_t nS, int requested, int num_sms) {
 }
 
 // m-way / m-pass: the fan-out joinconfig_t.PARTFANOUT asks for, rounded up to a
-// power of two (at most 2^15), else as above.
+// power of two (at most 2^16, two passes of 2^8), else as above.
 int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout, int num_sms) {
-    return partition_bits(nR, nS, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0, 15, num_sms);
+    return partition_bits(nR, nS, part_fanout > 1 ? (int)ceil_log2_u64((uint64_t)part_fanout) : 0, 16, num_sms);
 }
 
 static size_t pageset_bytes(uint64_t pages, uint32_t G, uint32_t F) {

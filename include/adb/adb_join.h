@@ -79,7 +79,7 @@ typedef struct adb_join_params {
                                    regions its inputs are grouped by (up to 9); 0 = chosen (one table
                                    while it stays in L2, |R| up to about 2^22, else the partitioned
                                    join on hashed digits), < 0 = one table, no grouping */
-    int32_t part_fanout;        /* joinconfig_t.PARTFANOUT for m-way/m-pass; 0 = chosen */
+    int32_t part_fanout;        /* joinconfig_t.PARTFANOUT for m-way/m-pass, taken up to 2^16; 0 = chosen */
     int32_t materialize;        /* 1: also write <S-key, S-payload> per match (JOIN_RESULT_MATERIALIZE) */
     int32_t batch_tuples;       /* eager joins: arrival micro-batch in tuples per side; 0 = 1 ms of stream */
     uint64_t seed;              /* JBCR's random split of S */

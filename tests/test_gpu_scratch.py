@@ -81,3 +81,17 @@ def test_a_join_that_fits_in_no_form_is_refused(relations):
     finally:
         hold.close()
     assert adb.join_device("PRO", dR, 1 << 24, dS, 1 << 24).count == 1 << 24
+
+
+def test_a_fan_out_of_2_16_is_taken(oracle, relations):
+    """Results do not depend on the fan-out; the page set of 2^16 partitions is larger than that of 2^15."""
+    R, S, dR, dS = relations(1 << 20, 1 << 20, 67)
+    want = oracle.pk_truth(R, S)
+    took = []
+    for fanout in (1 << 15, 1 << 16, 1 << 20):
+        adb.lib().adb_release_workspace()
+        before = free_bytes()
+        got = adb.join_device("m-way", dR, 1 << 20, dS, 1 << 20, adb.default_params(part_fanout=fanout))
+        took.append(before - free_bytes())
+        assert (got.count, got.checksum) == want
+    assert took[0] < took[1] == took[2]
