@@ -331,7 +331,7 @@ static size_t scratch_for(const AlgoEntry *a, uint64_t nR, uint64_t nS, const ad
         case Family::RadixHist:
             return radix_scratch(nR, nS, radix_bits_for(nR, nS, p ? p->radix_bits : 0, num_sms), num_sms);
         case Family::Npo:
-            if (npo_partitioned(nR, nS, p ? p->radix_bits : 0))
+            if (npo_partitioned(nR, nS, p ? p->radix_bits : 0, num_sms))
                 return radix_scratch(nR, nS, radix_bits_for(nR, nS, 0, num_sms), num_sms);
             return npo_scratch(nR, nS, p ? p->radix_bits : 0, num_sms);
         case Family::SortMerge:
@@ -360,7 +360,7 @@ static int reserve_for(Context *ctx, const AlgoEntry *a, uint64_t nR, uint64_t n
     } else if (a->fam == Family::SortMerge) {
         alt->part_fanout = 1 << (sort_bits_for(nR, nS, alt->part_fanout, ctx->num_sms) - 1);
         if (alt->part_fanout < 2) return s;
-    } else if (a->fam == Family::Npo && npo_partitioned(nR, nS, alt->radix_bits)) {
+    } else if (a->fam == Family::Npo && npo_partitioned(nR, nS, alt->radix_bits, ctx->num_sms)) {
         alt->radix_bits = -1;
     } else {
         return s;
@@ -377,7 +377,7 @@ static int dispatch(Context *ctx, const AlgoEntry *a, const DevJoin &j, const ad
             return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, p ? p->radix_bits : 0, ctx->num_sms), PartJoin::Chain,
                              acc);
         case Family::Npo:
-            if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0))
+            if (npo_partitioned(j.nR, j.nS, p ? p->radix_bits : 0, ctx->num_sms))
                 return run_radix(ctx, j, radix_bits_for(j.nR, j.nS, 0, ctx->num_sms), PartJoin::HashedChain, acc);
             return run_npo(ctx, j, p ? p->radix_bits : 0, acc);
         case Family::SortMerge:

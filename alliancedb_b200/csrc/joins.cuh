@@ -44,13 +44,14 @@ int run_small(Context *ctx, const DevJoin &j);
 int radix_bits_for(uint64_t nR, uint64_t nS, int requested, int num_sms);
 int sort_bits_for(uint64_t nR, uint64_t nS, int part_fanout, int num_sms);   // joinconfig_t.PARTFANOUT, 0 = chosen
 size_t radix_scratch(uint64_t nR, uint64_t nS, int bits, int num_sms);
+bool radix_fits(uint64_t nR, uint64_t nS, int bits, int num_sms);   // the slot numbers' 32 bits
 // How a partition is joined: a chained table over digits of the key's low bits
 // or of its hash, or a counting sort (the sort-merge names).
 enum class PartJoin { Chain, HashedChain, Sorted };
 int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned long long *acc);
 
 // ---- NPO / NPO_st ----
-bool npo_partitioned(uint64_t nR, uint64_t nS, int requested);
+bool npo_partitioned(uint64_t nR, uint64_t nS, int requested, int num_sms);
 uint32_t npo_region_bits(uint64_t nR, int requested);
 size_t npo_scratch(uint64_t nR, uint64_t nS, int region_bits, int num_sms);
 int run_npo(Context *ctx, const DevJoin &j, int region_bits, unsigned long long *acc);

@@ -45,17 +45,19 @@ static uint32_t npo_log2(uint64_t nR) {
 //   2^24   x 2^24   1210 / 570
 // Up to 2^22 the table still wins against a larger S, whose two extra trips
 // through memory the partitioning would add.
+// Relations whose pages overrun the passes' 32-bit slot numbers take the table too.
 constexpr uint64_t kNpoTableMax = 7ull << 19;   // 3.67 M tuples, an 88 MB table
-bool npo_partitioned(uint64_t nR, uint64_t nS, int requested) {
+bool npo_partitioned(uint64_t nR, uint64_t nS, int requested, int num_sms) {
     return requested == 0 && nR > kNpoTableMax && !(nR <= 1ull << 22 && nS >= 2 * nR) &&
-           nR < 1ull << 31 && nS < 1ull << 31;   // the paged passes' slot numbers are 32 bits
+           radix_fits(nR, nS, radix_bits_for(nR, nS, 0, num_sms), num_sms);
 }
 
 // Table-region bits: requested > 0 forces that many, at most 2^9 regions (one
-// partition pass) of at least 16 slots (one L2 line); otherwise none.
+// partition pass) of at least 16 slots (one L2 line); otherwise, and for a table
+// of more slots than the 32-bit hash tells apart, none.
 uint32_t npo_region_bits(uint64_t nR, int requested) {
-    if (requested <= 0) return 0;
     const int l2 = (int)npo_log2(nR);
+    if (requested <= 0 || l2 > 32) return 0;
     int rb = requested;
     if (rb > (int)kMaxPassBits) rb = (int)kMaxPassBits;
     if (rb > l2 - 4) rb = l2 - 4;

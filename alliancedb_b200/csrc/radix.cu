@@ -115,6 +115,12 @@ static void split_bits(int bits, uint32_t *b1, uint32_t *b2) {
     }
 }
 
+bool radix_fits(uint64_t nR, uint64_t nS, int bits, int num_sms) {
+    uint32_t b1, b2;
+    split_bits(bits, &b1, &b2);
+    return plan_partition(nR, nS, b1, b2, num_sms).fits();
+}
+
 // Fan-out bits: partitions of at most 2^13 tuples (one R chunk), and below that
 // size up to 2^8 partitions, down to 256 tuples each, so that the join's items
 // fill the SMs.  Device time of PRO / m-way, us, four of each key on both sides,
@@ -124,14 +130,6 @@ static void split_bits(int bits, uint32_t *b1, uint32_t *b2) {
 // The largest relations leave 32-bit slot numbers less room for partial pages:
 // where 2^b partitions do not fit them there are fewer, down to four R chunks per
 // partition (2^13 partitions above 2^27 tuples).
-static int bits_that_fit(uint64_t nR, uint64_t nS, int b, int least, int num_sms) {
-    for (;; b--) {
-        uint32_t b1, b2;
-        split_bits(b, &b1, &b2);
-        if (b <= least || plan_partition(nR, nS, b1, b2, num_sms).fits()) return b;
-    }
-}
-
 static int partition_bits(uint64_t nR, uint64_t nS, int requested, int most, int num_sms) {
     int b = requested, least = requested;
     if (requested <= 0) {
@@ -141,7 +139,9 @@ static int partition_bits(uint64_t nR, uint64_t nS, int requested, int most, int
         most = 15;
     }
     b = std::max(1, std::min(b, most));
-    return bits_that_fit(nR, nS, b, std::max(1, std::min(least, 15) - 2), num_sms);
+    least = std::max(1, std::min(least, 15) - 2);
+    while (b > least && !radix_fits(nR, nS, b, num_sms)) b--;
+    return b;
 }
 
 int radix_bits_for(uint64_t nR, uint64_t nS, int requested, int num_sms) {

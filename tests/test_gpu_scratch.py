@@ -1,6 +1,7 @@
 """The partitioned joins' device workspace: its size for relations of unlike
 sizes, and what a join does where it does not fit.  Free memory is read around
 a call and cut down by holding a buffer; counts and checksums are exact."""
+import numpy as np
 import pytest
 import torch
 
@@ -95,3 +96,38 @@ def test_a_fan_out_of_2_16_is_taken(oracle, relations):
         took.append(before - free_bytes())
         assert (got.count, got.checksum) == want
     assert took[0] < took[1] == took[2]
+
+
+def fmix(z):
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    return z ^ (z >> np.uint64(31))
+
+
+@pytest.mark.parametrize("n_r", [1 << 31, (1 << 31) + 12345])
+def test_npo_of_2_31_build_tuples(relations, n_r):
+    """The largest build sides are partitioned like the others (the one table costs a random
+    DRAM access per tuple), and none is grouped into regions of more than 2^32 slots."""
+    n_s = 3_000_001
+    torch.cuda.empty_cache()
+    if free_bytes() < 130 << 30:
+        pytest.skip("needs 130 GB of free device memory")
+    bufs = [adb.DeviceBuffer(8 * n_r), adb.DeviceBuffer(8 * n_s), adb.DeviceBuffer(4 * n_s)]
+    dR, dS, dI = (b.ptr for b in bufs)
+    try:
+        adb._check(adb.lib().adb_gen_pk(dR, n_r, 71, 1))
+        adb._check(adb.lib().adb_gen_fk(dS, n_s, dR, n_r, 0.0, 72, dI, 1))
+        s = bufs[1].to_host(np.uint64, n_s)
+        i = bufs[2].to_host(np.uint32, n_s).astype(np.uint64)     # the R row each S row was drawn from
+        key, pay = s >> np.uint64(32), s & np.uint64(0xFFFFFFFF)
+        want = int(fmix((key << np.uint64(32) | i) ^ fmix(pay << np.uint64(32) | key)).sum(dtype=np.uint64))
+        got = adb.join_device("NPO", dR, n_r, dS, n_s)
+        assert (got.count, got.checksum) == (n_s, want) and got.kernels > 4
+        for bits in (-1, 3):
+            if bits > 0 and n_r == 1 << 31:
+                continue                                          # regions of 2^32 slots: as at any size
+            got = adb.join_device("NPO", dR, n_r, dS, n_s, adb.default_params(radix_bits=bits))
+            assert (got.count, got.checksum) == (n_s, want) and got.kernels == 2
+    finally:
+        for b in bufs:
+            b.close()
