@@ -40,15 +40,22 @@ static uint32_t npo_log2(uint64_t nR) {
 // bits, four of each key on both sides, and dense keys with theta 1:
 //   2^21.8 x 2^21.8  154 / 170    299 / 225    122 / 175
 //   2^22   x 2^22    184 / 190    346 / 253    148 / 199
-//   2^22   x 2^24    336 / 558    818 / 806    238 / 438
+//   2^22   x 2^24    351 / 406    828 / 553    253 / 396
 //   2^23   x 2^23    470 / 342    642 / 421    412 / 389
 //   2^24   x 2^24   1210 / 570
-// Up to 2^22 the table still wins against a larger S, whose two extra trips
-// through memory the partitioning would add.
+// A larger S makes two more trips through memory where it is partitioned, and its
+// hot keys' buckets stay in L1 where it is not, so against one the table goes on
+// further, but for repeated build keys, whose runs it walks:
+//   2^22.5 x 2^25.5  814 / 894   1926 / 1352   558 / 852
+//   2^22.7 x 2^25.7  969 / 1008  1958 / 1476   664 / 977
+//   2^22.7 x 2^27.7 2942 / 3385  6843 / 5164  1839 / 3147
+//   2^23   x 2^26   1239 / 1228  2336 / 1868  1020 / 1130
+// (S of eight times R is a foreign key's side, R's keys then being unique.)
 // Relations whose pages overrun the passes' 32-bit slot numbers take the table too.
 constexpr uint64_t kNpoTableMax = 7ull << 19;   // 3.67 M tuples, an 88 MB table
 bool npo_partitioned(uint64_t nR, uint64_t nS, int requested, int num_sms) {
     return requested == 0 && nR > kNpoTableMax && !(nR <= 1ull << 22 && nS >= 2 * nR) &&
+           !(nR <= 7ull << 20 && nS >= 8 * nR) &&
            radix_fits(nR, nS, radix_bits_for(nR, nS, 0, num_sms), num_sms);
 }
 
