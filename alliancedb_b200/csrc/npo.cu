@@ -12,7 +12,7 @@
 // With a forced region count (radix_bits > 0) the table is an open-addressing
 // array of 2^l2 slots cut into 2^rb regions: region g
 // holds the slots whose index has top bits g, i.e. the keys whose top rb bits
-// of key * kFibMul are g.  One paged partition pass (paged.cuh, hashed digit)
+// of key * kHashMul are g.  One paged partition pass (paged.cuh, hashed digit)
 // groups R and S by region, and build and probe walk the page lists in region
 // order, each warp taking a few adjacent pages at a time and every warp of the
 // grid sweeping the same stretch of the list.  At any time the grid inserts into
@@ -35,7 +35,7 @@ static uint32_t npo_log2(uint64_t nR) {
 }
 
 // Build sides whose table would not stay in L2 are joined by the partitioned
-// join, on digits of key * kFibMul (radix.cu): the same join without a random
+// join, on digits of key * kHashMul (radix.cu): the same join without a random
 // DRAM access per tuple.  Device time, us, table / partitioned, for keys over 32
 // bits, four of each key on both sides, and dense keys with theta 1:
 //   2^21.8 x 2^21.8  154 / 170    299 / 225    122 / 175

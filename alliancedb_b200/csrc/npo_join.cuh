@@ -23,8 +23,7 @@ namespace adb {
 constexpr uint64_t kEmpty = ~0ULL;
 
 __host__ __device__ __forceinline__ uint32_t npo_hash(uint32_t key, uint32_t log2n) {
-    // Fibonacci hashing: the top log2n bits of key * 2^32/phi
-    return log2n ? (uint32_t)((key * kFibMul) >> (32 - log2n)) : 0u;
+    return log2n ? (uint32_t)((key * kHashMul) >> (32 - log2n)) : 0u;
 }
 
 // Inserts tuple word w (not the empty marker) by linear probing from `slot`.
@@ -173,7 +172,7 @@ npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ ta
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += T) {
         const uint64_t w = ld_stream(R + i);
         if (w == kEmpty) { atomicAdd(sentinel_cnt, 1ull); continue; }
-        const uint32_t h = tkey(w) * kFibMul, st = h >> 5 & 3;
+        const uint32_t h = tkey(w) * kHashMul, st = h >> 5 & 3;
         uint32_t b = __umulhi(h, nb);
         if (cas(4ull * b + st, w)) continue;
         // the slot was taken: read the bucket for a free one, the next where there is none
@@ -244,7 +243,7 @@ npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restric
 #pragma unroll
         for (int u = 0; u < kProbeU; u++) {   // the buckets' loads, then the next tuples', before any is used
             s[u] = n[u];
-            b[u] = __umulhi(tkey(s[u]) * kFibMul, nb);
+            b[u] = __umulhi(tkey(s[u]) * kHashMul, nb);
             npo_ld_bucket(table + 4ull * b[u], v[u]);
         }
 #pragma unroll

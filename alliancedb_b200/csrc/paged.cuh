@@ -160,7 +160,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
 // still in L2.  Three barriers per tile (four above 32 digits); the next
 // tile's loads are in flight during D.  kMode: 0 flat input, 1 paged input
 // (pass 2), 2 segmented flat input (batched windows).  kHashed: the digit is
-// taken from key * kFibMul instead of the key.
+// taken from key * kHashMul instead of the key.
 //
 // Bound: shared-memory data wavefronts (about 23 per 32 tuples, the pipe 73 %
 // busy in pass 1 with 4096-tuple tiles) and, between them, the barriers around
@@ -210,7 +210,7 @@ partition_pass(PassArgs a) {
         }
     }
     const uint32_t F = df.mask + 1;
-    auto dig = [&](uint64_t w) { return df(kHashed ? tkey(w) * kFibMul : tkey(w)); };
+    auto dig = [&](uint64_t w) { return df(kHashed ? tkey(w) * kHashMul : tkey(w)); };
     uint64_t *stage = reinterpret_cast<uint64_t *>(smem);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + kTile);   // [2][F]
     uint16_t *toff = reinterpret_cast<uint16_t *>(cnt + 2 * F);   // 16 bits: half the banks' conflicts in C

@@ -293,7 +293,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
     cudaStream_t st = ctx->stream;
     uint32_t b1, b2;
     split_bits(bits, &b1, &b2);
-    // the key's low bits, or the high bits of key * kFibMul
+    // the key's low bits, or the high bits of key * kHashMul
     const DigitFn d1{hashed ? 32u - b1 : 0u, (1u << b1) - 1, hashed};
     const DigitFn d2{hashed ? 32u - b1 - b2 : b1, (1u << b2) - 1, hashed};
     PartOut po;

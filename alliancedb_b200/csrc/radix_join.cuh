@@ -225,7 +225,7 @@ struct ItemRec {
 // in flight ahead of the one it probes.
 //
 // The table: bucket heads indexed by the lnb key bits above the b bits the
-// partitioning consumed (kHashed: the lnb bits of key * kFibMul below the b
+// partitioning consumed (kHashed: the lnb bits of key * kHashMul below the b
 // highest), one head per R slot (up to 2^13), and chains through the tuples
 // themselves.  All keys of a bucket share their low b + lnb bits, so a linked
 // tuple's key holds the next slot of its chain there (its own slot: the end);
@@ -382,7 +382,7 @@ radix_join_items(JoinArgs a) {
         const uint32_t lnb = C.lnb, link = shift + lnb;
         const uint32_t bmask = (1u << lnb) - 1;
         const uint32_t lim = 1u << link, lmask = lim - 1;
-        auto hash = [&](uint64_t t) { return kHashed ? tkey(t) * kFibMul : tkey(t); };
+        auto hash = [&](uint64_t t) { return kHashed ? tkey(t) * kHashMul : tkey(t); };
         auto bucket = [&](uint32_t x) { return kHashed ? x >> (32 - link) & bmask : x >> shift & bmask; };
         auto linked = [&](uint32_t x, uint32_t next) {
             return kHashed ? next << (32 - link) | (x << link) >> link : (x & ~lmask) | next;

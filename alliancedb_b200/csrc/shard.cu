@@ -9,9 +9,11 @@
 // (alliancedb_b200/dist.py), so this file holds no communication code.
 //
 // The destination of a key is the high bits of a multiplicative hash,
-// part = (key * 0x9E3779B1 mod 2^32) * parts / 2^32, so it does not depend on
-// the low key bits that the local partitioned join splits on: the received
-// tuples spread over all of a rank's partitions.
+// part = (key * 0x9E3779B1 mod 2^32) * parts / 2^32 (kShardMul).  The local
+// joins split on low key bits (PRO and its kin) or on high bits of key * kHashMul
+// (NPO, the sort-merge names, small build sides), neither of which the
+// destination fixes: the received tuples spread over all of a rank's partitions
+// and buckets.
 //
 // Kernels (HBM-bound byte work): a per-block count of destinations over
 // contiguous chunks (read 8 B per tuple), one small scan, and a scatter that
@@ -34,9 +36,9 @@ constexpr uint32_t kMaxShardParts = 32;
 // at -Xptxas -O0 and with __umulhi, a masked index or global atomics.
 __host__ __device__ __forceinline__ uint32_t shard_of(uint32_t key, uint32_t parts) {
 #ifdef __CUDA_ARCH__
-    return __umulhi(key * 0x9E3779B1u, parts);
+    return __umulhi(key * kShardMul, parts);
 #else
-    return (uint32_t)(((uint64_t)(key * 0x9E3779B1u) * parts) >> 32);
+    return (uint32_t)(((uint64_t)(key * kShardMul) * parts) >> 32);
 #endif
 }
 

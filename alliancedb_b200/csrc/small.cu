@@ -8,7 +8,7 @@
 // every hash-join name (PRO, RJ_st, PRH, PRHO, NPO, NPO_st): their results are
 // the same join.
 //
-// The table is radix_join.cuh's, over hk = key * kFibMul instead of the key (a
+// The table is radix_join.cuh's, over hk = key * kHashMul instead of the key (a
 // bijection): bucket = the top lnb bits of hk, so that keys with equal low bits
 // spread; a linked tuple holds its chain's next slot (its own: the end) in
 // those bits and the rest of hk below them.
@@ -60,7 +60,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
         for (int j = 0; j < 4; j++) {
             const uint32_t k = i + j * kSmallThreads;
             if (k < nR) {
-                const uint32_t hk = tkey(r[j]) * kFibMul;
+                const uint32_t hk = tkey(r[j]) * kHashMul;
                 const uint32_t old = atomicExch(&heads[hk >> rest], k);
                 tup[k] = tword((old == kSmallNone ? k : old) << rest | (hk << lnb) >> lnb, tpay(r[j]));
             }
@@ -78,7 +78,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
 #pragma unroll
         for (int u = 0; u < kSmallU; u++) {
             if (i0 + 32 * u < e) {
-                const uint32_t key = tkey(s[u]), hk = key * kFibMul;
+                const uint32_t key = tkey(s[u]), hk = key * kHashMul;
                 uint32_t at = heads[hk >> rest];
                 if (at != kSmallNone) {
                     const uint64_t sh = s_half(key, tpay(s[u]));
