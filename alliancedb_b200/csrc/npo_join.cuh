@@ -172,7 +172,10 @@ npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ ta
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += T) {
         const uint64_t w = ld_stream(R + i);
         if (w == kEmpty) { atomicAdd(sentinel_cnt, 1ull); continue; }
-        const uint32_t h = tkey(w) * kHashMul, st = h >> 5 & 3;
+        // the bucket, and the quarter of its hash range that h lies in: evenly spread hashes
+        // (dense keys) then claim their slots without meeting (adb_npo_join_noalloc, 2^21 x
+        // 300,000 dense: 83 -> 79 us; bits of h below the bucket's would do for others)
+        const uint32_t h = tkey(w) * kHashMul, st = h * nb >> 30;
         uint32_t b = __umulhi(h, nb);
         if (cas(4ull * b + st, w)) continue;
         // the slot was taken: read the bucket for a free one, the next where there is none
