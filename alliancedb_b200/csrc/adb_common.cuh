@@ -90,6 +90,25 @@ __device__ __forceinline__ void block_flush(Acc a, unsigned long long *out, uint
     __syncthreads();
 }
 
+// c copies of row s (an S tuple with c matches) into the materialisation buffer of
+// cap rows; *n counts them all.  Every lane of the warp calls it, so that a warp's
+// rows take one atomic; one per match, or per group of lanes that find theirs in
+// the same step of their walks, was most of a materialising join's time.
+__device__ __forceinline__ void mat_rows(uint64_t *mat, uint64_t cap, unsigned long long *n, uint64_t s, uint32_t c) {
+    if (!__any_sync(0xffffffffu, c)) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    unsigned long long at = 0;
+    if (lane == 31) at = atomicAdd(n, (unsigned long long)inc);
+    at = __shfl_sync(0xffffffffu, at, 31) + (inc - c);
+    for (; c && at < cap; c--, at++) mat[at] = s;
+}
+
 // Loads of words that other CTAs of the same launch wrote, after a ticket showed
 // that they are done: from L2, and not moved ahead of the ticket (volatile).
 __device__ __forceinline__ ulonglong2 ld_done(const ulonglong2 *p) {

@@ -476,10 +476,6 @@ radix_join_items(JoinArgs a) {
                 auto add = [&](uint64_t r) {
                     acc.sum += pair_hash_pre(key, tpay(r), sh);
                     matches++;
-                    if (kMat) {
-                        const unsigned long long m = atomicAdd(a.mat_n, 1ull);
-                        if (m < a.mat_cap) a.mat[m] = s;
-                    }
                 };
                 if (kSorted) {
                     uint32_t n = at & 0xFFFFu;
@@ -502,10 +498,16 @@ radix_join_items(JoinArgs a) {
                 const uint32_t n = n0;
                 n0 = 0;
                 if (i + 1 < npw) load_page(i + 1, x0, n0);
+                const uint32_t m0 = matches;
                 if (2 * lane < (int)n) probe(c.x);
                 __syncwarp();
+                const uint32_t m1 = matches;
                 if (2 * lane + 1 < (int)n) probe(c.y);
                 __syncwarp();
+                if (kMat) {
+                    mat_rows(a.mat, a.mat_cap, a.mat_n, c.x, m1 - m0);
+                    mat_rows(a.mat, a.mat_cap, a.mat_n, c.y, matches - m1);
+                }
             }
             acc.count += matches;
             my_pg = nx_pg;

@@ -77,6 +77,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
             n[u] = i1 + 32 * u < e ? __ldcs(reinterpret_cast<const unsigned long long *>(S) + i1 + 32 * u) : 0ULL;
 #pragma unroll
         for (int u = 0; u < kSmallU; u++) {
+            uint32_t rows = 0;
             if (i0 + 32 * u < e) {
                 const uint32_t key = tkey(s[u]), hk = key * kHashMul;
                 uint32_t at = heads[hk >> rest];
@@ -87,10 +88,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
                         if ((tkey(r) ^ hk) << lnb == 0) {
                             a.count++;
                             a.sum += pair_hash_pre(key, tpay(r), sh);
-                            if (kMat) {
-                                const unsigned long long m = atomicAdd(acc + 3, 1ull);
-                                if (m < mat_cap) mat[m] = s[u];
-                            }
+                            if (kMat) rows++;
                         }
                         const uint32_t nx = tkey(r) >> rest;
                         if (nx == at) break;
@@ -99,6 +97,7 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
                 }
             }
             __syncwarp();
+            if (kMat) mat_rows(mat, mat_cap, acc + 3, s[u], rows);
         }
 #pragma unroll
         for (int u = 0; u < kSmallU; u++) s[u] = n[u];
