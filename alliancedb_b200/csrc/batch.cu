@@ -246,7 +246,7 @@ int batch_launch(Context *ctx, const uint64_t *dR, const uint64_t *r_off, const 
     uint64_t *bsum64 = ctx->ws.take<uint64_t>(nbs);
     uint32_t *bsum32 = reinterpret_cast<uint32_t *>(bsum64);   // the scans run one after the other
     WorkList wl;
-    wl.take(ctx->ws, Dt, pages, kChunkW);
+    wl.take(ctx->ws, Dt, pages, kChunkW, ctx->num_sms);
 
     ADB_CK(cudaMemsetAsync(wacc, 0, (2 * W + 8) * 8, st));
     ADB_CK(cudaMemsetAsync(tot, 0, 2ull * Dt * 4, st));

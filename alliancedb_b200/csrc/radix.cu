@@ -303,7 +303,7 @@ int run_radix(Context *ctx, const DevJoin &j, int bits, PartJoin kind, unsigned 
 
     const uint32_t F = po.Fout;
     WorkList wl;
-    wl.take(ctx->ws, F, po.pool_pages, kChunkW, ctr);
+    wl.take(ctx->ws, F, po.pool_pages, kChunkW, ctx->num_sms, ctr);
     ctx->kernels += make_work_list(st, po.pstart, po.R.plist, po.R.pcount, F, wl);
     ADB_CK(cudaGetLastError());
     ADB_CK(mark(ctx, 3));

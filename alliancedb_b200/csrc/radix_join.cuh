@@ -43,28 +43,52 @@ __device__ __forceinline__ uint32_t page_weight(uint32_t cnt) {
 // cstart[chunk_off[p]], +1, .. (page-list indexes), rch[p] of them.
 struct WorkList {
     uint32_t *rch, *chunk_off, *items, *items_off;   // [F], [F], [F], [F + 1]
+    uint32_t *spp;                                   // [F] pages per S chunk
     uint64_t *cstart;
+    uint32_t ctas;                                   // CTAs of the join
     uint32_t *ctr;                                   // items, work counter, blocks done (zeroed before part_chunks)
     // A partition's chunks weigh more than chunk_w but for the last, so at
     // most 64 x pages / chunk_w + 1 of them: chunk_off needs no scan.
     static size_t chunks(uint64_t F, uint64_t pages, uint32_t chunk_w) { return pages * kPageTuples / chunk_w + F + 1; }
     static size_t bytes(uint64_t F, uint64_t pages, uint32_t chunk_w) {
-        return 3 * Workspace::need(F, 4) + Workspace::need(F + 1, 4) + Workspace::need(chunks(F, pages, chunk_w), 8) +
+        return 4 * Workspace::need(F, 4) + Workspace::need(F + 1, 4) + Workspace::need(chunks(F, pages, chunk_w), 8) +
                Workspace::need(3, 4);
     }
-    void take(Workspace &ws, uint64_t F, uint64_t pages, uint32_t chunk_w, uint32_t *counters = nullptr) {
+    void take(Workspace &ws, uint64_t F, uint64_t pages, uint32_t chunk_w, int num_sms, uint32_t *counters = nullptr) {
+        ctas = (uint32_t)(num_sms * kJoinMinBlocks);
         rch = ws.take<uint32_t>(F);
         chunk_off = ws.take<uint32_t>(F);
         items = ws.take<uint32_t>(F);
+        spp = ws.take<uint32_t>(F);
         items_off = ws.take<uint32_t>(F + 1);
         cstart = ws.take<uint64_t>(chunks(F, pages, chunk_w));
         ctr = counters ? counters : ws.take<uint32_t>(3);
     }
 };
 
+// Pages per S chunk of a partition with nsp of all the S pages in F partitions, and
+// rch R chunks: up to kSPages, but where the partition has more than twice the
+// mean, no more than makes a CTA's share of the join's items.  A few hot keys on
+// both sides would else be a few items, each with all the pairs of a key, while the
+// other CTAs have none.  300,007 x 300,007 tuples, 4,096 / 16,384 of each key, ms:
+// sorted 8.4 / 58.7 -> 4.2 / 8.3, chained 9.9 / 70 -> 5.0 / 9.8.  (From 1.25 times the
+// mean on: 2^20 x 2^22, theta 1, 0.149 -> 0.166, its items no longer one wave of CTAs.)
+__device__ __forceinline__ uint32_t s_chunk_pages(uint32_t nsp, uint32_t rch, uint32_t all, uint32_t F, uint32_t ctas) {
+    if ((uint64_t)nsp * F <= 2ull * all) return kSPages;
+    const uint32_t share = (min(all / ctas, kSPages) + 1) * min(rch, kSPages);
+    const uint32_t most = max(max(share, 2 * (all / F)), (uint32_t)kProbeWarps + 1);
+    if (most >= kSPages || nsp <= most) return kSPages;
+    const uint32_t chunks = (nsp + most - 1) / most, per = (nsp + chunks - 1) / chunks;   // of like size
+    return per <= 4 * kProbeWarps ? per : (per + kProbeWarps - 1) / kProbeWarps * kProbeWarps;
+}
+
+__device__ __forceinline__ uint32_t s_chunks(uint32_t nsp, uint32_t per) {
+    return per == kSPages ? (nsp + kSPages - 1) / kSPages : (nsp + per - 1) / per;   // (the usual divisor is a constant)
+}
+
 // R chunks and item counts, one warp per partition: chunk c of a partition
 // starts at the first page whose preceding weight reaches c * kChunkW (greedy
-// by page weight); S chunks are kSPages pages each.  With `scan` (F <= 1024) the
+// by page weight); S chunks are spp[p] pages each.  With `scan` (F <= 1024) the
 // last block to finish also makes items_off and the item count, so that one
 // launch stands between the passes and the join.
 static __global__ void __launch_bounds__(1024)
@@ -75,6 +99,7 @@ part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount
     if (p < F) {
         const uint64_t *pS = pstart + (F + 1);
         const uint64_t r0 = pstart[p], r1 = pstart[p + 1];
+        const uint32_t nsp = (uint32_t)(pS[p + 1] - pS[p]), all = (uint32_t)pS[F];
         const uint64_t cid = r0 * kPageTuples / kChunkW + p;
         uint64_t carry = 0;                 // weight before this round
         uint32_t prev_chunk = 0xFFFFFFFFu;  // chunk of the page before this round
@@ -101,8 +126,10 @@ part_chunks(const uint64_t *pstart, const uint32_t *Rlist, const uint8_t *Rcount
         }
         if (lane == 0) {
             const uint32_t rc = r1 > r0 ? prev_chunk + 1 : 0u;
-            const uint32_t sc = (uint32_t)((pS[p + 1] - pS[p] + kSPages - 1) / kSPages);
+            const uint32_t per = s_chunk_pages(nsp, rc, all, F, wl.ctas);
+            const uint32_t sc = s_chunks(nsp, per);
             wl.rch[p] = rc;
+            wl.spp[p] = per;
             wl.chunk_off[p] = (uint32_t)cid;
             wl.items[p] = rc * sc;
         }
@@ -158,12 +185,12 @@ struct ItemGeo {
 };
 
 template <typename Args>
-__device__ __forceinline__ ItemGeo item_geo(const Args &a, uint32_t item, uint32_t p, uint32_t s_pages) {
+__device__ __forceinline__ ItemGeo item_geo(const Args &a, uint32_t item, uint32_t p) {
     const uint64_t *pR = a.pstart, *pS = a.pstart + (a.F + 1);
     const uint64_t r0 = pR[p], nrp = pR[p + 1] - r0;
     const uint64_t s0 = pS[p], nsp = pS[p + 1] - s0;
-    const uint32_t sch = (uint32_t)((nsp + s_pages - 1) / s_pages);
-    const uint32_t local = item - a.wl.items_off[p], rch = a.wl.rch[p];
+    const uint32_t local = item - a.wl.items_off[p], rch = a.wl.rch[p], s_pages = a.wl.spp[p];
+    const uint32_t sch = s_chunks((uint32_t)nsp, s_pages);
     const uint32_t rc = local / sch, sc = local % sch;
     const uint32_t cid = a.wl.chunk_off[p] + rc;
     ItemGeo g;
@@ -279,7 +306,7 @@ radix_join_items(JoinArgs a) {
         if (lane == 0) {
             r->item = item;
             if (item < n_items) {
-                const ItemGeo g = item_geo(a, item, p, kSPages);
+                const ItemGeo g = item_geo(a, item, p);
                 r->p = p;
                 r->win = w;
                 r->shift = a.wacc ? a.wbits[w] : a.bits;
