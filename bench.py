@@ -50,21 +50,42 @@ sys.path.insert(0, str(ROOT))
 # algorithmic bytes per input tuple of each family (whole pipeline)
 ALG_BYTES = {"PRO": 24, "RJ_st": 24, "PRH": 24, "PRHO": 24, "NPO": 16, "NPO_st": 16,
              "m-way": 24, "m-pass": 24, "m-way+skew": 24}
-# Per family: phase index (adb_join_result.ms_phase) -> (kernel, algorithmic
-# bytes per input tuple of one launch, DRAM bytes per input tuple of one launch
-# from an ncu capture of dram__bytes_read.sum + dram__bytes_write.sum at
+# Per route of a join (route_of): phase index (adb_join_result.ms_phase) -> (kernel,
+# algorithmic bytes per input tuple of one launch, DRAM bytes per input tuple of one
+# launch from an ncu capture of dram__bytes_read.sum + dram__bytes_write.sum at
 # |R| = |S| = 2^24; None where not captured).  The traffic of a full-size
 # launch is that figure times the launch's tuples: the kernels stream every
 # tuple once, so traffic grows in proportion.
 KERNELS = {
+    "small": {3: ("small_join", 8, None)},
+    "table": {1: ("npo_build", 8, None), 3: ("npo_probe", 8, None)},
+    "regions": {0: ("partition_pass<0,1024,8192,hashed>", 16, None), 1: ("npo_build_pages", 8, None),
+                3: ("npo_probe_pages", 8, None)},
     "radix": {0: ("partition_pass<0,512,6144> (pass 1)", 16, (269430016 + 214572288) / 2**25),
               1: ("partition_pass<1,512,8192> (pass 2)", 16, (274856704 + 217763840) / 2**25),
               3: ("radix_join_items", 8, (281964544 + 3466752) / 2**25)},
-    "npo": {1: ("npo_build", 8, None), 3: ("npo_probe", 8, None)},
-    "smj": {0: ("partition_pass<0,512,6144,hashed> (pass 1)", 16, None),
-            1: ("partition_pass<1,512,8192,hashed> (pass 2)", 16, None),
-            3: ("radix_join_items<sorted>", 8, (282349568 + 3129088) / 2**25)},
+    "radix, one pass": {0: ("partition_pass<0,1024,8192>", 16, None), 3: ("radix_join_items", 8, None)},
+    "hashed": {0: ("partition_pass<0,512,6144,hashed> (pass 1)", 16, None),
+               1: ("partition_pass<1,512,8192,hashed> (pass 2)", 16, None),
+               3: ("radix_join_items<hashed>", 8, None)},
+    "hashed, one pass": {0: ("partition_pass<0,1024,8192,hashed>", 16, None), 3: ("radix_join_items<hashed>", 8, None)},
+    "sorted": {0: ("partition_pass<0,512,6144,hashed> (pass 1)", 16, None),
+               1: ("partition_pass<1,512,8192,hashed> (pass 2)", 16, None),
+               3: ("radix_join_items<sorted>", 8, (282349568 + 3129088) / 2**25)},
+    "sorted, one pass": {0: ("partition_pass<0,1024,8192,hashed>", 16, None), 3: ("radix_join_items<sorted>", 8, None)},
 }
+
+
+def route_of(algo, kernels, phases):
+    """Which of KERNELS a join took, from the launches and phases it reported:
+    one launch is the small join; NPO's table takes two and, grouped by region,
+    four; the partitioned joins take four with one pass, whose second phase is 0."""
+    if kernels == 1:
+        return "small"
+    if algo.startswith("NPO") and kernels <= 4 and phases[1] > 0:
+        return "table" if kernels == 2 else "regions"
+    name = "sorted" if algo.startswith("m-") else "hashed" if algo.startswith("NPO") else "radix"
+    return name if phases[1] > 0 else name + ", one pass"
 
 
 def peaks():
@@ -494,11 +515,9 @@ def main():
     e2e_value = 2 * n * world / (e2e_ms / 1e3)
 
     # ---- roofline of the dominant kernel
-    # (NPO is the partitioned join on hashed digits once its table outgrows L2, |R| > 3.67 M)
-    fam = ("npo" if args.algo.startswith("NPO") and n <= 7 << 19 else "smj" if args.algo.startswith("m-")
-           else "radix")
     ph = np.array(phases).mean(axis=0)
-    cands = KERNELS[fam]
+    route = route_of(args.algo, kernels_per_step, ph)
+    cands = KERNELS[route]
     dom = max(cands, key=lambda k: ph[k])
     kname, alg_per_tuple, traffic_per_tuple = cands[dom]
     hbm, peak_kind = peaks()
@@ -527,7 +546,7 @@ def main():
         **({"random_access": {
             "note": "NPO's table (3 slots per R tuple) stays in L2: the inserts (one compare-and-swap each) and the "
                     "probes (one 32-byte bucket each) are bound by its random access rate",
-            "build_cas_per_s": n / (ph[1] / 1e3), "probes_per_s": n / (ph[3] / 1e3)}} if fam == "npo" else {}),
+            "build_cas_per_s": n / (ph[1] / 1e3), "probes_per_s": n / (ph[3] / 1e3)}} if route == "table" else {}),
         "gpu_launches": kernels_per_step * args.steps,
         "clocks": clk.summary(),
         "result": {"count": total[0], "checksum": hex(total[1]), "over_ranks": world,
