@@ -31,7 +31,6 @@ constexpr uint32_t kScanBlock = 8192;         // elements per block of the devic
 // ---- device-wide exclusive scan (reduce, scan of block sums, apply) --------
 template <class T>
 __global__ void dscan_reduce(const uint32_t *in, uint32_t n, T *bsum) {
-    __shared__ uint32_t tmp[32];
     const uint64_t b = (uint64_t)blockIdx.x * kScanBlock;
     T loc = 0;
     for (uint32_t i = threadIdx.x; i < kScanBlock; i += blockDim.x)
@@ -46,7 +45,6 @@ __global__ void dscan_reduce(const uint32_t *in, uint32_t n, T *bsum) {
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += part[w];
         bsum[blockIdx.x] = s;
     }
-    (void)tmp;
 }
 
 template <class T>

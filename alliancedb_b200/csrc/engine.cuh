@@ -95,7 +95,6 @@ struct Context {
     cudaEvent_t copy_ev[kCopyWorkers][2] = {};
     cudaEvent_t copy_start = nullptr, copy_done = nullptr;
     unsigned char *h_copy = nullptr;       // kCopyWorkers x 2 x kCopyChunk
-    bool attrs_set = false;
     int kernels = 0;                       // kernels launched by the current call
     std::recursive_mutex mu;               // held by the call that uses this context
 };

@@ -23,10 +23,6 @@ struct DevJoin {
     int test_flags = 0;           // adb_join_params.test_flags
 };
 
-struct JoinTimes {
-    float ms[4] = {0, 0, 0, 0};
-};
-
 enum class Family { Radix, RadixHist, Npo, SortMerge, Shj, Pmj, Unsupported };
 
 // ---- paged partitioning front end (radix and sort-merge joins), paged.cuh ----

@@ -20,7 +20,7 @@
 // the build each page of region g also prefetches its share of region g + 1's
 // table lines into L2, so the next region arrives by line reads instead of
 // random sector misses.  At |R| = |S| = 2^27 with 7 bits: 4.26 ms (grouping 1.06,
-// build 1.95, probe 1.19) against 10.9 ms in input order and 3.2 ms partitioned.
+// build 1.95, probe 1.19) against 10.9 ms in input order and 2.98 ms partitioned.
 // Matches, count and checksum are the same as in input order.
 #include "joins.cuh"
 #include "npo_join.cuh"

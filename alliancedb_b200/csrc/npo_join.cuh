@@ -4,11 +4,12 @@
 // np_distribute, NPO) and its table code in hashing/joins/common_functions.cpp
 // (allocate_hashtable :75-102, build_hashtable_mt :350-400, probe_hashtable
 // :221-280).  The reference chains 32-byte buckets of two tuples behind
-// per-bucket latches; on the GPU the table is an open-addressing array of
-// 8-byte tuple slots (the tuple word itself is the slot content), claimed with
-// one 64-bit atomicCAS, probed linearly from a four-slot window.
-// With 2 slots per build tuple (load <= 0.5) a probe touches one or two
-// sectors; a table of up to ~60 MB stays resident in the 126 MB L2.
+// per-bucket latches; on the GPU a slot is 8 bytes, the tuple word itself,
+// claimed with one 64-bit atomicCAS.  Two forms: buckets of four slots, three slots
+// per build tuple (npo_build, npo_probe: NPO by default while the table stays in
+// the 126 MB L2, and adb_npo_join_noalloc), and an open-addressing array of 2^l2
+// slots, load <= 0.5, probed linearly from a four-slot window (by table region,
+// npo.cu, where the caller asks for regions).
 //
 // The empty marker is the all-ones word.  A build tuple equal to it (key and
 // payload both 0xFFFFFFFF) is counted on the side instead of stored, and
@@ -159,8 +160,6 @@ __device__ __forceinline__ void npo_ld_bucket(const uint64_t *p, uint64_t (&v)[4
                  : "l"(p));
 }
 
-constexpr int kProbeU = 1;      // probe: tuples per lane in flight
-
 static __global__ void __launch_bounds__(256)
 npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ table, uint32_t nb,
           unsigned long long *sentinel_cnt, int *err) {
@@ -195,7 +194,8 @@ npo_build(const uint64_t *__restrict__ R, uint64_t nR, uint64_t *__restrict__ ta
             } else {
                 b = b + 1 == nb ? 0 : b + 1;
             }
-            if (tries > 8ull * nb) { atomicExch(err, kErrTableFull); break; }   // table full: cannot happen at load <= 0.5
+            // cannot happen: a third of the slots is used, of the fixed table's at most half
+            if (tries > 8ull * nb) { atomicExch(err, kErrTableFull); break; }
         }
     }
 }
@@ -235,49 +235,28 @@ npo_probe(const uint64_t *__restrict__ S, uint64_t nS, const uint64_t *__restric
     const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t nsent = *sentinel_cnt;
     NpoSink<kMaterialize> sink{Acc(), mat, mat_n, mat_cap};
-    uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t n[kProbeU];
-#pragma unroll
-    for (int u = 0; u < kProbeU; u++) n[u] = i0 + u * T < nS ? ld_stream(S + i0 + u * T) : 0ULL;
-    for (; i0 < nS; i0 += kProbeU * T) {
-        uint64_t s[kProbeU], v[kProbeU][4], sh[kProbeU];
-        uint32_t b[kProbeU], pay[kProbeU];
-        bool found[kProbeU];
-#pragma unroll
-        for (int u = 0; u < kProbeU; u++) {   // the buckets' loads, then the next tuples', before any is used
-            s[u] = n[u];
-            b[u] = __umulhi(tkey(s[u]) * kHashMul, nb);
-            npo_ld_bucket(table + 4ull * b[u], v[u]);
+    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint64_t n = i < nS ? ld_stream(S + i) : 0ULL;
+    for (; i < nS; i += T) {
+        const uint64_t s = n;
+        uint32_t b = __umulhi(tkey(s) * kHashMul, nb);
+        uint64_t v[4];
+        npo_ld_bucket(table + 4ull * b, v);
+        n = i + T < nS ? ld_stream(S + i + T) : 0ULL;   // in flight with the bucket
+        const uint64_t sh = s_half(tkey(s), tpay(s));
+        bool found = false;
+        uint32_t pay = 0;
+        bool more = npo_scan(sink, s, sh, v, found, pay);
+        for (uint32_t t = 1; more && t < nb; t++) {
+            b = b + 1 == nb ? 0 : b + 1;
+            uint64_t x[4];
+            npo_ld_bucket(table + 4ull * b, x);
+            more = npo_scan(sink, s, sh, x, found, pay);
         }
-#pragma unroll
-        for (int u = 0; u < kProbeU; u++) {
-            const uint64_t k = i0 + (kProbeU + u) * T;
-            n[u] = k < nS ? ld_stream(S + k) : 0ULL;
-        }
-#pragma unroll
-        for (int u = 0; u < kProbeU; u++) {
-            sh[u] = s_half(tkey(s[u]), tpay(s[u]));
-            found[u] = false;
-            pay[u] = 0;
-        }
-#pragma unroll
-        for (int u = 0; u < kProbeU; u++) {
-            if (i0 + u * T < nS) {
-                bool more = npo_scan(sink, s[u], sh[u], v[u], found[u], pay[u]);
-                for (uint32_t t = 1; more && t < nb; t++) {
-                    b[u] = b[u] + 1 == nb ? 0 : b[u] + 1;
-                    uint64_t x[4];
-                    npo_ld_bucket(table + 4ull * b[u], x);
-                    more = npo_scan(sink, s[u], sh[u], x, found[u], pay[u]);
-                }
-                if (tkey(s[u]) == 0xFFFFFFFFu && nsent) npo_add_sentinels(sink, s[u], nsent);
-            }
-        }
+        if (tkey(s) == 0xFFFFFFFFu && nsent) npo_add_sentinels(sink, s, nsent);
         // the lanes of a warp find their matches in different buckets; the
         // checksum then runs once for all of them
-#pragma unroll
-        for (int u = 0; u < kProbeU; u++)
-            if (found[u]) sink.match(s[u], tkey(s[u]), pay[u], sh[u]);
+        if (found) sink.match(s, tkey(s), pay, sh);
     }
     block_flush(sink.a, acc, red);
     if (out && threadIdx.x == 0) finish_call(acc, out);

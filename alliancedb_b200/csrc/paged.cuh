@@ -398,7 +398,9 @@ partition_pass(PassArgs a) {
             return L > room ? (L - room + kPageTuples - 1) / kPageTuples : 0u;
         };
         if (F <= 32) {
-            constexpr int kQ = 1;   // digits per lane
+            // (one digit per lane; without the loops ptxas schedules the paged pass of
+            // 2^7 digits, which does not come here, 2.7 % slower: 1.040 -> 1.068 ms)
+            constexpr int kQ = 1;
             const uint32_t q = (F + 31) / 32;
             if (tid < 32) {
                 uint32_t Ls[kQ], Ps[kQ], sumL = 0, sumN = 0;
@@ -457,9 +459,9 @@ partition_pass(PassArgs a) {
             __syncthreads();   // every B warp has read misc[0] and written its total
             if (bw < (int)nbw) {
                 // totals of the warps before this one, and of all of them: by a
-                // shuffle scan, or where four warps are usual one by one (2^22 x
-                // 2^22, 16 warps: pass 1 58.6 -> 56.3 us; 512 batched windows 5.275 ->
-                // 5.255 ms; 2^27 x 2^27, four warps: pass 2 1.038 -> 1.057 ms)
+                // shuffle scan, in the paged pass one by one (2^22 x 2^22, 16 warps:
+                // pass 1 58.6 -> 56.3 us; 512 batched windows 5.275 -> 5.255 ms; 2^27 x
+                // 2^27, four warps: pass 1 0.926 either way, pass 2 1.038 -> 1.057 ms)
                 uint32_t before_t = 0, before_p = 0, all_t = 0, all_p = 0;
                 if (!kPaged) {
                     const uint32_t tv = lane < (int)nbw ? misc[8 + lane] : 0u;
@@ -538,15 +540,11 @@ partition_pass(PassArgs a) {
         // its B / C run after the next barrier, when every thread is past D
     }
     __syncthreads();
-    // E. fill of each digit's last page; an odd fill gets the all-ones word in
-    //    its next slot, so that a 16-byte multiple copy of the page carries a
-    //    pad that sorts last (every other page of a stream is full)
+    // E. fill of each digit's last page (every other page of a stream is full); a
+    //    page's readers take tuples two at a time and leave out what is past its count
     for (uint32_t d = tid; d < F; d += kThreads) {
         const uint32_t p = npos[d];
-        if (p != kNone && (p & (kPageTuples - 1))) {
-            o.pcount[p / kPageTuples] = (uint8_t)(p & (kPageTuples - 1));
-            if (p & 1) o.pages[p] = ~0ULL;
-        }
+        if (p != kNone && (p & (kPageTuples - 1))) o.pcount[p / kPageTuples] = (uint8_t)(p & (kPageTuples - 1));
     }
     // F. pages per digit of this CTA
     uint32_t *tot = a.totals + (size_t)relidx * a.Dtot;

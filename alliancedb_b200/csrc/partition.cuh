@@ -2,10 +2,10 @@
 // partitioned joins (paged.cuh does the partitioning itself).
 // The digit is (key >> shift) & (F - 1): the low-bit radix of PRO
 // (HASH_BIT_MODULO, hashing/joins/parallel_radix_join.cpp:68), shift = the bits
-// an earlier pass consumed.  The sort-merge joins partition on the same low
-// bits (equal keys still meet in one partition; the reference's range split of
-// the high bits, sorting/joins/sortmergejoin_multiway.cpp:475-487, is not needed
-// for that).
+// an earlier pass consumed.  NPO's partitioned form and the sort-merge names take
+// it from the top bits of key * kHashMul (equal keys still meet in one partition;
+// the reference's range split of the high bits, sorting/joins/
+// sortmergejoin_multiway.cpp:475-487, is not needed for that).
 #pragma once
 
 #include "adb_common.cuh"

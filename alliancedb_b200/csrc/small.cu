@@ -113,6 +113,8 @@ small_join(const uint64_t *__restrict__ R, uint64_t allR, uint32_t lnb, const ui
 // 51, 2^16 x 2^16 20 / 79 / 47, 2^17 x 2^18 38 / 96 / 63, 2^18 x 2^18 (2^23 probes) 54 /
 // 76 / 55 (64 / 91 / 67), and past it 2^18 x 2^19 90 / 90 / 62, 2^19 x 2^18 (110 / 86 / 86).
 // With one chunk: 2^13 x 2^23 79 / 196 / 223, 2^13 x 2^27 1007 / 1895 / 2796.
+// With many and a short S, whole calls, us, here / partitioned: 2^22 x 2^11 41 / 165,
+// 2^24 x 2^11 82 / 356, 2^26 x 2^8 229 / 735, 2^27.5 x 2^8 578 / 1793.
 bool small_fits(uint64_t nR, uint64_t nS) {
     const uint64_t chunks = (nR + (1u << kSmallLog2) - 1) >> kSmallLog2;
     return chunks <= 1 || (chunks <= kSmallMaxChunks && chunks * nS <= kSmallMaxProbes);

@@ -43,8 +43,8 @@ __device__ __forceinline__ void bitonic_words(uint64_t *dst, uint32_t n) {
 // holds 64 scratch words.  All threads call it.
 //
 // MSD counting sort on the (at most) 12 highest key bits that differ within
-// the chunk, all-ones words in a bucket of their own behind the rest (they
-// pad callers' page slots, so they are kept out of the bit analysis); then an
+// the chunk, all-ones words in a bucket of their own behind the rest (out of the
+// bit analysis: as a bitonic sort's padding they must come last); then an
 // insertion sort inside each bucket when the buckets are wider than one key.
 // A bucket of more than 128 tuples that needs sorting makes the whole chunk
 // take the bitonic path instead.

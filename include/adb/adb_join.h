@@ -108,7 +108,8 @@ typedef struct adb_join_result {
                                    radix: partition pass 1, pass 2 (0 with one pass),
                                    work list, join kernel; NPO: grouping by table region, build, -, probe
                                    (partitioned: as radix);
-                                   m-way: as radix, the last the sort + merge-join kernel */
+                                   m-way: as radix, the last counts R's tuples into buckets of their
+                                   hash and scans the bucket of every S tuple */
     float ms_h2d;               /* host->device copy time (adb_join only) */
     uint64_t materialized;      /* tuples written to the materialisation buffer */
 } adb_join_result;
