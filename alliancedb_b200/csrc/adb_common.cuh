@@ -15,14 +15,9 @@ namespace adb {
 
 constexpr int kNumSMs = 148;          // B200: 2 dies x 74 SMs
 constexpr int kWarp = 32;
-// Multiplicative hashing (Knuth, TAOCP 6.4): tables and digits take the top bits
-// of key * kHashMul, 2^32 (sqrt 3 - 1) made odd.  A sharded join's ranks hold the
-// keys with equal top bits of key * kShardMul, 2^32 / golden ratio (shard.cu), so
-// the two must not be multiples of one another: with one constant for both, a
-// rank of N filled an Nth of its partitions and buckets, and NPO's table there
-// overflowed from N = 4 on (20,000 tuples: 600 bucket reads an insert).
-constexpr uint32_t kHashMul = 0xBB67AE85u;
-constexpr uint32_t kShardMul = 0x9E3779B1u;
+// Fibonacci hashing (Knuth, TAOCP 6.4): tables and digits take the top bits of
+// key * 2^32 / golden ratio, which spread dense keys evenly.
+constexpr uint32_t kHashMul = 0x9E3779B1u;
 
 __host__ __device__ __forceinline__ uint32_t tkey(uint64_t w) { return (uint32_t)(w >> 32); }
 __host__ __device__ __forceinline__ uint32_t tpay(uint64_t w) { return (uint32_t)w; }

@@ -50,11 +50,12 @@ def sum_results(count: int, checksum: int, device=None) -> tuple[int, int]:
 
 
 def shard_of(keys, parts: int):
-    """Destination rank of each key: (key * 0x9E3779B1 mod 2^32) * parts / 2^32
-    (the rule of adb_shard_split)."""
-    k = np.asarray(keys, dtype=np.uint64)
-    h = (k * np.uint64(0x9E3779B1)) & np.uint64(0xFFFFFFFF)
-    return ((h * np.uint64(parts)) >> np.uint64(32)).astype(np.int64)
+    """Destination rank of each key: h * parts / 2^32, h the MurmurHash3 finalizer of the
+    key without its last shift (the rule of adb_shard_split)."""
+    h = np.asarray(keys).astype(np.uint32)
+    h = (h ^ (h >> np.uint32(16))) * np.uint32(0x85EBCA6B)
+    h = (h ^ (h >> np.uint32(13))) * np.uint32(0xC2B2AE35)
+    return ((h.astype(np.uint64) * np.uint64(parts)) >> np.uint64(32)).astype(np.int64)
 
 
 def exchange(send, counts, device=None):

@@ -282,7 +282,10 @@ int adb_serve_run(const adb_serve_config *cfg, const adb_serve_request *req, uin
  * rank into dOut (device, n tuples): the tuples of part p (p < parts <= 32)
  * are dOut[off_p .. off_p + counts[p]), off_p = counts[0] + .. + counts[p-1],
  * in no particular order; counts is a host array of `parts` entries.  The
- * destination of a key is (key * 0x9E3779B1 mod 2^32) * parts / 2^32.  After an
+ * destination of a key is h * parts / 2^32 with h = fmix32(key), in 32 bits
+ *     h = (key ^ key >> 16) * 0x85EBCA6B,  h = (h ^ h >> 13) * 0xC2B2AE35:
+ * independent of the bits the joins' digits and tables are taken from, so that a
+ * rank's tuples spread over all of its partitions and buckets.  After an
  * all-to-all of the parts, every rank holds all tuples of its keys from both
  * relations and joins them alone; the ranks' (count, checksum) pairs add up
  * (mod 2^64) to the join of the whole relations.  Synchronises `stream`

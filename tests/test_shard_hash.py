@@ -1,10 +1,10 @@
-"""A rank of a sharded join holds the keys of one destination (the top bits of
-key * kShardMul); the tables and digits of its local join take the top bits of
-key * kHashMul.  The two must not fix one another: the keys of one shard must
-spread over all of the local join's partitions and buckets.
+"""A rank of a sharded join holds the keys of one destination (adb_shard_split);
+the tables and digits of its local join take the top bits of key * kHashMul.  The
+two must not fix one another: the keys of one shard must spread over all of the
+local join's partitions and buckets.
 
-On the CPU a model of the rules with the constants read from the source; on the
-GPU the joins of one shard, right and not slower than those of all keys."""
+On the CPU a model of the joins' rules with the constant read from the source; on
+the GPU the joins of one shard, right and not slower than those of all keys."""
 import re
 from pathlib import Path
 
@@ -15,13 +15,18 @@ import alliancedb_b200 as adb
 from alliancedb_b200.dist import shard_of
 
 SRC = (Path(adb.__file__).parent / "csrc" / "adb_common.cuh").read_text()
-HASH, SHARD = (int(re.search(rf"{n} = (0x[0-9A-Fa-f]+)u", SRC)[1], 16) for n in ("kHashMul", "kShardMul"))
+HASH = int(re.search(r"kHashMul = (0x[0-9A-Fa-f]+)u", SRC)[1], 16)
 
 
-def test_the_split_and_the_package_use_one_rule():
-    k = np.arange(0, 1 << 32, 9_999_991, dtype=np.uint64)
-    for parts in (1, 3, 8, 32):
-        assert np.array_equal(shard_of(k, parts), ((k * np.uint64(SHARD) & np.uint64(0xFFFFFFFF)) * np.uint64(parts)) >> np.uint64(32))
+def test_the_split_rule():
+    """Values of the rule worked out with Python's integers."""
+    m = (1 << 32) - 1
+    for key in (0, 1, 2, 0x7FFFFFFF, 0x9E3779B1, 0xFFFFFFFF):
+        h = ((key ^ (key >> 16)) * 0x85EBCA6B) & m
+        h = ((h ^ (h >> 13)) * 0xC2B2AE35) & m
+        for dtype in (np.uint32, np.uint64, np.int64):
+            for parts in (1, 3, 8, 32):
+                assert shard_of(np.array([key], dtype), parts)[0] == h * parts >> 32
 
 
 def one_shard(n, parts, sparse, seed=1):
