@@ -76,9 +76,10 @@ typedef struct adb_join_params {
     int32_t progressive_step;   /* param_t.progressive_step, PMJ run size in % of each side */
     int32_t merge_step;         /* param_t.merge_step, PMJ runs merged per step */
     int32_t radix_bits;         /* PRO/PRH/RJ fan-out bits; 0 = chosen from |R|.  NPO: bits of the table
-                                   regions its inputs are grouped by (up to 9); 0 = chosen (one table
-                                   while it stays in L2, |R| up to about 2^22, else the partitioned
-                                   join on hashed digits), < 0 = one table, no grouping */
+                                   regions its inputs are grouped by (up to 9; none above |R| = 2^31);
+                                   0 = chosen (one table while it stays in L2, |R| up to about 2^22 or,
+                                   with |S| >= 8 |R|, 7.3M, else the partitioned join on hashed digits),
+                                   < 0 = one table, no grouping */
     int32_t part_fanout;        /* joinconfig_t.PARTFANOUT for m-way/m-pass, taken up to 2^16; 0 = chosen */
     int32_t materialize;        /* 1: also write <S-key, S-payload> per match (JOIN_RESULT_MATERIALIZE) */
     int32_t batch_tuples;       /* eager joins: arrival micro-batch in tuples per side; 0 = 1 ms of stream */
